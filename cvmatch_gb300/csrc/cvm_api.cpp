@@ -505,11 +505,14 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     }
     const int cnS = J.mode == 1 ? 4 : J.cnFixed;
     const SepGrid sg = sep_grid(rw, rh);
+    // (a Matcher's cached spectra were built for the same effective form)
+    const int form = effective_form(J.form, *G);
     int nparts = 0, partOff[2] = {0, 0};
     for (int c = 0; c < G->nclass; c++) {
         int P = 0;
         partOff[c] = nparts;
-        nparts += G->fc[c].ntiles * inv_rows_ctas_per_tile(G->fc[c], G->g.blockH, &P);
+        nparts += G->fc[c].ntiles *
+                  inv_rows_ctas_per_tile(G->fc[c], G->g.blockH, &P, 0, form == CVM_FORM_MIXED && G->fc[c].log2n == 10, 1);
     }
     const size_t hElems = (size_t)stat_pitch(cnS) * J.ih * sg.hp;
     // a tall template with a fixed channel count: 16-row block sums of the
@@ -522,8 +525,6 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     size_t bytes = Arena::bytes(1, sizeof(DevParams)) + Arena::bytes(1, sizeof(DevFrame)) +
                    Arena::bytes(nparts, sizeof(Partial)) + Arena::bytes(hElems, sizeof(unsigned int)) +
                    Arena::bytes((size_t)rw * rh, sizeof(float2)) + (bElems ? Arena::bytes(bElems, sizeof(unsigned int)) : 0);
-    // (a Matcher's cached spectra were built for the same effective form)
-    const int form = effective_form(J.form, *G);
     const bool fast = form != CVM_FORM_EXACT;
     // one channel: the fused forward + conj-multiply + inverse column pass
     // already yields the single correlation spectrum the fast form sums to
@@ -711,7 +712,7 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     CVM_CUDA(cudaStreamWaitEvent(st, ss.joinStats, 0));
     for (int c = 0; c < G->nclass; c++)
         CVM_CUDA(launch_inv_rows(G->g, G->fc[c], c, fast ? 1 : cnS, ms, 1, G->g.blockH, partOff[c], nparts, parts,
-                                 &F->normDone, J.out, st));
+                                 &F->normDone, J.out, st, 0, F->bounds));
     return CVM_OK;
 }
 
@@ -1420,7 +1421,8 @@ int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, 
             int P = 0;
             bg->partOff[c] = nparts;
             nparts += G.fc[c].ntiles * inv_rows_ctas_per_tile(G.fc[c], G.fc[c].dftH, &P, bfast,
-                                                              bg->form == CVM_FORM_MIXED && G.fc[c].log2n == 10);
+                                                              bg->form == CVM_FORM_MIXED && G.fc[c].log2n == 10,
+                                                              (int)b.members.size());
         }
         bg->nparts = nparts;
         std::vector<DevMember> tab(b.members.size());
@@ -1571,7 +1573,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     const bool blkOk = anyStatsKernel && 16ull * (unsigned)twMax * (cnP == 4 ? 3u : 1u) * 65025ull < (1ull << 32);
     const size_t blkElems = blkOk ? prefixRow * (size_t)(ph / 16) : 0;
     const size_t bytes = Arena::bytes(n, sizeof(DevParams)) + Arena::bytes(1, sizeof(DevFrame)) +
-                         Arena::bytes(n, sizeof(int)) + Arena::bytes(prefixElems, sizeof(unsigned int)) +
+                         Arena::bytes((size_t)3 * n, sizeof(int)) + Arena::bytes(prefixElems, sizeof(unsigned int)) +
                          (blkElems ? Arena::bytes(blkElems, sizeof(unsigned int)) : 0) +
                          (satElems ? Arena::bytes(satElems, sizeof(unsigned int)) +
                                          Arena::bytes(satBlkElems, sizeof(unsigned int))
@@ -1598,7 +1600,8 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     A.base = static_cast<char *>(buf.p);
     DevParams *P = A.take<DevParams>(n);
     DevFrame *F = A.take<DevFrame>(1);
-    int *counters = A.take<int>(n);
+    int *counters = A.take<int>((size_t)3 * n);  // per member: finished CTAs, then two words of extrema so far
+    unsigned int *bounds = reinterpret_cast<unsigned int *>(counters + n);
     unsigned int *prefix = A.take<unsigned int>(prefixElems);
     unsigned int *prefixBlk = blkElems ? A.take<unsigned int>(blkElems) : nullptr;
     unsigned int *sat = satElems ? A.take<unsigned int>(satElems) : nullptr;
@@ -1625,7 +1628,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     } sideJoin{ss, st};
     CVM_CUDA(cudaMemcpyAsync(P, f->dP, n * sizeof(DevParams), cudaMemcpyDeviceToDevice, st));
     CVM_CUDA(cudaMemsetAsync(F, 0, sizeof(DevFrame), st));
-    CVM_CUDA(cudaMemsetAsync(counters, 0, n * sizeof(int), st));
+    CVM_CUDA(cudaMemsetAsync(counters, 0, (size_t)3 * n * sizeof(int), st));
     CVM_CUDA(launch_prep(nullptr, 0, 0, 0, f->step, 0, f->step == 4 ? dParent : nullptr, pstride, pw, ph, P, n, 0, 0,
                          0, F, st));
     CVM_CUDA(launch_row_prefix(dParent, pstride, f->step, pw, ph, cnP, prefix, hpP, st));
@@ -1710,7 +1713,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
             }
             for (int c = 0; c < G.nclass; c++)
                 CVM_CUDA(launch_inv_rows(G.g, G.fc[c], c, fast ? 1 : cnS, ms, nw, G.fc[c].dftH, bg.partOff[c],
-                                         bg.nparts, parts, counters, dOut, rst, fast));
+                                         bg.nparts, parts, counters, dOut, rst, fast, bounds, nm));
             if (overlap) CVM_CUDA(cudaEventRecord(ss->rowsDone[set], rst));
         }
     }

@@ -76,6 +76,9 @@ struct InvArgs {
     int nparts;       // partial records per member (all classes)
     Partial *partials;
     int *counters;    // per member params index
+    // per member params index: keys of the largest score and of the negated
+    // smallest score of the CTAs that have finished (0: none), or nullptr
+    unsigned int *bounds;
     cvm_result *out;
     const void *tcTab;  // the tensor-core kernel's tables (set by its launcher)
 };
@@ -150,6 +153,12 @@ bool encode_frame_map(CUtensorMap *map, const void *img, long long istride, long
 // and cleared).
 int rows_error_read_clear();
 void launch_inv_rows_fixed(const InvArgs &a, dim3 grid, size_t smem, cudaStream_t st);
+// The inverse rows with a small thread group per row pair, 2^7 .. 2^11
+// (cvm_lines.cu; grid: members x CTAs per tile x tiles), and how many row
+// pairs a CTA holds at a time.
+bool inv_lines_length(int log2n);
+int inv_lines_cta(int log2n);
+void launch_inv_lines(const InvArgs &a, dim3 grid, cudaStream_t st);
 // The column kernels specialised on dftH = 2^5 .. 2^12 (cvm_cols.cu).
 bool cols_fixed_length(int log2H);
 void launch_cols_fixed(const ColsArgs &a, dim3 grid, size_t smem, cudaStream_t st);
@@ -251,6 +260,69 @@ __device__ __forceinline__ void bfly4_one(float2 *pa, float2 *pc, float2 *pb, fl
     *pc = make_float2(s1x + rr, s1y + ri);
     *pb = make_float2(s0x - s2x, s0y - s2y);
     *pd = make_float2(s1x - rr, s1y - ri);
+}
+
+__host__ __device__ constexpr int ilog2k(int v) { return v <= 1 ? 0 : 1 + ilog2k(v >> 1); }
+
+__host__ __device__ constexpr int brevk(int x, int bits) {
+    int r = 0;
+    for (int i = 0; i < bits; i++) r |= ((x >> i) & 1) << (bits - 1 - i);
+    return r;
+}
+
+// Stage h's table starts at h - 1 (even L) or h - 2 (odd L, after the
+// head's h=2 table) in makeTriTwiddles' concatenation (radix4.go:45-73).
+__host__ __device__ constexpr int tw_off(int L, int h) { return (L & 1) ? h - 2 : h - 1; }
+
+// Units in registers: radix 16 (two stages, quarters H and 4H), radix 4
+// (quarter H) and the head of an odd log2 length (the radix-2 stage and the
+// h = 2 stage on 8 contiguous elements); t points at the unit's column of
+// its stage's twiddle table.
+template <bool INV, int H, bool F = false>
+__device__ __forceinline__ void math16(float2 *e, const float2 *__restrict__ t) {
+    const float2 *tB = t + 3 * H;
+    if constexpr (F && H == 1) {
+        // quarter 1: the first stage's twiddles and the second stage's
+        // column 0 are all 1
+#pragma unroll
+        for (int b = 0; b < 4; b++) bfly4_one<INV>(&e[4 * b], &e[4 * b + 1], &e[4 * b + 2], &e[4 * b + 3]);
+        bfly4_one<INV>(&e[0], &e[4], &e[8], &e[12]);
+#pragma unroll
+        for (int q = 1; q < 4; q++)
+            bfly4<INV, F>(&e[q], &e[q + 4], &e[q + 8], &e[q + 12], __ldg(tB + q), __ldg(tB + 4 + q),
+                          __ldg(tB + 8 + q));
+        return;
+    }
+    const float2 a1 = __ldg(t), a2 = __ldg(t + H), a3 = __ldg(t + 2 * H);
+#pragma unroll
+    for (int b = 0; b < 4; b++) bfly4<INV, F>(&e[4 * b], &e[4 * b + 1], &e[4 * b + 2], &e[4 * b + 3], a1, a2, a3);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        bfly4<INV, F>(&e[q], &e[q + 4], &e[q + 8], &e[q + 12], __ldg(tB + H * q), __ldg(tB + 4 * H + H * q),
+                   __ldg(tB + 8 * H + H * q));
+}
+
+template <bool INV, int H, bool F = false>
+__device__ __forceinline__ void math4(float2 *e, const float2 *__restrict__ t) {
+    bfly4<INV, F>(&e[0], &e[1], &e[2], &e[3], __ldg(t), __ldg(t + H), __ldg(t + 2 * H));
+}
+
+template <bool INV, bool F = false>
+__device__ __forceinline__ void math_head(float2 *e, const float2 *__restrict__ t) {
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+        const float2 u = e[i], v = e[i + 1];
+        e[i] = make_float2(__fadd_rn(u.x, v.x), __fadd_rn(u.y, v.y));
+        e[i + 1] = make_float2(__fsub_rn(u.x, v.x), __fsub_rn(u.y, v.y));
+    }
+    if constexpr (F) {
+        bfly4_one<INV>(&e[0], &e[2], &e[4], &e[6]);
+        bfly4<INV, F>(&e[1], &e[3], &e[5], &e[7], __ldg(t + 1), __ldg(t + 3), __ldg(t + 5));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            bfly4<INV, F>(&e[j], &e[j + 2], &e[j + 4], &e[j + 6], __ldg(t + j), __ldg(t + 2 + j), __ldg(t + 4 + j));
+    }
 }
 
 // normOne's score ladder (impl.go:825-849): |num| < den -> num / den,

@@ -75,6 +75,7 @@ struct DevFrame {
     int cnMax;                   // largest effective cn among the members
     int done;                    // CTAs of k_prep finished (last one finalises)
     int normDone;                // CTAs of a solo k_norm finished (last one merges)
+    unsigned int bounds[2];      // a solo match's extrema so far (InvArgs::bounds)
 };
 
 // One correlation target of the tail kernels: a solo match or one fleet
@@ -174,12 +175,21 @@ cudaError_t launch_cols(int mode, const float2 *in, float2 *out, int cnS, const 
 // a fleet: dftH), the same value for the launch and the partial count.
 // wide (fleets in the fast form, whose waves have CTAs to spare): twice
 // the row pairs per CTA, no channel accumulator in shared memory.
+// bounds (optional): two words per params index, zero before the first
+// class's launch, where the member's finished CTAs leave their extrema for
+// the later ones.  membersAll: the members of the partial count (a bucket's;
+// the launch's nmembers are one wave of them).
 cudaError_t launch_inv_rows(const TileGeom &g, const FftClass &fc, int cls, int cnS, const MemberSet &ms,
                             int nmembers, int rowsMax, int partOffset, int nparts, Partial *partials, int *counters,
-                            cvm_result *out, cudaStream_t st, int wide = 0);
+                            cvm_result *out, cudaStream_t st, int wide = 0, unsigned int *bounds = nullptr,
+                            int membersAll = 1);
 // tc: the launch runs the tensor-core kernel (CVM_FORM_MIXED, 1024-point
-// rows), which takes 32 row pairs per CTA in a fleet (wide)
-int inv_rows_ctas_per_tile(const FftClass &fc, int rowsMax, int *pairsPerCta, int wide = 0, int tc = 0);
+// rows), which takes 32 row pairs per CTA in a fleet (wide); members: the targets
+// of all launches with these partial records (a fleet bucket's members);
+// lanes: the launch has statistics lanes (all but the fixed-scratch entry
+// point's)
+int inv_rows_ctas_per_tile(const FftClass &fc, int rowsMax, int *pairsPerCta, int wide, int tc, int members,
+                           int lanes = 1);
 // Normalisation + first-occurrence extrema: CW x B results per CTA, ncx x
 // nby CTAs per member, result rows in groups of G; the member's last CTA
 // writes its result to out[outIdx].  counters (one int per member of the

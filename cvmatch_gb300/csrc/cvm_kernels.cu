@@ -2062,7 +2062,7 @@ cudaError_t launch_cols(int mode, const float2 *in, float2 *out, int cnS, const 
     return cudaGetLastError();
 }
 
-int inv_rows_ctas_per_tile(const FftClass &fc, int rowsMax, int *pairsPerCta, int wide, int tc) {
+int inv_rows_ctas_per_tile(const FftClass &fc, int rowsMax, int *pairsPerCta, int wide, int tc, int members, int lanes) {
     // 4096 elements per CTA: the radix-16 passes (n/16 units per line) keep
     // all 256 threads busy, ~68 KB of shared memory (three CTAs per SM);
     // wide: 8192 elements (two units per thread per pass), ~70 KB without
@@ -2077,13 +2077,24 @@ int inv_rows_ctas_per_tile(const FftClass &fc, int rowsMax, int *pairsPerCta, in
     // SM slot, and a third CTA on an SM makes that SM the kernel's tail.
     const int rows = rowsMax < fc.dftH ? rowsMax : fc.dftH;
     const int pairs = (rows + 1) / 2;
+    if (lanes && !tc && inv_lines_length(fc.log2n)) {
+        // cvm_lines.cu: a CTA takes several pairs one after another (each
+        // one's loads run ahead of it, its extrema merge once).  256
+        // templates on 2560x1440, fast form: 4096 elements per CTA 2.01 ms
+        // of rows, 8192 1.93; 64 templates on 1920x1080, exact form (a third
+        // of the CTAs, each pair three transforms long): 0.84 and 0.89.
+        // Fewer pairs until there are ten CTAs for every SM.
+        const int nl = inv_lines_cta(fc.log2n);
+        P = (wide ? 8192 : 4096) / fc.n;
+        while (P > nl && (long long)((pairs + P - 1) / P) * fc.ntiles * members < 10 * 152) P >>= 1;
+    }
     *pairsPerCta = P;
     return (pairs + P - 1) / P;
 }
 
 cudaError_t launch_inv_rows(const TileGeom &g, const FftClass &fc, int cls, int cnS, const MemberSet &ms,
                             int nmembers, int rowsMax, int partOffset, int nparts, Partial *partials, int *counters,
-                            cvm_result *out, cudaStream_t st, int wide) {
+                            cvm_result *out, cudaStream_t st, int wide, unsigned int *bounds, int membersAll) {
     InvArgs a;
     a.g = g;
     a.fc = fc;
@@ -2093,12 +2104,13 @@ cudaError_t launch_inv_rows(const TileGeom &g, const FftClass &fc, int cls, int 
     int P = 0;
     if (wide && (!ms.form || !rows_fixed_length(fc.log2n))) return cudaErrorInvalidValue;
     const bool tc = inv_rows_tc_applies(fc, ms);
-    const int ctas = inv_rows_ctas_per_tile(fc, rowsMax, &P, wide, tc);
+    const int ctas = inv_rows_ctas_per_tile(fc, rowsMax, &P, wide, tc, membersAll, ms.lanes != nullptr);
     a.pairsPerCta = P;
     a.partOffset = partOffset;
     a.nparts = nparts;
     a.partials = partials;
     a.counters = counters;
+    a.bounds = bounds;
     a.out = out;
     dim3 grid(ctas, fc.ntiles, nmembers);
     if (tc) {
@@ -2109,7 +2121,9 @@ cudaError_t launch_inv_rows(const TileGeom &g, const FftClass &fc, int cls, int 
     }
     const size_t smem = (size_t)P * (padded_len(fc.n) * sizeof(float2) + (wide ? 0 : 2 * fc.n * sizeof(float)));
     ProfScope ps("k_inv_rows", st);
-    if (rows_fixed_length(fc.log2n)) {
+    if (inv_lines_length(fc.log2n) && ms.lanes) {
+        launch_inv_lines(a, dim3(nmembers, ctas, fc.ntiles), st);
+    } else if (rows_fixed_length(fc.log2n)) {
         launch_inv_rows_fixed(a, grid, smem, st);
     } else {
         set_smem(k_inv_rows, smem);

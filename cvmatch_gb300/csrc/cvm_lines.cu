@@ -1,0 +1,497 @@
+// cvm_lines.cu -- the inverse row transforms of 2^7 .. 2^11 points, one
+// small group of threads per row pair.
+//
+// inverseRowPair (impl.go:394-444), the channel sum, the correlation's end
+// of normOne (impl.go:825-849) and the first-occurrence extrema, with the
+// butterflies, twiddles and rounded operations of k_inv_rows_t
+// (cvm_rows.cu) in the same order: the scores are the same bits.  What
+// differs is who does what.
+//
+// What bounds it.  A transform of N points is N/16 units of 16 elements per
+// pass, so N/16 threads hold a whole line in registers and its passes need
+// no more threads than that.  With 256-thread CTAs over several lines (four
+// per SM) every pass ended in a barrier over all of them, and the loads of
+// the spectrum rows and of the score's denominators (both from DRAM)
+// stalled the whole CTA; a third of the 4100 warp instructions per
+// 1024-point line were the score ladder of results that are no extremum.
+// Here a line belongs to N/16 threads of a 64-thread CTA (128 for N = 2048):
+// barriers span two warps (one for N <= 512), the groups drift apart, the
+// next row pair's rows and den are on their way to L2 while the current one
+// is transformed, and results that cannot be extrema skip the ladder (Track,
+// below): 2400 warp instructions per line, 54 % of the issue slots, the
+// instructions' own latency first among the stalls.
+//
+// Measured (GB300, the rows of one FindAll in sequence): 256 RGBA templates
+// on 2560x1440, fast form, 571 thousand 1024-point lines: 3.17 -> 1.86 ms;
+// 64 templates on 1920x1080, exact form: 1.19 -> 0.83 ms.
+//
+// Data path of a line: pass 1 combines Z = U + iV (and its mirror) from the
+// two spectrum rows on the way into registers, so the combined line is never
+// stored; its outputs go to the line buffer; the last pass's outputs are
+// scored in registers.  Staging the rows in shared memory (cp.async) instead
+// of reading each value twice from L1 measured 2.62 ms: 17 KB per line
+// leaves the twiddles no L1.
+//
+// Layout of the line buffer: pass 1's unit of natural index k0 (logical
+// block v = brev(k0)) stores output i at i * PITCH + k0.  Pass 2's unit
+// (block b, column j) reads its 16 elements at j * PITCH + brev4(i) * NB +
+// brev(b) and stores them in place, output i at j * PITCH + i * NB +
+// brev(b); pass 3's unit jj = j + R1 * i then reads NB consecutive
+// elements.  PITCH keeps the three access patterns free of bank conflicts.
+#include "cvm_device.cuh"
+
+namespace cvm {
+namespace {
+
+// Floats as unsigned integers of the same order (every finite float's key is
+// above 0, which stands for "none yet").
+__device__ __forceinline__ unsigned int ordered_key(float f) {
+    const unsigned int u = __float_as_uint(f);
+    return (u >> 31) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float from_key(unsigned int k) {
+    return __uint_as_float((k >> 31) ? (k & 0x7fffffffu) : ~k);
+}
+
+// Only the extrema leave a match without a score map, so a result that
+// cannot be one needs no quotient: scores outside (lo, hi) may be extrema.
+// hi lies below the largest known score by 2^-20 of it and 1e-15: num < hi *
+// den then implies that the computed quotient (within 2 ulp, 2^-22) is below
+// that score, the product's rounding (2^-24, or 1e-45 where it underflows:
+// den >= kCutDen) included, and, scores being at most 1 (+ 2 ulp), that num <
+// den.  lo is its mirror.  A result at or above the cut, ties included,
+// takes the whole ladder.
+constexpr float kCutDen = 1e-20f;
+__device__ __forceinline__ float below(float v) { return v - (fabsf(v) * 9.5367431640625e-07f + 1e-15f); }
+__device__ __forceinline__ float above(float v) { return v + (fabsf(v) * 9.5367431640625e-07f + 1e-15f); }
+
+struct Track {
+    float minV, maxV, hi, lo;
+    int minL, maxL;       // CTA-local raster index (row x N + x)
+};
+
+__device__ __forceinline__ void track(Track &t, float sc, int l) {
+    if (sc < t.minV || (sc == t.minV && l < t.minL)) {
+        t.minV = sc;
+        t.minL = l;
+    }
+    if (sc > t.maxV || (sc == t.maxV && l < t.maxL)) {
+        t.maxV = sc;
+        t.maxL = l;
+    }
+}
+
+// A result that may be an extremum.  Out of line: rare, and inlined copies
+// of it at sixteen to thirty-two results cost the kernel its instruction
+// cache (half its stalls).
+template <bool FAST>
+__device__ __noinline__ Track score_track(Track t, float num, float den, float denFlat, int l) {
+    const float sc = FAST ? score_fast(num, den, denFlat) : score_exact(num, den);
+    track(t, sc, l);
+    t.hi = fmaxf(t.hi, below(sc));
+    t.lo = fminf(t.lo, above(sc));
+    return t;
+}
+
+// The group's extrema so far as the cuts of all its threads.
+__device__ __forceinline__ void cut_share(Track &t, unsigned int mask) {
+    const float hi = from_key(__reduce_max_sync(mask, ordered_key(t.maxV)));
+    const float lo = -from_key(__reduce_max_sync(mask, ordered_key(-t.minV)));
+    if (hi > -FLT_MAX) t.hi = fmaxf(t.hi, below(hi));
+    if (lo < FLT_MAX) t.lo = fminf(t.lo, above(lo));
+}
+
+// The cuts from the extrema (keys of the maximum and of the negated minimum)
+// of the member's CTAs that have finished; false when there are none.
+__device__ __forceinline__ bool cut_load(Track &t, const unsigned int *b) {
+    const unsigned int kx = *reinterpret_cast<const volatile unsigned int *>(b);
+    const unsigned int kn = *reinterpret_cast<const volatile unsigned int *>(b + 1);
+    if (kx) t.hi = fmaxf(t.hi, below(from_key(kx)));
+    if (kn) t.lo = fminf(t.lo, above(-from_key(kn)));
+    return kx != 0u && kn != 0u;
+}
+
+// den and (t, den): read once, so they leave the L1 lines to the twiddles.
+__device__ __forceinline__ float ld_once(const float *p) {
+    float v;
+    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 ld_once(const float2 *p) {
+    float2 v;
+    asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+
+// Out of line: the option's code stays out of the loads' way.
+__device__ __noinline__ float sat_den_call(const MemberSet &ms, const DevMember &m, const DevParams &Pm, int y, int x) {
+    return sat_den(ms, m, Pm, y, x);
+}
+
+template <int L>
+struct Lines {
+    static constexpr int N = 1 << L;
+    static constexpr int R1 = (L & 1) ? 8 : 16;           // pass 1: the head, or radix 16 at quarter 1
+    static constexpr int K1 = N / R1;                     // its units
+    static constexpr int NB = N / (16 * R1);              // blocks of pass 2 = pass 3's radix (1: no pass 3)
+    static constexpr int H2 = R1, H3 = 16 * R1;           // quarters of passes 2 and 3
+    // line pitch: conflict-free for pass 2's reads (8-byte words of NB-wide
+    // blocks) and pass 3's 16-byte reads over consecutive columns
+    static constexpr int PITCH = NB == 1 ? K1 + 1 : (NB == 4 ? K1 + 6 : K1 + 2);
+    static constexpr int LINE = (R1 * PITCH + 1) & ~1;    // elements
+    static constexpr int G = N / 16;                      // threads of a line
+    static constexpr int CTA = G > 64 ? G : 64;
+    static constexpr int NL = CTA / G;                    // lines of a CTA at a time
+    static constexpr size_t SMEM = (size_t)NL * LINE * sizeof(float2);
+};
+
+// The barrier of a line's threads: the CTA (one line at a time) or the
+// group's lanes of its warp.
+template <int G>
+__device__ __forceinline__ void group_sync(unsigned int mask) {
+    if constexpr (G <= 32)
+        __syncwarp(mask);
+    else
+        __syncthreads();
+}
+
+// CTAs per SM the registers are budgeted for: 96 registers hold a fast-form
+// thread's 32 den values ahead of the last pass (12 CTAs spill: 2.13 against
+// 2.01 ms; without them 14 CTAs 2.00 at the same 4096 elements per CTA); the
+// exact form keeps the channel sum of its 16 results, 128 registers (nine
+// CTAs spill: 1.17 against 0.84 ms).
+__host__ __device__ constexpr int lines_ctas(int L, bool fast, bool lean) {
+    return (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 7) : (fast ? 10 : 8))) * (lean ? 4 : 3) / 4;
+}
+
+// LEAN: the extrema alone leave (no score map, no region of interest, den
+// from the statistics kernel): every Match, Find and fleet FindAll without
+// them.
+template <int L, bool FAST, bool LEAN>
+__global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, LEAN)) k_inv_lines(InvArgs a) {
+    griddep_wait();
+    using S = Lines<L>;
+    constexpr int N = S::N, R1 = S::R1, K1 = S::K1, NB = S::NB, G = S::G, NL = S::NL, PITCH = S::PITCH;
+        constexpr int NU = NB == 1 ? 1 : 16 / NB;             // last-pass units of a thread
+    constexpr int RL = NB == 1 ? 16 : NB;                 // their radix
+    constexpr int HL = NB == 1 ? S::H2 : S::H3;           // their quarter
+    constexpr bool BOTH = RL == 4;                        // both rows' den values in registers at once
+    constexpr bool AHEAD = BOTH && FAST;                  // and every unit's
+    extern __shared__ __align__(16) float2 smem[];
+    __shared__ Ext shExt[S::CTA / 32];
+    __shared__ int isLast;
+    const FftClass &fc = a.fc;
+    // members vary fastest: a member's CTAs spread over the whole launch, so
+    // all but its first start from the extrema of earlier ones (a.bounds)
+    const int slot = blockIdx.x;
+    const int tileLocal = blockIdx.z;
+    const int tile = fc.tileFirst + tileLocal;
+    const DevMember &m = member_of(a.ms, slot);
+    const DevParams &Pm = a.ms.params[m.pIdx];
+    const TileBox tb = tile_box(a.g, tile);
+    const int tx = tile % a.g.ntx, ty = tile / a.g.ntx;
+    const int bw = (tx == a.g.ntx - 1) ? m.rw - tb.x0 : a.g.blockW;
+    const int bh = (ty == a.g.nty - 1) ? m.rh - tb.y0 : a.g.blockH;
+    const int pair0 = blockIdx.y * a.pairsPerCta;
+    // the CTA's row pairs; none when its results all lie outside the
+    // member's region of interest (no transform, no extrema)
+    int P = 2 * pair0 < bh ? min(a.pairsPerCta, (bh - 2 * pair0 + 1) >> 1) : 0;
+    if (!LEAN && P > 0 && a.ms.anyRoi) {
+        const int ya = tb.y0 + 2 * pair0, yb = tb.y0 + min(2 * (pair0 + P), bh);
+        if (ya >= m.roiY1 || yb <= m.roiY0 || tb.x0 >= m.roiX1 || tb.x0 + bw <= m.roiX0) P = 0;
+    }
+    const int tid = threadIdx.x;
+    unsigned int *bnd = a.bounds ? a.bounds + 2 * m.pIdx : nullptr;
+    Ext e;
+    ext_init(e);
+    if (P > 0 && Pm.flat) {
+        // a flat template scores 1 everywhere (impl.go:1137-1144)
+        for (int rr = 0; rr < 2 * P && 2 * pair0 + rr < bh; rr++) {
+            const int yy = tb.y0 + 2 * pair0 + rr;
+            if (yy < m.roiY0 || yy >= m.roiY1) continue;
+            for (int x = tid; x < bw; x += S::CTA) {
+                const long long i = (long long)yy * m.rw + tb.x0 + x;
+                if (a.ms.map) a.ms.map[i] = 1.f;
+                if (tb.x0 + x >= m.roiX0 && tb.x0 + x < m.roiX1) ext_add(e, 1.f, i);
+            }
+        }
+    } else if (P > 0) {
+        const int g = tid / G, lt = tid - g * G;          // the thread's group and its place in it
+        const unsigned int mask = G >= 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((tid & 31) / G * G);
+        float2 *ln = smem + (size_t)g * S::LINE;
+        const int hwp = fc.hwp, log2H = fc.log2H;
+        const int cn = FAST ? 1 : Pm.cn;
+        const size_t chanStride = (size_t)fc.dftH * hwp;
+        const float2 *scr = a.ms.scratch[a.cls] + (size_t)slot * a.ms.scratchStride[a.cls] +
+                            (size_t)tileLocal * a.cnS * chanStride;
+        const float2 *lanes = a.ms.lanes + (size_t)slot * a.ms.lanesStride;
+        const float *dens = reinterpret_cast<const float *>(lanes);
+        const float denFlat = near_flat_den(m.tw, m.th, Pm.templNorm);  // fast form: near-flat windows below it
+        float *map = LEAN ? nullptr : a.ms.map;
+        const float denLow = FAST ? fmaxf(denFlat, kCutDen) : kCutDen;
+        const bool ownStats = FAST && !LEAN && a.ms.sat != nullptr;
+        const int rw = m.rw, xlo = m.roiX0 - tb.x0, xhi = m.roiX1 - tb.x0, roiY0 = m.roiY0, roiY1 = m.roiY1;
+        const float2 *triW = fc.triW;
+        bool warm = false;                                // the cuts have been shared once
+        Track t = {FLT_MAX, -FLT_MAX, -INFINITY, INFINITY, INT_MAX, INT_MAX};
+        // rows r and r + 1 of channel k
+        auto row_ptr = [&](int p, int k, int h) {
+            return scr + (size_t)k * chanStride + (size_t)brev_bits(2 * (pair0 + p) + h, log2H) * hwp;
+        };
+        // towards L2, one 128-byte line per thread and step: the two rows
+        // and (last channel) their den
+        auto prefetch = [&](int p, int k) {
+            for (int o = lt; o < 2 * (N / 32 + 1); o += G) {
+                const int h = o > N / 32, c = h ? o - (N / 32 + 1) : o;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(row_ptr(p, k, h) + 16 * c));
+            }
+            if (k == cn - 1 && !ownStats) {
+                constexpr int EB = FAST ? 4 : 8;
+                const int r = 2 * (pair0 + p);
+                for (int h = 0; h < 2 && r + h < bh; h++) {
+                    const char *q = reinterpret_cast<const char *>(lanes) +
+                                    ((long long)(tb.y0 + r + h) * rw + tb.x0) * EB;
+                    for (int o = lt * 128; o < bw * EB; o += G * 128)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
+                }
+            }
+        };
+        float2 acc[FAST ? 1 : 16];                        // the earlier channels' sum, the thread's results
+        for (int p = g; p < P; p += NL)
+#pragma unroll 1
+            for (int k = 0; k < cn; k++) {
+                // pass 1: unit k0's elements are Z[k0 + K1 * brev(i)]
+                // (bit-reversed input), Z = U + iV below N/2 and its mirror
+                // above (impl.go:405-413)
+                const float2 *ur = row_ptr(p, k, 0), *vr = row_ptr(p, k, 1);
+#pragma unroll
+                for (int q = 0; q < 16 / R1; q++) {
+                    const int k0 = lt + q * G;
+                    float2 z[R1];
+                    constexpr int LR1 = R1 == 16 ? 4 : 3;
+#pragma unroll
+                    for (int i = 0; i < R1 / 2; i++) {
+                        const float2 u = __ldg(ur + k0 + K1 * i), v = __ldg(vr + k0 + K1 * i);
+                        z[brevk(i, LR1)] = make_float2(__fsub_rn(u.x, v.y), __fadd_rn(u.y, v.x));
+                    }
+#pragma unroll
+                    for (int i = R1 / 2; i < R1; i++) {
+                        const int n = K1 * (R1 - i) - k0;
+                        const float2 u = __ldg(ur + n);
+                        float2 v = __ldg(vr + n);
+                        float uy = u.y;
+                        if (i == R1 / 2 && k0 == 0) {  // N/2 itself: the direct form
+                            uy = -uy;
+                            v.y = -v.y;
+                        }
+                        z[brevk(i, LR1)] = make_float2(__fadd_rn(u.x, v.y), __fsub_rn(v.x, uy));
+                    }
+                    if constexpr (R1 == 16)
+                        math16<true, 1, FAST>(z, triW);
+                    else
+                        math_head<true, FAST>(z, triW);
+                    // the previous pair's last pass has read the line
+                    if (q == 0) group_sync<G>(mask);
+#pragma unroll
+                    for (int i = 0; i < R1; i++) ln[i * PITCH + k0] = z[i];
+                }
+                if (k + 1 < cn || p + NL < P) prefetch(k + 1 < cn ? p : p + NL, k + 1 < cn ? k + 1 : 0);
+                group_sync<G>(mask);
+                float2 z[16];
+                {
+                    // pass 2: unit (b, j); lanes run over the blocks first
+                    // (NB = 4: even columns, then odd ones, in groups of eight,
+                    // keep the half-warps on distinct banks)
+                    const int bb = lt & (NB - 1), jl = lt / NB;
+                    const int j = NB == 4 ? (jl & 8) | ((jl & 3) << 1) | ((jl >> 2) & 1) : jl;
+                    float2 *q = ln + j * PITCH + bb;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) z[i] = q[brevk(i, 4) * NB];
+                    math16<true, S::H2, FAST>(z, triW + tw_off(L, S::H2) + j);
+                    if constexpr (NB > 1) {
+#pragma unroll
+                        for (int i = 0; i < 16; i++) q[i * NB] = z[i];
+                    }
+                }
+                const bool last = k == cn - 1;
+                const bool odd = 2 * (pair0 + p) + 1 < bh;  // the imaginary part's row exists
+                const int y0 = tb.y0 + 2 * (pair0 + p);
+                const long long row0 = (long long)y0 * rw + tb.x0;
+                // den (and t) of the thread's results, unit it
+                float den[AHEAD ? NU : 1][BOTH ? 2 : 1][RL], tt[BOTH ? 2 : 1][FAST ? 1 : RL];
+                auto load_den = [&](int it, int h) {
+                    const int jj = lt + it * G, is = AHEAD ? it : 0, hs = BOTH ? h : 0;
+                    const long long row = row0 + h * rw;
+                    const int xe = h == 0 || odd ? bw : 0;
+                    if (FAST && ownStats) {
+#pragma unroll
+                        for (int i = 0; i < RL; i++) {
+                            const int x = jj + HL * i;
+                            den[is][hs][i] = x < xe ? sat_den_call(a.ms, m, Pm, y0 + h, tb.x0 + x) : 0.f;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < RL; i++) {
+                            const int x = jj + HL * i;
+                            if constexpr (FAST) {
+                                den[is][hs][i] = x < xe ? ld_once(dens + row + x) : 0.f;
+                            } else {
+                                const float2 td = x < xe ? ld_once(lanes + row + x) : make_float2(0.f, 0.f);
+                                tt[hs][i] = td.x;
+                                den[is][hs][i] = td.y;
+                            }
+                        }
+                    }
+                };
+                if constexpr (AHEAD) {
+                    // every unit's, in flight together while the barrier gathers the line
+#pragma unroll
+                    for (int it = 0; it < NU; it++) {
+                        load_den(it, 0);
+                        load_den(it, 1);
+                    }
+                }
+                if (LEAN && last && p < NL && bnd) warm = cut_load(t, bnd);
+                if constexpr (NB > 1) group_sync<G>(mask);
+#pragma unroll
+                for (int it = 0; it < NU; it++) {
+                    // last-pass unit jj: results x = jj + HL * i of the two rows
+                    const int jj = lt + it * G;
+                    if (last && !AHEAD) {
+                        load_den(it, 0);
+                        if (BOTH) load_den(it, 1);
+                    }
+                    float2 *o = z;
+                    float2 zu[NB == 1 ? 1 : RL];
+                    if constexpr (NB > 1) {
+                        const float4 *q = reinterpret_cast<const float4 *>(ln + (jj & (R1 - 1)) * PITCH + (jj / R1) * NB);
+#pragma unroll
+                        for (int i = 0; i < NB / 2; i++) {
+                            const float4 w = q[i];
+                            // block b sits at brev(b)
+                            zu[brevk(2 * i, ilog2k(NB))] = make_float2(w.x, w.y);
+                            zu[brevk(2 * i + 1, ilog2k(NB))] = make_float2(w.z, w.w);
+                        }
+                        if constexpr (NB == 16)
+                            math16<true, HL, FAST>(zu, triW + tw_off(L, HL) + jj);
+                        else
+                            math4<true, HL, FAST>(zu, triW + tw_off(L, HL) + jj);
+                        o = zu;
+                    }
+                    if (!FAST && !last) {
+                        // the channels' sum, in channel order (impl.go:425-443)
+#pragma unroll
+                        for (int i = 0; i < RL; i++) {
+                            float2 &s = acc[FAST ? 0 : it * RL + i];
+                            s = k == 0 ? o[i] : make_float2(__fadd_rn(s.x, o[i].x), __fadd_rn(s.y, o[i].y));
+                        }
+                        continue;
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        if (h == 1 && !odd) break;
+                        if (h == 1 && !BOTH) load_den(it, 1);
+                        const bool rowIn = y0 + h >= roiY0 && y0 + h < roiY1;
+#pragma unroll
+                        for (int i = 0; i < RL; i++) {
+                            const int x = jj + HL * i, l = (2 * p + h) * N + x;
+                            float num = h ? o[i].y : o[i].x;
+                            if constexpr (!FAST) {
+                                const float2 s = acc[it * RL + i];
+                                if (cn > 1) num = __fadd_rn(h ? s.y : s.x, num);
+                                num = __fsub_rn(num, tt[BOTH ? h : 0][i]);
+                            }
+                            const float d = den[AHEAD ? it : 0][BOTH ? h : 0][i];
+                            // (the results of zero and, in the fast form, near-flat dens take the ladder)
+                            const bool cand = x < bw && !(d >= denLow && num < t.hi * d && num > t.lo * d);
+                            if constexpr (LEAN) {
+                                if (cand) t = score_track<FAST>(t, num, d, denFlat, l);
+                            } else if (x < bw) {
+                                const float sc = FAST ? score_fast(num, d, denFlat) : score_exact(num, d);
+                                if (map) map[row0 + h * rw + x] = sc;
+                                if (rowIn && x >= xlo && x < xhi) track(t, sc, l);
+                            }
+                        }
+                    }
+                    if (LEAN && it == 0 && !warm) {
+                        cut_share(t, mask);
+                        warm = true;
+                    }
+                }
+            }
+        // widen: CTA-local (row, x) -> the member's raster index
+        auto widen = [&](int l) {
+            return l == INT_MAX ? LLONG_MAX
+                                : (long long)(tb.y0 + 2 * pair0 + (l >> L)) * m.rw + tb.x0 + (l & (N - 1));
+        };
+        e.minV = t.minV;
+        e.maxV = t.maxV;
+        e.minI = widen(t.minL);
+        e.maxI = widen(t.maxL);
+    }
+    // a CTA none of whose results passed its member's cuts has nothing to reduce
+    if (__syncthreads_or(e.minI != LLONG_MAX || e.maxI != LLONG_MAX)) ext_block_reduce(e, shExt);
+    if (tid == 0) {
+        Partial &o = a.partials[m.partBase + a.partOffset + tileLocal * gridDim.y + blockIdx.y];
+        o.minV = e.minV;
+        o.maxV = e.maxV;
+        o.minI = e.minI;
+        o.maxI = e.maxI;
+        if (bnd) {
+            if (e.maxI != LLONG_MAX) atomicMax(bnd, ordered_key(e.maxV));
+            if (e.minI != LLONG_MAX) atomicMax(bnd + 1, ordered_key(-e.minV));
+        }
+        __threadfence();
+        isLast = atomicAdd(&a.counters[m.pIdx], 1) == a.nparts - 1;
+    }
+    __syncthreads();
+    if (!isLast) return;
+    __threadfence();
+    ext_init(e);
+    for (int i = tid; i < a.nparts; i += S::CTA) {
+        const volatile Partial *p = a.partials + m.partBase + i;
+        Ext o;
+        o.minV = p->minV;
+        o.maxV = p->maxV;
+        o.minI = p->minI;
+        o.maxI = p->maxI;
+        ext_merge(e, o);
+    }
+    __syncthreads();
+    ext_block_reduce(e, shExt);
+    if (tid == 0) ext_store_result(e, m.rw, a.out + m.outIdx);
+}
+
+template <int L, bool FAST, bool LEAN>
+void lines_one(const InvArgs &a, dim3 grid, cudaStream_t st) {
+    set_smem(k_inv_lines<L, FAST, LEAN>, Lines<L>::SMEM);
+    launch_k(k_inv_lines<L, FAST, LEAN>, grid, dim3(Lines<L>::CTA), Lines<L>::SMEM, st, a);
+}
+
+template <int L>
+void lines_form(const InvArgs &a, dim3 grid, cudaStream_t st) {
+    const bool lean = !a.ms.map && !a.ms.anyRoi && !a.ms.sat;
+    if (a.ms.form)
+        lean ? lines_one<L, true, true>(a, grid, st) : lines_one<L, true, false>(a, grid, st);
+    else
+        lean ? lines_one<L, false, true>(a, grid, st) : lines_one<L, false, false>(a, grid, st);
+}
+
+}  // namespace
+
+bool inv_lines_length(int log2n) { return log2n >= 7 && log2n <= 11; }
+
+// Lines of a CTA at a time.
+int inv_lines_cta(int log2n) { return log2n >= 10 ? 1 : 1 << (10 - log2n); }
+
+void launch_inv_lines(const InvArgs &a, dim3 grid, cudaStream_t st) {
+    switch (a.fc.log2n) {
+        case 7: lines_form<7>(a, grid, st); break;
+        case 8: lines_form<8>(a, grid, st); break;
+        case 9: lines_form<9>(a, grid, st); break;
+        case 10: lines_form<10>(a, grid, st); break;
+        default: lines_form<11>(a, grid, st); break;
+    }
+}
+
+}  // namespace cvm

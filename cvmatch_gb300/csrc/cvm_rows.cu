@@ -805,14 +805,21 @@ void fwd_one(const FwdRowsArgs &a, const CUtensorMap &map, dim3 grid, int thread
     }
 }
 
+// Lengths cvm_lines.cu scores: here only the raw correlation of the
+// fixed-scratch entry point (the exact form, no statistics lanes).
+template <int L>
+void inv_raw(const InvArgs &a, dim3 grid, size_t smem, cudaStream_t st) {
+    set_smem(k_inv_rows_t<L, false>, smem);
+    launch_k(k_inv_rows_t<L, false>, grid, dim3(kThreads), smem, st, a);
+}
+
 template <int L>
 void inv_one(const InvArgs &a, dim3 grid, size_t smem, cudaStream_t st) {
     if (a.ms.form) {
         set_smem(k_inv_rows_t<L, true>, smem);
         launch_k(k_inv_rows_t<L, true>, grid, dim3(kThreads), smem, st, a);
     } else {
-        set_smem(k_inv_rows_t<L, false>, smem);
-        launch_k(k_inv_rows_t<L, false>, grid, dim3(kThreads), smem, st, a);
+        inv_raw<L>(a, grid, smem, st);
     }
 }
 
@@ -874,11 +881,11 @@ void launch_inv_rows_fixed(const InvArgs &a, dim3 grid, size_t smem, cudaStream_
     switch (a.fc.log2n) {
         case 5: inv_one<5>(a, grid, smem, st); break;
         case 6: inv_one<6>(a, grid, smem, st); break;
-        case 7: inv_one<7>(a, grid, smem, st); break;
-        case 8: inv_one<8>(a, grid, smem, st); break;
-        case 9: inv_one<9>(a, grid, smem, st); break;
-        case 10: inv_one<10>(a, grid, smem, st); break;
-        case 11: inv_one<11>(a, grid, smem, st); break;
+        case 7: inv_raw<7>(a, grid, smem, st); break;
+        case 8: inv_raw<8>(a, grid, smem, st); break;
+        case 9: inv_raw<9>(a, grid, smem, st); break;
+        case 10: inv_raw<10>(a, grid, smem, st); break;
+        case 11: inv_raw<11>(a, grid, smem, st); break;
         default: inv_one<12>(a, grid, smem, st); break;
     }
 }
