@@ -392,10 +392,10 @@ class Fleet:
         _check(lib().cvm_fleet_set_overlap(self._h, 1 if on else 0))
 
     def SetStats(self, mode: int):
-        """STATS_KERNEL (the default: the statistics kernel) or
-        STATS_EPILOGUE (window statistics inside the inverse-rows epilogue
-        from the frame's summed-area table, where it applies); the results
-        are the same bits.  See cvm_fleet_set_stats."""
+        """STATS_KERNEL (the statistics kernel) or STATS_EPILOGUE (den on
+        demand inside the inverse rows, from the frame's summed-area table,
+        where it applies); the results are the same bits.  Without a call the
+        fleet chooses by itself.  See cvm_fleet_set_stats."""
         _check(lib().cvm_fleet_set_stats(self._h, mode))
 
     def buckets(self, pw: int, ph: int):

@@ -1112,6 +1112,7 @@ struct FleetBucketGeom {
 
 struct FleetGeom {
     int pw = 0, ph = 0;
+    int stats = CVM_STATS_KERNEL;  // the library's choice of den's source (choose_stats)
     int form = CVM_FORM_EXACT;  // the form the spectra were built for
     std::vector<std::unique_ptr<FleetBucketGeom>> bg;
 };
@@ -1127,7 +1128,7 @@ struct cvm_fleet {
     uint64_t roiGen = 0;       // bumped by every cvm_fleet_set_roi
     int form = CVM_FORM_EXACT; // arithmetic of the member tails (cvm_fleet_set_form)
     int waveMembers = 0;       // members per wave of tails (0: by the 4 GB workspace budget)
-    int statsMode = CVM_STATS_KERNEL;  // or CVM_STATS_EPILOGUE (cvm_fleet_set_stats)
+    int statsMode = -1;        // the library's choice, until cvm_fleet_set_stats
     int overlapWaves = 1;      // cvm_fleet_set_overlap
     Plan forcedPlan;           // every bucket's plan when dftW > 0 (the autotuner's trial fleets)
     ~cvm_fleet() {
@@ -1136,6 +1137,21 @@ struct cvm_fleet {
 };
 
 namespace {
+
+// Statistics lanes of a member, in float2: (t, den) per result, or den alone
+// (a float) in the fast forms.
+size_t lanes_elems(const FleetBucketGeom &bg) {
+    const size_t n = (size_t)bg.rwMax * bg.rhMax;
+    return bg.form != CVM_FORM_EXACT ? (n + 1) / 2 : n;
+}
+
+// True when the summed-area table serves a w x h member: the squared sum of
+// the widest window asked for -- the member's, enlarged by a block of results
+// on either axis -- must be restorable from its residue modulo 2^32: area *
+// cn * 16256 < 2^32, cn up to the frame's channels.
+bool den_table_area(int w, int h, int step) {
+    return (unsigned long long)(w + 15) * (h + 15) * (step == 4 ? 4u : 1u) * 16256ull < (1ull << 32);
+}
 
 // Budget for one wave of member tails' column-pass output.
 constexpr size_t kWaveBytes = size_t(4) << 30;
@@ -1201,7 +1217,7 @@ struct FleetTuneEntry {
 std::map<FleetTuneKey, FleetTuneEntry> g_fleetTune;
 
 int tune_bucket_plan(cvm_fleet *f, const Bucket &b, const uint8_t *dParent, long long pstride, int pw, int ph,
-                     cudaStream_t st, Plan *out) {
+                     cudaStream_t st, int stats, Plan *out) {
     const int rwF = pw - b.tw + 1, rhF = ph - b.th + 1;
     *out = make_plan(b.tw, b.th, rwF, rhF);
     const int nm = (int)b.members.size();
@@ -1254,7 +1270,7 @@ int tune_bucket_plan(cvm_fleet *f, const Bucket &b, const uint8_t *dParent, long
                 cvm_fleet trial;
                 trial.step = f->step;
                 trial.form = f->form;
-                trial.statsMode = f->statsMode;
+                trial.statsMode = stats;
                 trial.forcedPlan = cands[c];
                 Bucket one;
                 one.tw = b.tw;
@@ -1383,6 +1399,80 @@ std::vector<Bucket> fast_buckets(const cvm_fleet *f, int pw, int ph) {
     return out;
 }
 
+// Where a fast-form fleet's den comes from on frames like this one, unless
+// cvm_fleet_set_stats said: on demand (CVM_STATS_EPILOGUE) when blocks of its
+// members' results bound den well, else the statistics kernel.  Blocks without
+// a bound -- flat panels beside thin strokes, under small templates -- make
+// their results form den one by one: 64 icons of 12..32 px on a 1920x1080 user
+// interface (13 % of blocks unbounded) 1.44 ms against 1.08 with the kernel,
+// 64 templates of 16..192 x 16..128 there (2 %) 1.05 against 1.25; more than 3
+// % choose the kernel.  Measured on the first frame of a size, outside stream
+// capture (in one: on demand); results do not depend on it.
+constexpr int kPoorShare = 32;
+
+int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, int ph, cudaStream_t cst, int *out) {
+    *out = CVM_STATS_KERNEL;
+    if (f->form != CVM_FORM_FAST || !dParent) return CVM_OK;
+    *out = f->statsMode >= 0 ? f->statsMode : CVM_STATS_EPILOGUE;
+    if (f->statsMode >= 0) return CVM_OK;
+    const int np = f->step == 4 ? 4 : 2, hp = (int)align_up((size_t)pw + 1, 32);
+    std::vector<DevMember> tab;
+    for (const Bucket &b : f->buckets)
+        for (int i : b.members) {
+            const cvm_matcher *m = f->ms[i];
+            DevMember d;
+            memset(&d, 0, sizeof d);
+            d.pIdx = i;
+            d.tw = m->w;
+            d.th = m->h;
+            d.rw = pw - m->w + 1;
+            d.rh = ph - m->h + 1;
+            if (den_table_area(m->w, m->h, f->step)) tab.push_back(d);
+        }
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (tab.empty() || cudaStreamIsCapturing(cst, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return CVM_OK;
+    }
+    CVM_CUDA(cudaStreamSynchronize(cst));  // the frame, written on the caller's stream
+    cudaStream_t ts = thread_stream();
+    const int n = (int)f->ms.size();
+    const size_t lanes = (size_t)(ph + 1) * hp * (np == 4 ? 6 : 2);
+    PoolBuf buf;
+    CVM_TRY(pool_alloc(buf,
+                       Arena::bytes(n, sizeof(DevParams)) + Arena::bytes(1, sizeof(DevFrame)) +
+                           Arena::bytes(tab.size(), sizeof(DevMember)) + Arena::bytes(1, sizeof(int)) +
+                           Arena::bytes(lanes, 4) + Arena::bytes(sat_scratch_elems(ph, hp, np), 4),
+                       ts));
+    Arena A;
+    A.base = static_cast<char *>(buf.p);
+    DevParams *P = A.take<DevParams>(n);
+    DevFrame *F = A.take<DevFrame>(1);
+    DevMember *T = A.take<DevMember>(tab.size());
+    int *dPoor = A.take<int>(1), poor = 0;
+    unsigned int *sat = A.take<unsigned int>(lanes), *blk = A.take<unsigned int>(sat_scratch_elems(ph, hp, np));
+    CVM_CUDA(cudaMemcpyAsync(P, f->dP, n * sizeof(DevParams), cudaMemcpyDeviceToDevice, ts));
+    CVM_CUDA(cudaMemsetAsync(F, 0, sizeof(DevFrame), ts));
+    CVM_CUDA(cudaMemsetAsync(dPoor, 0, sizeof(int), ts));
+    CVM_CUDA(cudaMemcpyAsync(T, tab.data(), tab.size() * sizeof(DevMember), cudaMemcpyHostToDevice, ts));
+    CVM_CUDA(launch_prep(nullptr, 0, 0, 0, f->step, 0, f->step == 4 ? dParent : nullptr, pstride, pw, ph, P, n, 0, 0, 0,
+                         F, ts));
+    CVM_CUDA(launch_sat(dParent, pstride, pw, ph, hp, np, &F->cnMax, blk, sat, ts));
+    MemberSet ms;
+    memset(&ms, 0, sizeof ms);
+    ms.table = T;
+    ms.params = P;
+    ms.sat = sat;
+    ms.satRow = (size_t)np * hp;
+    ms.satAlpha = np == 4 ? (size_t)(ph + 1) * 4 * hp : 0;
+    ms.satNp = np;
+    CVM_CUDA(launch_den_poor(ms, (int)tab.size(), dPoor, ts));
+    CVM_CUDA(cudaMemcpyAsync(&poor, dPoor, sizeof(int), cudaMemcpyDeviceToHost, ts));
+    CVM_CUDA(cudaStreamSynchronize(ts));
+    if ((long long)poor * kPoorShare > 256LL * (long long)tab.size()) *out = CVM_STATS_KERNEL;
+    return CVM_OK;
+}
+
 int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, int ph, cudaStream_t cst,
                std::shared_ptr<FleetGeom> &out) {
     std::lock_guard<std::mutex> lk(f->mu);
@@ -1394,6 +1484,7 @@ int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, 
     fg->pw = pw;
     fg->ph = ph;
     fg->form = f->form;
+    CVM_TRY(choose_stats(f, dParent, pstride, pw, ph, cst, &fg->stats));
     cudaStream_t st = thread_stream();
     const std::vector<Bucket> buckets =
         f->form != CVM_FORM_EXACT && f->forcedPlan.dftW == 0 ? fast_buckets(f, pw, ph) : f->buckets;
@@ -1404,7 +1495,7 @@ int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, 
         if (f->forcedPlan.dftW > 0)
             plan = f->forcedPlan;
         else
-            CVM_TRY(tune_bucket_plan(f, b, dParent, pstride, pw, ph, cst, &plan));
+            CVM_TRY(tune_bucket_plan(f, b, dParent, pstride, pw, ph, cst, fg->stats, &plan));
         CVM_TRY(make_geom(b.tw, b.th, rwF, rhF, b.th, bg->G, &plan));
         bg->form = effective_form(f->form, bg->G);
         const bool bfast = bg->form != CVM_FORM_EXACT;
@@ -1506,6 +1597,25 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
         }
     }
     const int cnS = f->step;
+    const int cnP = f->step == 4 ? 4 : 1;
+    // Fast-form buckets without regions of interest take den on demand from
+    // the frame's summed-area table (cvm_lines.cu): no statistics kernel, no
+    // den lanes.  The rows need a length that kernel takes, the members an
+    // area the table serves.  (256 templates on 2560x1440, launches in
+    // sequence: statistics 2.72 ms and rows 1.86 ms with the lanes, rows 2.31
+    // ms on demand.)
+    const int stats = f->statsMode >= 0 ? f->statsMode : fg->stats;
+    std::vector<char> satUse(fg->bg.size(), 0);
+    bool anySat = false, anyStatsKernel = false;  // anyStatsKernel: a bucket's every member
+    for (size_t b = 0; b < fg->bg.size(); b++) {
+        const FleetBucketGeom &bg = *fg->bg[b];
+        bool ok = stats != CVM_STATS_KERNEL && bg.form == CVM_FORM_FAST && f->roi.empty();
+        for (int c = 0; c < bg.G.nclass; c++) ok = ok && den_table_rows(bg.G.fc[c]);
+        for (int i : bg.members) ok = ok && den_table_area(f->ms[i]->w, f->ms[i]->h, f->step);
+        satUse[b] = ok;
+        anySat |= ok;
+        anyStatsKernel |= !ok;
+    }
     size_t frameBytes = 0, partBytes = 0, waveBytes = 0;
     std::vector<int> wave(fg->bg.size());
     for (size_t b = 0; b < fg->bg.size(); b++) {
@@ -1515,7 +1625,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
             fb += Arena::bytes(spec_elems(bg.G.fc[c], cnS), sizeof(float2));
             per += bg.memberScratch[c] * sizeof(float2);
         }
-        const size_t lanesPer = (size_t)bg.rwMax * bg.rhMax;
+        const size_t lanesPer = satUse[b] ? 0 : lanes_elems(bg);
         const int nparts = bg.nparts;
         per += lanesPer * sizeof(float2);
         frameBytes = std::max(frameBytes, fb);
@@ -1537,9 +1647,8 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
         waveBytes = std::max(waveBytes, wb);
     }
     // one set of row prefixes for every member (each differences it at its own width)
-    const int cnP = f->step == 4 ? 4 : 1;
     const int hpP = (int)align_up((size_t)pw + 1, 32);
-    const size_t prefixElems = (size_t)(cnP == 4 ? 6 : stat_pitch(cnP)) * ph * hpP;
+    const size_t prefixElems = anyStatsKernel ? (size_t)(cnP == 4 ? 6 : stat_pitch(cnP)) * ph * hpP : 0;
     // and their 16-row block sums (the main block), from which each band of
     // every member's vertical slide starts
     // (u32 sums: 16 rows of a member's squared window sum over the main
@@ -1547,29 +1656,9 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     int twMax = 0;
     for (const Bucket &b : f->buckets) twMax = std::max(twMax, b.tw);
     const size_t prefixRow = (size_t)(cnP == 4 ? 4 : stat_pitch(cnP)) * hpP;
-    // CVM_STATS_EPILOGUE: fast-form buckets without regions of interest take
-    // their window statistics from the frame's summed-area table inside the
-    // inverse-rows epilogue (no statistics kernel, no den written and read
-    // back) when every member's squared window sum can be restored from its
-    // residue modulo 2^32: area * cn * 16256 < 2^32, cn up to the frame's
-    // channels.
-    std::vector<char> satUse(fg->bg.size(), 0);
-    bool anySat = false, anyStatsKernel = false;
-    for (size_t b = 0; b < fg->bg.size(); b++) {
-        const FleetBucketGeom &bg = *fg->bg[b];
-        bool ok = f->statsMode == CVM_STATS_EPILOGUE && bg.form == CVM_FORM_FAST && f->roi.empty() && (f->step == 4 || f->step == 1);
-        for (int i : bg.members) {
-            if (!ok) break;
-            const cvm_matcher *m = f->ms[i];
-            ok = (unsigned long long)m->w * m->h * (unsigned)cnP * 16256ull < (1ull << 32);
-        }
-        satUse[b] = ok;
-        anySat |= ok;
-        anyStatsKernel |= !ok;
-    }
     const size_t alphaRow = cnP == 4 ? (size_t)2 * hpP : 0;
     const size_t satElems = anySat ? (size_t)(ph + 1) * (prefixRow + alphaRow) : 0;
-    const size_t satBlkElems = anySat ? (size_t)((ph + 15) / 16 + 1) * prefixRow : 0;
+    const size_t satBlkElems = anySat ? sat_scratch_elems(ph, hpP, cnP == 4 ? 4 : 2) : 0;
     const bool blkOk = anyStatsKernel && 16ull * (unsigned)twMax * (cnP == 4 ? 3u : 1u) * 65025ull < (1ull << 32);
     const size_t blkElems = blkOk ? prefixRow * (size_t)(ph / 16) : 0;
     const size_t bytes = Arena::bytes(n, sizeof(DevParams)) + Arena::bytes(1, sizeof(DevFrame)) +
@@ -1600,8 +1689,9 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     A.base = static_cast<char *>(buf.p);
     DevParams *P = A.take<DevParams>(n);
     DevFrame *F = A.take<DevFrame>(1);
-    int *counters = A.take<int>((size_t)3 * n);  // per member: finished CTAs, then two words of extrema so far
-    unsigned int *bounds = reinterpret_cast<unsigned int *>(counters + n);
+    // per member two words of extrema so far, then the finished CTAs
+    unsigned int *bounds = A.take<unsigned int>((size_t)3 * n);
+    int *counters = reinterpret_cast<int *>(bounds + 2 * (size_t)n);
     unsigned int *prefix = A.take<unsigned int>(prefixElems);
     unsigned int *prefixBlk = blkElems ? A.take<unsigned int>(blkElems) : nullptr;
     unsigned int *sat = satElems ? A.take<unsigned int>(satElems) : nullptr;
@@ -1628,17 +1718,12 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     } sideJoin{ss, st};
     CVM_CUDA(cudaMemcpyAsync(P, f->dP, n * sizeof(DevParams), cudaMemcpyDeviceToDevice, st));
     CVM_CUDA(cudaMemsetAsync(F, 0, sizeof(DevFrame), st));
-    CVM_CUDA(cudaMemsetAsync(counters, 0, (size_t)3 * n * sizeof(int), st));
+    CVM_CUDA(cudaMemsetAsync(bounds, 0, (size_t)3 * n * sizeof(int), st));
     CVM_CUDA(launch_prep(nullptr, 0, 0, 0, f->step, 0, f->step == 4 ? dParent : nullptr, pstride, pw, ph, P, n, 0, 0,
                          0, F, st));
-    CVM_CUDA(launch_row_prefix(dParent, pstride, f->step, pw, ph, cnP, prefix, hpP, st));
+    if (sat) CVM_CUDA(launch_sat(dParent, pstride, pw, ph, hpP, cnP == 4 ? 4 : 2, &F->cnMax, satBlk, sat, st));
+    if (anyStatsKernel) CVM_CUDA(launch_row_prefix(dParent, pstride, f->step, pw, ph, cnP, prefix, hpP, st));
     if (prefixBlk) CVM_CUDA(launch_vblock(prefix, prefixBlk, ph / 16, prefixRow, st));
-    if (sat) {
-        CVM_CUDA(launch_sat(prefix, ph, prefixRow, satBlk, sat, st));
-        if (alphaRow)  // the (s3, alpha squares) block after the main one, in both
-            CVM_CUDA(launch_sat(prefix + (size_t)ph * prefixRow, ph, alphaRow, satBlk, sat + (size_t)(ph + 1) * prefixRow,
-                                st));
-    }
     for (size_t b = 0; b < fg->bg.size(); b++) {
         const FleetBucketGeom &bg = *fg->bg[b];
         const Geom &G = bg.G;
@@ -1655,7 +1740,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
                 wa.base = waveBase[set];
                 for (int c = 0; c < G.nclass; c++)
                     scratch[set][c] = wa.take<float2>((size_t)wave[b] * bg.memberScratch[c]);
-                lanes[set] = wa.take<float2>((size_t)wave[b] * bg.rwMax * bg.rhMax);
+                if (!satUse[b]) lanes[set] = wa.take<float2>((size_t)wave[b] * lanes_elems(bg));
             }
         }
         // Phase 1: the frame's tile spectra, once per bucket (fleet.go:240-263).
@@ -1675,7 +1760,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
         ms.table = bg.table;
         ms.params = P;
         ms.lanes = lanes[0];
-        ms.lanesStride = (size_t)bg.rwMax * bg.rhMax;
+        ms.lanesStride = lanes_elems(bg);
         ms.anyRoi = !f->roi.empty();
         ms.form = bg.form;
         if (satUse[b]) {

@@ -362,63 +362,115 @@ __device__ __forceinline__ float score_fast(float num, float den, float denFlat)
     return 0.f;
 }
 
-// The fast form's den of the window at result (x, y) of member m, formed
-// from the frame's summed-area table (MemberSet::sat) instead of read from
-// the statistics kernel's lanes.  Four corners give the window's channel
-// sums and its squared sum modulo 2^32; each channel sum is below 2^32,
-// and the squared sum q is restored from its residue as
+// The channel sums s and the squared sum q of the tw x th window at (x, y),
+// from the frame's summed-area table (MemberSet::sat).  Four corners give
+// the channel sums and the squared sum modulo 2^32; each channel sum is
+// below 2^32, and q is restored from its residue as
 //   q = U - ((U - q) mod 2^32),   U = 255 * (sum of the channel sums),
 // exact while U - q = sum over the window's bytes of v (255 - v), at most
-// area * cn * 16256, stays below 2^32 (the host uses the table only
-// then).  The rest is the statistics kernel's fast den sequence on the same
-// integers (vstat_cols, FAST), so den has the same bits.
-__device__ __forceinline__ float sat_den(const MemberSet &ms, const DevMember &m, const DevParams &Pm, int y, int x) {
+// area * cn * 16256, stays below 2^32 (the host uses the table only then).
+struct WinSums {
+    unsigned int s0, s1, s2, s3;
+    unsigned long long q;
+    // area^2 x the variance summed over the channels
+    __device__ __forceinline__ unsigned long long spread(int area) const {
+        return (unsigned long long)area * q -
+               ((unsigned long long)s0 * s0 + (unsigned long long)s1 * s1 + (unsigned long long)s2 * s2 +
+                (unsigned long long)s3 * s3);
+    }
+};
+
+__device__ __forceinline__ WinSums sat_window(const MemberSet &ms, int cn, int y, int x, int tw, int th) {
     const size_t row = ms.satRow;
-    unsigned int s0, s1 = 0u, s2 = 0u, s3 = 0u, qm;
+    WinSums w;
+    unsigned int qm;
+    w.s1 = w.s2 = w.s3 = 0u;
     if (ms.satNp == 4) {
         const unsigned int *r0 = ms.sat + (size_t)y * row + (size_t)x * 4;
-        const unsigned int *r1 = r0 + (size_t)m.th * row;
-        const int dx = 4 * m.tw;
+        const unsigned int *r1 = r0 + (size_t)th * row;
+        const int dx = 4 * tw;
         const uint4 A = __ldg(reinterpret_cast<const uint4 *>(r1 + dx)), B = __ldg(reinterpret_cast<const uint4 *>(r1));
         const uint4 C = __ldg(reinterpret_cast<const uint4 *>(r0 + dx)), D = __ldg(reinterpret_cast<const uint4 *>(r0));
-        s0 = A.x - B.x - C.x + D.x;
-        s1 = A.y - B.y - C.y + D.y;
-        s2 = A.z - B.z - C.z + D.z;
+        w.s0 = A.x - B.x - C.x + D.x;
+        w.s1 = A.y - B.y - C.y + D.y;
+        w.s2 = A.z - B.z - C.z + D.z;
         qm = A.w - B.w - C.w + D.w;
-        if (Pm.cn == 4) {
+        if (cn == 4) {
             // the (s3, alpha squares) block: half the main block's lanes per row
             const size_t arow = row >> 1;
             const unsigned int *a0 = ms.sat + ms.satAlpha + (size_t)y * arow + (size_t)x * 2;
-            const unsigned int *a1 = a0 + (size_t)m.th * arow;
-            const int da = 2 * m.tw;
+            const unsigned int *a1 = a0 + (size_t)th * arow;
+            const int da = 2 * tw;
             const uint2 A2 = __ldg(reinterpret_cast<const uint2 *>(a1 + da)), B2 = __ldg(reinterpret_cast<const uint2 *>(a1));
             const uint2 C2 = __ldg(reinterpret_cast<const uint2 *>(a0 + da)), D2 = __ldg(reinterpret_cast<const uint2 *>(a0));
-            s3 = A2.x - B2.x - C2.x + D2.x;
+            w.s3 = A2.x - B2.x - C2.x + D2.x;
             qm += A2.y - B2.y - C2.y + D2.y;
         }
     } else {
         const unsigned int *r0 = ms.sat + (size_t)y * row + (size_t)x * 2;
-        const unsigned int *r1 = r0 + (size_t)m.th * row;
-        const int dx = 2 * m.tw;
+        const unsigned int *r1 = r0 + (size_t)th * row;
+        const int dx = 2 * tw;
         const uint2 A = __ldg(reinterpret_cast<const uint2 *>(r1 + dx)), B = __ldg(reinterpret_cast<const uint2 *>(r1));
         const uint2 C = __ldg(reinterpret_cast<const uint2 *>(r0 + dx)), D = __ldg(reinterpret_cast<const uint2 *>(r0));
-        s0 = A.x - B.x - C.x + D.x;
+        w.s0 = A.x - B.x - C.x + D.x;
         qm = A.y - B.y - C.y + D.y;
     }
-    const unsigned long long U = 255ull * ((unsigned long long)s0 + s1 + s2 + s3);
-    const unsigned long long q = U - (unsigned int)((unsigned int)U - qm);
-    const unsigned long long sq = (unsigned long long)s0 * s0 + (unsigned long long)s1 * s1 +
-                                  (unsigned long long)s2 * s2 + (unsigned long long)s3 * s3;
-    const unsigned long long idv = (unsigned long long)m.tw * m.th * q - sq;
+    const unsigned long long U = 255ull * ((unsigned long long)w.s0 + w.s1 + w.s2 + w.s3);
+    w.q = U - (unsigned int)((unsigned int)U - qm);
+    return w;
+}
+
+// The fast form's den of the window at result (x, y) of member m, formed
+// from the summed-area table instead of read from the statistics kernel's
+// lanes: that kernel's den sequence on the same integers (vstat_cols, FAST),
+// so the same bits.
+__device__ __forceinline__ float sat_den(const MemberSet &ms, const DevMember &m, const DevParams &Pm, int y, int x) {
+    const WinSums w = sat_window(ms, Pm.cn, y, x, m.tw, m.th);
+    const unsigned long long idv = w.spread(m.tw * m.th);
     const float id = fmaf(__uint2float_rn((unsigned int)(idv >> 32)), 4294967296.0f, __uint2float_rn((unsigned int)idv));
     const float diff2 = __fmul_rn(id, Pm.varScale);
     float lim = 0.5f;
-    if (q < (1ull << 24)) {
-        lim = __fmul_rn(1.1920928955078125e-06f, __uint2float_rn((unsigned int)q));  // 10 * 2^-23 * q
+    if (w.q < (1ull << 24)) {
+        lim = __fmul_rn(1.1920928955078125e-06f, __uint2float_rn((unsigned int)w.q));  // 10 * 2^-23 * q
         if (lim > 0.5f) lim = 0.5f;
     }
     const float sd = __fmul_rn(diff2, rsqrtf(diff2));
     return diff2 > lim ? __fmul_rn(sd, Pm.templNorm) : 0.f;
+}
+
+// Den on demand.  A fleet's extrema need the den of few windows: a result is
+// out of the running when num < hi * lb and num > lo * lb for any lower
+// bound 0 < lb <= den (hi > 0 > lo, the cuts just inside the known extrema).
+// den is bounded over blocks of results: every window of a block contains
+// the intersection of them all, and a window's sum of squared deviations is
+// at least that of any part of it (its own mean minimises the part's).  So
+// lb = sqrt(deviations of the intersection) * templNorm, from four corners of
+// the frame's summed-area table per block, less 2^-11 for the roundings of
+// both sides, and 0 unless it exceeds the guard below which den may be 0 (lim
+// <= 0.5).  Windows whose union has no deviation at all have den = 0, hence
+// the score 0: never an extremum between lo < 0 < hi, and lb is infinite.
+// Any other result forms its window's den from the table (sat_den, the
+// statistics kernel's bits) and takes the ladder as ever.
+// log2 of the block's side along an axis of the window: the intersection
+// keeps most of the window, and blocks are few beside the results.
+__device__ __forceinline__ int block_log2(int side) { return side >= 64 ? 4 : (side >= 32 ? 3 : 2); }
+
+// lb of the block of cw x ch results at frame position (x, y).
+__device__ __forceinline__ float block_bound(const MemberSet &ms, const DevMember &m, const DevParams &Pm, int y, int x,
+                                          int cw, int ch) {
+    const int w = m.tw - cw + 1, h = m.th - ch + 1;
+    bool none = true;
+    if (w > 0 && h > 0) {
+        const unsigned long long v = sat_window(ms, Pm.cn, y + ch - 1, x + cw - 1, w, h).spread(w * h);
+        none = v == 0ull;
+        const float dev = __ull2float_rn(v) / (float)(w * h) * 0.9995f;
+        if (dev > 0.51f) return sqrtf(dev) * Pm.templNorm * 0.9995f;
+    }
+    if (none) {
+        const int uw = m.tw + cw - 1, uh = m.th + ch - 1;
+        if (sat_window(ms, Pm.cn, y, x, uw, uh).spread(uw * uh) == 0ull) return INFINITY;
+    }
+    return 0.f;
 }
 
 // Padded shared-memory line layout: one spare slot every 16 elements keeps

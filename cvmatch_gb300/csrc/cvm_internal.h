@@ -118,9 +118,9 @@ struct MemberSet {
     int form;
     // Fast-form fleet waves without score maps or regions of interest: the
     // frame's summed-area table of the shared row prefix (ih + 1 rows, the
-    // prefix's lanes; all sums modulo 2^32), from which the inverse-rows
-    // epilogue forms every window's statistics itself instead of reading
-    // den from `lanes` (nullptr: the statistics kernel filled `lanes`).
+    // prefix's lanes; all sums modulo 2^32), from which the inverse rows form
+    // the den of the windows that may be extrema (nullptr: the statistics
+    // kernel filled `lanes`).
     const unsigned int *sat;
     size_t satRow;     // u32 per row of the main block (satNp * hp)
     size_t satAlpha;   // u32 offset of the (s3, alpha squares) block; 0: none
@@ -190,6 +190,8 @@ cudaError_t launch_inv_rows(const TileGeom &g, const FftClass &fc, int cls, int 
 // point's)
 int inv_rows_ctas_per_tile(const FftClass &fc, int rowsMax, int *pairsPerCta, int wide, int tc, int members,
                            int lanes = 1);
+// True when the inverse rows of fc can take den from the summed-area table.
+bool den_table_rows(const FftClass &fc);
 // Normalisation + first-occurrence extrema: CW x B results per CTA, ncx x
 // nby CTAs per member, result rows in groups of G; the member's last CTA
 // writes its result to out[outIdx].  counters (one int per member of the
@@ -242,11 +244,18 @@ cudaError_t launch_vblock(const unsigned int *H, unsigned int *B, int nblk, size
 // launch_sep_stats with sharedPrefix reads it with cnMax == cnP.
 cudaError_t launch_row_prefix(const uint8_t *img, long long istride, int step, int iw, int ih, int cnP,
                               unsigned int *P, int hp, cudaStream_t st);
-// Summed-area table of `rows` rows of rowElems u32 lanes (one block of the
-// row prefix): S[y][e] = sum_{r<y} P[r][e], y = 0..rows, modulo 2^32.
-// B: scratch of ((rows + 15) / 16 + 1) * rowElems u32.
-cudaError_t launch_sat(const unsigned int *P, int rows, size_t rowElems, unsigned int *B, unsigned int *S,
-                       cudaStream_t st);
+// Summed-area table of the frame, np = 4 (RGBA; the second block, (s3, alpha
+// squares), at S + (ih + 1) * hp * 4, written when *cnMax == 4) or 2 (gray)
+// lanes per x, rows of hp >= iw + 1 columns, ih + 1 rows; modulo 2^32.
+// B: scratch of sat_scratch_elems u32.
+size_t sat_scratch_elems(int ih, int hp, int np);
+cudaError_t launch_sat(const uint8_t *img, long long istride, int iw, int ih, int hp, int np, const int *cnMax,
+                       unsigned int *B, unsigned int *S, cudaStream_t st);
+
+// Adds to *poor how many of 256 sampled blocks of each member's results (the
+// table's first nmembers) have no lower bound of den from the summed-area
+// table ms.sat.
+cudaError_t launch_den_poor(const MemberSet &ms, int nmembers, int *poor, cudaStream_t st);
 
 // Stores small host values into device memory through kernel arguments
 // (stream ordered, no host buffer lifetime to manage).

@@ -1563,62 +1563,268 @@ __global__ void k_vblock(const unsigned int *__restrict__ H, unsigned int *__res
     B[(size_t)b * rowElems + e] = sum;
 }
 
-// The frame's summed-area table over the shared row prefix's lanes,
-// S[y][e] = sum_{r < y} P[r][e] for y = 0 .. rows (u32, modulo 2^32 like
-// the prefix), in three steps: 16-row block sums, their exclusive scan down
-// each lane (the total in block nb), then each block's rows from its start.
-__global__ void k_sat_blocks(const unsigned int *__restrict__ P, int rows, size_t rowElems,
-                             unsigned int *__restrict__ B) {
-    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= rowElems) return;
-    const int r0 = 16 * blockIdx.y, n = min(16, rows - r0);
-    const unsigned int *p = P + (size_t)r0 * rowElems + e;
-    unsigned int v[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = i < n ? __ldg(p + (size_t)i * rowElems) : 0u;
-    unsigned int sum = 0u;
-#pragma unroll
-    for (int i = 0; i < 16; i++) sum += v[i];
-    B[(size_t)blockIdx.y * rowElems + e] = sum;
+// The frame's summed-area table, S[y][x] = the sums over rows < y and
+// columns < x (y = 0 .. ih, x = 0 .. iw; u32, modulo 2^32): per x the four
+// lanes (s0, s1, s2, RGB squares) of an RGBA frame and, in a second block
+// written only when some target has four channels (*cnMax == 4), (s3, alpha
+// squares); (s, squares) of a gray frame.  Three steps: column sums of
+// kSatRows-row blocks, their exclusive scan down each column, and each
+// block's rows, in which every warp scans its span of columns.  The frame is
+// read twice and the table written once: 59 MB of table at 2560x1440 in 7 + 10
+// + 32 us (through the row prefix, written and then read twice: 37 + 71).
+// kSatRows: with eight rows a CTA holds more sums than registers and half as
+// many CTAs wait on each other's loads (87 us for the last step).
+constexpr int kSatRows = 4;
+constexpr int kSatThreads = 256;
+
+struct SatArgs {
+    const uint8_t *img;
+    long long istride;
+    int iw, ih, hp, nb;
+    int pix32, pix128;        // RGBA pixels readable as aligned 32-bit words, four as 16 bytes
+    const int *cnMax;         // RGBA: 4 when the alpha block is wanted
+    unsigned int *B, *Ba;     // block column sums: [nb][hp][NP], [nb][hp][2]
+    unsigned int *S, *Sa;     // the table: [ih + 1][hp][NP], [ih + 1][hp][2]
+};
+
+// Pixel x of a row as one word (RGBA: its four bytes; gray: one).
+template <int NP>
+__device__ __forceinline__ unsigned int sat_word(const SatArgs &a, const uint8_t *row, int x) {
+    if constexpr (NP == 4) {
+        const uint8_t *p = row + 4LL * x;
+        if (a.pix32) return __ldg(reinterpret_cast<const unsigned int *>(p));
+        return p[0] | (unsigned int)p[1] << 8 | (unsigned int)p[2] << 16 | (unsigned int)p[3] << 24;
+    } else {
+        return row[x];
+    }
 }
 
-__global__ void k_sat_scan(unsigned int *B, int nb, size_t rowElems) {
-    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= rowElems) return;
+// A pixel word's lanes: v[0 .. NP) and the alpha block's w[0 .. 2).
+template <int NP>
+__device__ __forceinline__ void sat_lanes(unsigned int c, unsigned int *v, unsigned int *w) {
+    if constexpr (NP == 4) {
+        const unsigned int r = c & 255u, g = (c >> 8) & 255u, b = (c >> 16) & 255u, a = c >> 24;
+        v[0] = r;
+        v[1] = g;
+        v[2] = b;
+        v[3] = r * r + g * g + b * b;
+        w[0] = a;
+        w[1] = a * a;
+    } else {
+        v[0] = c;
+        v[1] = c * c;
+    }
+}
+
+template <int NP>
+__global__ void __launch_bounds__(256) k_sat_cols(SatArgs a) {
+    const int x = blockIdx.x * 256 + threadIdx.x, y0 = blockIdx.y * kSatRows;
+    if (x >= a.iw) return;
+    unsigned int v[NP] = {}, w[2] = {}, c[kSatRows];
+#pragma unroll
+    for (int r = 0; r < kSatRows; r++)
+        c[r] = y0 + r < a.ih ? sat_word<NP>(a, a.img + (long long)(y0 + r) * a.istride, x) : 0u;
+#pragma unroll
+    for (int r = 0; r < kSatRows; r++) {
+        unsigned int pv[NP], pw[2] = {0u, 0u};
+        sat_lanes<NP>(c[r], pv, pw);
+#pragma unroll
+        for (int q = 0; q < NP; q++) v[q] += pv[q];
+        w[0] += pw[0];
+        w[1] += pw[1];
+    }
+    const size_t e = (size_t)blockIdx.y * a.hp + x;
+    stv<NP>(a.B + e * NP, v);
+    if (NP == 4 && *a.cnMax == 4) stv<2>(a.Ba + e * 2, w);
+}
+
+// Exclusive scan of a lane (pitch elements a block) over the nb blocks by
+// eight threads (seg = 0 .. 7), an eighth of the blocks each: every eighth's
+// total first, then its blocks from its start.
+__device__ __forceinline__ void sat_scan_lane(unsigned int *B, int nb, size_t pitch, bool in, int col, int seg,
+                                              unsigned int (*part)[32]) {
+    const int per = (nb + 7) / 8, b1 = min(nb, (seg + 1) * per);
     unsigned int run = 0u;
-    for (int b0 = 0; b0 < nb; b0 += 8) {
-        unsigned int v[8];
+    for (int pass = 0; pass < 2; pass++) {
+        if (in)
+            for (int b0 = seg * per; b0 < b1; b0 += 16) {
+                unsigned int v[16];
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = b0 + i < nb ? B[(size_t)(b0 + i) * rowElems + e] : 0u;
+                for (int i = 0; i < 16; i++) v[i] = b0 + i < b1 ? B[(size_t)(b0 + i) * pitch] : 0u;
 #pragma unroll
-        for (int i = 0; i < 8; i++)
-            if (b0 + i < nb) {
-                B[(size_t)(b0 + i) * rowElems + e] = run;
-                run += v[i];
+                for (int i = 0; i < 16; i++) {
+                    if (pass == 1 && b0 + i < b1) B[(size_t)(b0 + i) * pitch] = run;
+                    run += v[i];
+                }
+            }
+        if (pass == 1) break;
+        part[seg][col] = run;
+        __syncthreads();
+        run = 0u;
+        for (int q = 0; q < seg; q++) run += part[q][col];
+        __syncthreads();
+    }
+}
+
+template <int NP>
+__global__ void __launch_bounds__(256) k_sat_scan(SatArgs a) {
+    __shared__ unsigned int part[8][32];
+    const int col = threadIdx.x & 31, seg = threadIdx.x >> 5, e = blockIdx.x * 32 + col;
+    sat_scan_lane(a.B + e, a.nb, (size_t)a.hp * NP, e < a.iw * NP, col, seg, part);
+    if (NP == 4 && *a.cnMax == 4 && blockIdx.x * 32 < a.iw * 2)
+        sat_scan_lane(a.Ba + e, a.nb, (size_t)a.hp * 2, e < a.iw * 2, col, seg, part);
+}
+
+// The lanes of the table's main block (or alpha block, ALPHA) for block
+// blockIdx.x's rows.  "Row" 0 of the scans is the block's column start.  A
+// thread holds four adjacent columns, so one warp scan serves 128.
+template <int NP, bool ALPHA>
+__device__ __forceinline__ void sat_block(const SatArgs &a, unsigned int (*tot)[kSatThreads / 32][4]) {
+    constexpr int NL = ALPHA ? 2 : NP, NR = kSatRows + 1, NW = kSatThreads / 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int y0 = blockIdx.x * kSatRows;
+    // x = iw (all zero lanes) included: its exclusive sums are the totals
+    const int span = ((a.iw + 1 + NW - 1) / NW + 127) & ~127, c0 = warp * span, c1 = min(a.iw + 1, c0 + span);
+    const unsigned int *B = (ALPHA ? a.Ba : a.B) + (size_t)blockIdx.x * a.hp * NL;
+    unsigned int *S = ALPHA ? a.Sa : a.S;
+    // the block's rows at the thread's columns x .. x + 3, all in flight
+    auto words = [&](int x, unsigned int (*c)[4]) {
+#pragma unroll
+        for (int r = 0; r < kSatRows; r++) {
+            const uint8_t *row = a.img + (long long)(y0 + r) * a.istride;
+            const bool in = y0 + r < a.ih;
+            if (NP == 4 && a.pix128 && in && x + 3 < a.iw) {
+                const uint4 t = __ldg(reinterpret_cast<const uint4 *>(row + 4LL * x));
+                c[r][0] = t.x;
+                c[r][1] = t.y;
+                c[r][2] = t.z;
+                c[r][3] = t.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++) c[r][i] = in && x + i < a.iw ? sat_word<NP>(a, row, x + i) : 0u;
+            }
+        }
+    };
+    auto start = [&](int x, unsigned int (*v)[NL]) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (x + i < a.iw) {
+                ldv<NL>(v[i], B + (size_t)(x + i) * NL);
+            } else {
+#pragma unroll
+                for (int q = 0; q < NL; q++) v[i][q] = 0u;
+            }
+    };
+    auto pick = [&](unsigned int c, unsigned int *v) {
+        unsigned int pv[NP], pw[2] = {0u, 0u};
+        sat_lanes<NP>(c, pv, pw);
+#pragma unroll
+        for (int q = 0; q < NL; q++) v[q] = ALPHA ? pw[q] : pv[q];
+    };
+    // 1. every row's total over the warp's span
+    unsigned int carry[NR][NL];
+#pragma unroll
+    for (int r = 0; r < NR; r++)
+#pragma unroll
+        for (int q = 0; q < NL; q++) carry[r][q] = 0u;
+    for (int g = c0; g < c1; g += 128) {
+        unsigned int c[kSatRows][4], v[4][NL];
+        start(g + 4 * lane, v);
+        words(g + 4 * lane, c);
+#pragma unroll
+        for (int q = 0; q < NL; q++) carry[0][q] += v[0][q] + v[1][q] + v[2][q] + v[3][q];
+#pragma unroll
+        for (int r = 0; r < kSatRows; r++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                unsigned int t[NL];
+                pick(c[r][i], t);
+#pragma unroll
+                for (int q = 0; q < NL; q++) carry[r + 1][q] += t[q];
             }
     }
-    B[(size_t)nb * rowElems + e] = run;
+#pragma unroll
+    for (int r = 0; r < NR; r++)
+#pragma unroll
+        for (int q = 0; q < NL; q++) {
+            const unsigned int t = __reduce_add_sync(0xffffffffu, carry[r][q]);
+            if (lane == 0) tot[r][warp][q] = t;
+        }
+    __syncthreads();
+    // 2. the sums left of the span
+#pragma unroll
+    for (int r = 0; r < NR; r++)
+#pragma unroll
+        for (int q = 0; q < NL; q++)
+            carry[r][q] = __reduce_add_sync(0xffffffffu, lane < warp ? tot[r][lane][q] : 0u);
+    // 3. the span, 128 columns at a time, running down the block's rows
+    for (int g = c0; g < c1; g += 128) {
+        const int x = g + 4 * lane;
+        unsigned int c[kSatRows][4], s[4][NL], v[4][NL];
+        start(x, v);
+        words(x, c);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int q = 0; q < NL; q++) s[i][q] = 0u;
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            unsigned int left[NL];
+            if (r > 0) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) pick(c[r > 0 ? r - 1 : 0][i], v[i]);
+            }
+#pragma unroll
+            for (int q = 0; q < NL; q++) {
+                const unsigned int own = v[0][q] + v[1][q] + v[2][q] + v[3][q];
+                unsigned int t = own;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned int u = __shfl_up_sync(0xffffffffu, t, o);
+                    if (lane >= o) t += u;
+                }
+                left[q] = carry[r][q] + t - own;
+                carry[r][q] += __shfl_sync(0xffffffffu, t, 31);
+            }
+            const bool store = y0 + r <= a.ih && (r < kSatRows || y0 + r == a.ih);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+#pragma unroll
+                for (int q = 0; q < NL; q++) {
+                    s[i][q] += left[q];
+                    left[q] += v[i][q];
+                }
+                if (store && x + i <= a.iw) stv<NL>(S + ((size_t)(y0 + r) * a.hp + x + i) * NL, s[i]);
+            }
+        }
+    }
 }
 
-__global__ void k_sat_fill(const unsigned int *__restrict__ P, int rows, size_t rowElems,
-                           const unsigned int *__restrict__ B, unsigned int *__restrict__ S) {
-    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= rowElems) return;
-    const int r0 = 16 * blockIdx.y;
-    if (r0 > rows) return;
-    const int n = min(16, rows - r0);  // prefix rows added inside this block
-    const unsigned int *p = P + (size_t)r0 * rowElems + e;
-    unsigned int v[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = i < n ? __ldg(p + (size_t)i * rowElems) : 0u;
-    unsigned int run = B[(size_t)blockIdx.y * rowElems + e];
-    unsigned int *s = S + (size_t)r0 * rowElems + e;
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        if (r0 + i > rows) break;
-        s[(size_t)i * rowElems] = run;
-        run += v[i];
-    }
+template <int NP>
+__global__ void __launch_bounds__(kSatThreads, 3) k_sat_rows(SatArgs a) {
+    __shared__ unsigned int tot[kSatRows + 1][kSatThreads / 32][4];
+    sat_block<NP, false>(a, tot);
+    if constexpr (NP == 4)
+        if (*a.cnMax == 4) {
+            __syncthreads();
+            sat_block<NP, true>(a, tot);
+        }
+}
+
+// How well do blocks of a member's results bound den (block_bound)?  One CTA
+// per member tries 256 blocks spread over its results and adds those without
+// a bound to *poor.
+__global__ void __launch_bounds__(256) k_den_poor(const __grid_constant__ MemberSet ms, int *poor) {
+    const DevMember &m = ms.table[blockIdx.x];
+    const DevParams &Pm = ms.params[m.pIdx];
+    if (Pm.flat) return;
+    const int lx = block_log2(m.tw), ly = block_log2(m.th);
+    const int nbx = (m.rw + (1 << lx) - 1) >> lx, nby = (m.rh + (1 << ly) - 1) >> ly;
+    const int x = (int)((2 * (threadIdx.x & 15) + 1) * (long long)nbx / 32) << lx;
+    const int y = (int)((2 * (threadIdx.x >> 4) + 1) * (long long)nby / 32) << ly;
+    const float lb = block_bound(ms, m, Pm, y, x, min(1 << lx, m.rw - x), min(1 << ly, m.rh - y));
+    const int n = __syncthreads_count(lb == 0.f);
+    if (threadIdx.x == 0) atomicAdd(poor, n);
 }
 
 // PRE: H is the shared row prefix built for PCN channels (window sum =
@@ -2062,6 +2268,8 @@ cudaError_t launch_cols(int mode, const float2 *in, float2 *out, int cnS, const 
     return cudaGetLastError();
 }
 
+bool den_table_rows(const FftClass &fc) { return inv_lines_length(fc.log2n); }
+
 int inv_rows_ctas_per_tile(const FftClass &fc, int rowsMax, int *pairsPerCta, int wide, int tc, int members, int lanes) {
     // 4096 elements per CTA: the radix-16 passes (n/16 units per line) keep
     // all 256 threads busy, ~68 KB of shared memory (three CTAs per SM);
@@ -2104,7 +2312,8 @@ cudaError_t launch_inv_rows(const TileGeom &g, const FftClass &fc, int cls, int 
     int P = 0;
     if (wide && (!ms.form || !rows_fixed_length(fc.log2n))) return cudaErrorInvalidValue;
     const bool tc = inv_rows_tc_applies(fc, ms);
-    const int ctas = inv_rows_ctas_per_tile(fc, rowsMax, &P, wide, tc, membersAll, ms.lanes != nullptr);
+    const int ctas = inv_rows_ctas_per_tile(fc, rowsMax, &P, wide, tc, membersAll,
+                                            ms.lanes != nullptr || ms.sat != nullptr);
     a.pairsPerCta = P;
     a.partOffset = partOffset;
     a.nparts = nparts;
@@ -2121,7 +2330,7 @@ cudaError_t launch_inv_rows(const TileGeom &g, const FftClass &fc, int cls, int 
     }
     const size_t smem = (size_t)P * (padded_len(fc.n) * sizeof(float2) + (wide ? 0 : 2 * fc.n * sizeof(float)));
     ProfScope ps("k_inv_rows", st);
-    if (inv_lines_length(fc.log2n) && ms.lanes) {
+    if (inv_lines_length(fc.log2n) && (ms.lanes || ms.sat)) {
         launch_inv_lines(a, dim3(nmembers, ctas, fc.ntiles), st);
     } else if (rows_fixed_length(fc.log2n)) {
         launch_inv_rows_fixed(a, grid, smem, st);
@@ -2357,16 +2566,45 @@ cudaError_t launch_vblock(const unsigned int *H, unsigned int *B, int nblk, size
     return cudaGetLastError();
 }
 
-cudaError_t launch_sat(const unsigned int *P, int rows, size_t rowElems, unsigned int *B, unsigned int *S,
-                       cudaStream_t st) {
-    if (rows <= 0 || rowElems == 0) return cudaSuccess;
-    const int nb = (rows + 15) / 16;
-    const unsigned gx = (unsigned)((rowElems + kThreads - 1) / kThreads);
+size_t sat_scratch_elems(int ih, int hp, int np) {
+    return (size_t)((ih + kSatRows - 1) / kSatRows) * hp * (np == 4 ? 6 : 2);
+}
+
+cudaError_t launch_sat(const uint8_t *img, long long istride, int iw, int ih, int hp, int np, const int *cnMax,
+                       unsigned int *B, unsigned int *S, cudaStream_t st) {
+    SatArgs a;
+    a.img = img;
+    a.istride = istride;
+    a.iw = iw;
+    a.ih = ih;
+    a.hp = hp;
+    a.nb = (ih + kSatRows - 1) / kSatRows;
+    a.pix32 = ((reinterpret_cast<uintptr_t>(img) | (uintptr_t)istride) & 3) == 0;
+    a.pix128 = ((reinterpret_cast<uintptr_t>(img) | (uintptr_t)istride) & 15) == 0;
+    a.cnMax = cnMax;
+    a.B = B;
+    a.Ba = np == 4 ? B + (size_t)a.nb * hp * 4 : nullptr;
+    a.S = S;
+    a.Sa = np == 4 ? S + (size_t)(ih + 1) * hp * 4 : nullptr;
+    const dim3 gc((iw + 255) / 256, a.nb);
+    const int gs = (iw * np + 31) / 32;
     ProfScope ps("k_sat", st);
-    k_sat_blocks<<<dim3(gx, nb), kThreads, 0, st>>>(P, rows, rowElems, B);
-    k_sat_scan<<<gx, kThreads, 0, st>>>(B, nb, rowElems);
-    k_sat_fill<<<dim3(gx, nb + 1), kThreads, 0, st>>>(P, rows, rowElems, B, S);
+    if (np == 4) {
+        k_sat_cols<4><<<gc, 256, 0, st>>>(a);
+        k_sat_scan<4><<<gs, 256, 0, st>>>(a);
+        k_sat_rows<4><<<a.nb, kSatThreads, 0, st>>>(a);
+    } else {
+        k_sat_cols<2><<<gc, 256, 0, st>>>(a);
+        k_sat_scan<2><<<gs, 256, 0, st>>>(a);
+        k_sat_rows<2><<<a.nb, kSatThreads, 0, st>>>(a);
+    }
     count_launches(3);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_den_poor(const MemberSet &ms, int nmembers, int *poor, cudaStream_t st) {
+    k_den_poor<<<nmembers, 256, 0, st>>>(ms, poor);
+    count_launches(1);
     return cudaGetLastError();
 }
 

@@ -56,12 +56,12 @@ __device__ __forceinline__ float from_key(unsigned int k) {
 // Only the extrema leave a match without a score map, so a result that
 // cannot be one needs no quotient: scores outside (lo, hi) may be extrema.
 // hi lies below the largest known score by 2^-20 of it and 1e-15: num < hi *
-// den then implies that the computed quotient (within 2 ulp, 2^-22) is below
-// that score, the product's rounding (2^-24, or 1e-45 where it underflows:
-// den >= kCutDen) included, and, scores being at most 1 (+ 2 ulp), that num <
-// den.  lo is its mirror.  A result at or above the cut, ties included,
-// takes the whole ladder.
-constexpr float kCutDen = 1e-20f;
+// den then implies that the computed quotient (within 2 ulp, 2^-22; near-flat
+// windows' within half of one) is below that score, the product's rounding
+// included (2^-24: a den is 0 or above 1e-6, since idiff / area exceeds its
+// guard), and, scores being at most 1 (+ 2 ulp), that num < den.  lo is its
+// mirror.  A result at or above the cut, ties included, takes the whole
+// ladder.
 __device__ __forceinline__ float below(float v) { return v - (fabsf(v) * 9.5367431640625e-07f + 1e-15f); }
 __device__ __forceinline__ float above(float v) { return v + (fabsf(v) * 9.5367431640625e-07f + 1e-15f); }
 
@@ -103,9 +103,7 @@ __device__ __forceinline__ void cut_share(Track &t, unsigned int mask) {
 
 // The cuts from the extrema (keys of the maximum and of the negated minimum)
 // of the member's CTAs that have finished; false when there are none.
-__device__ __forceinline__ bool cut_load(Track &t, const unsigned int *b) {
-    const unsigned int kx = *reinterpret_cast<const volatile unsigned int *>(b);
-    const unsigned int kn = *reinterpret_cast<const volatile unsigned int *>(b + 1);
+__device__ __forceinline__ bool cut_keys(Track &t, unsigned int kx, unsigned int kn) {
     if (kx) t.hi = fmaxf(t.hi, below(from_key(kx)));
     if (kn) t.lo = fminf(t.lo, above(-from_key(kn)));
     return kx != 0u && kn != 0u;
@@ -123,9 +121,20 @@ __device__ __forceinline__ float2 ld_once(const float2 *p) {
     return v;
 }
 
-// Out of line: the option's code stays out of the loads' way.
-__device__ __noinline__ float sat_den_call(const MemberSet &ms, const DevMember &m, const DevParams &Pm, int y, int x) {
-    return sat_den(ms, m, Pm, y, x);
+
+constexpr int kBlocksMax = 1024;  // of a CTA: 8192 results over two rows a pair, in 4 x 4 blocks
+
+// A result above its block's bound: its den, and the ladder unless that
+// already rules it out.
+__device__ __noinline__ Track score_table(Track t, float num, const MemberSet &ms, const DevMember &m,
+                                          const DevParams &Pm, int y, int x, float denFlat, int l) {
+    const float d = sat_den(ms, m, Pm, y, x);
+    if (d > 0.f && num < t.hi * d && num > t.lo * d) return t;
+    const float sc = score_fast(num, d, denFlat);
+    track(t, sc, l);
+    t.hi = fmaxf(t.hi, below(sc));
+    t.lo = fminf(t.lo, above(sc));
+    return t;
 }
 
 template <int L>
@@ -142,7 +151,7 @@ struct Lines {
     static constexpr int G = N / 16;                      // threads of a line
     static constexpr int CTA = G > 64 ? G : 64;
     static constexpr int NL = CTA / G;                    // lines of a CTA at a time
-    static constexpr size_t SMEM = (size_t)NL * LINE * sizeof(float2);
+    static constexpr size_t SMEM = (size_t)NL * LINE * sizeof(float2);  // + TABLE's bounds
 };
 
 // The barrier of a line's threads: the CTA (one line at a time) or the
@@ -160,31 +169,295 @@ __device__ __forceinline__ void group_sync(unsigned int mask) {
 // 2.01 ms; without them 14 CTAs 2.00 at the same 4096 elements per CTA); the
 // exact form keeps the channel sum of its 16 results, 128 registers (nine
 // CTAs spill: 1.17 against 0.84 ms).
-__host__ __device__ constexpr int lines_ctas(int L, bool fast, bool lean) {
-    return (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 7) : (fast ? 10 : 8))) * (lean ? 4 : 3) / 4;
+__host__ __device__ constexpr int lines_ctas(int L, bool fast, int mode) {
+    return mode == 2 ? (L == 11 ? 4 : (L <= 8 ? 8 : 9))
+                     : (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 7) : (fast ? 10 : 8))) * (mode ? 4 : 3) / 4;
 }
 
-// LEAN: the extrema alone leave (no score map, no region of interest, den
-// from the statistics kernel): every Match, Find and fleet FindAll without
-// them.
-template <int L, bool FAST, bool LEAN>
-__global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, LEAN)) k_inv_lines(InvArgs a) {
-    griddep_wait();
+// What a launch keeps of its results.  ALL: every score may be wanted (a
+// score map, regions of interest).  LANES: the extrema alone, den (and t)
+// from the statistics kernel's lanes.  TABLE: a fast-form fleet's extrema,
+// den on demand.
+enum Keep { ALL, LANES, TABLE };
+
+// The extrema (and scores) of the CTA's row pairs.
+template <int L, bool FAST, Keep MODE>
+__device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const DevMember &m, const DevParams &Pm,
+                                          const TileBox &tb, int bw, int bh, int pair0, int P, unsigned int *bnd) {
     using S = Lines<L>;
+    constexpr bool LEAN = MODE != ALL;
     constexpr int N = S::N, R1 = S::R1, K1 = S::K1, NB = S::NB, G = S::G, NL = S::NL, PITCH = S::PITCH;
-        constexpr int NU = NB == 1 ? 1 : 16 / NB;             // last-pass units of a thread
+    constexpr int NU = NB == 1 ? 1 : 16 / NB;             // last-pass units of a thread
     constexpr int RL = NB == 1 ? 16 : NB;                 // their radix
     constexpr int HL = NB == 1 ? S::H2 : S::H3;           // their quarter
     constexpr bool BOTH = RL == 4;                        // both rows' den values in registers at once
-    constexpr bool AHEAD = BOTH && FAST;                  // and every unit's
+    constexpr bool AHEAD = BOTH && FAST && MODE != TABLE;  // and every unit's
+    const FftClass &fc = a.fc;
+    const int slot = blockIdx.x, tileLocal = blockIdx.z, tid = threadIdx.x;
+    Ext e;
+    const int g = tid / G, lt = tid - g * G;          // the thread's group and its place in it
+    const unsigned int mask = G >= 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((tid & 31) / G * G);
+    float2 *ln = smem + (size_t)g * S::LINE;
+    const int hwp = fc.hwp, log2H = fc.log2H;
+    const int cn = FAST ? 1 : Pm.cn;
+    const size_t chanStride = (size_t)fc.dftH * hwp;
+    const float2 *scr = a.ms.scratch[a.cls] + (size_t)slot * a.ms.scratchStride[a.cls] +
+                        (size_t)tileLocal * a.cnS * chanStride;
+    const float2 *lanes = a.ms.lanes + (size_t)slot * a.ms.lanesStride;
+    const float *dens = reinterpret_cast<const float *>(lanes);
+    const float denFlat = near_flat_den(m.tw, m.th, Pm.templNorm);  // fast form: near-flat windows below it
+    float *map = LEAN ? nullptr : a.ms.map;
+    const int rw = m.rw, xlo = m.roiX0 - tb.x0, xhi = m.roiX1 - tb.x0, roiY0 = m.roiY0, roiY1 = m.roiY1;
+    const float2 *triW = fc.triW;
+    bool warm = false;                                // the cuts have been shared once
+    float postV = -FLT_MAX, postN = FLT_MAX;          // TABLE: the extrema the warp has posted
+    float *lbs = reinterpret_cast<float *>(smem + (size_t)NL * S::LINE);
+    int lgx = 0, lgy = 0, nbx = 0;
+    if constexpr (MODE == TABLE) {
+        lgx = block_log2(m.tw);
+        lgy = block_log2(m.th);
+        nbx = (bw + (1 << lgx) - 1) >> lgx;
+        const int rows = min(2 * P, bh - 2 * pair0), n = nbx * ((rows + (1 << lgy) - 1) >> lgy);
+#pragma unroll 1
+        for (int i = tid; i < n; i += S::CTA) {
+            const int by = i / nbx, x = (i - by * nbx) << lgx, y = by << lgy;
+            lbs[i] = block_bound(a.ms, m, Pm, tb.y0 + 2 * pair0 + y, tb.x0 + x, min(1 << lgx, bw - x),
+                                 min(1 << lgy, rows - y));
+        }
+        __syncthreads();
+    }
+    Track t = {FLT_MAX, -FLT_MAX, -INFINITY, INFINITY, INT_MAX, INT_MAX};
+    // rows r and r + 1 of channel k
+    auto row_ptr = [&](int p, int k, int h) {
+        return scr + (size_t)k * chanStride + (size_t)brev_bits(2 * (pair0 + p) + h, log2H) * hwp;
+    };
+    // towards L2, one 128-byte line per thread and step: the two rows
+    // and (last channel) their den
+    auto prefetch = [&](int p, int k) {
+        for (int o = lt; o < 2 * (N / 32 + 1); o += G) {
+            const int h = o > N / 32, c = h ? o - (N / 32 + 1) : o;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(row_ptr(p, k, h) + 16 * c));
+        }
+        if (MODE != TABLE && k == cn - 1) {
+            constexpr int EB = FAST ? 4 : 8;
+            const int r = 2 * (pair0 + p);
+            for (int h = 0; h < 2 && r + h < bh; h++) {
+                const char *q = reinterpret_cast<const char *>(lanes) +
+                                ((long long)(tb.y0 + r + h) * rw + tb.x0) * EB;
+                for (int o = lt * 128; o < bw * EB; o += G * 128)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
+            }
+        }
+    };
+    float2 acc[FAST ? 1 : 16];                        // the earlier channels' sum, the thread's results
+    for (int p = g; p < P; p += NL)
+#pragma unroll 1
+        for (int k = 0; k < cn; k++) {
+            // pass 1: unit k0's elements are Z[k0 + K1 * brev(i)]
+            // (bit-reversed input), Z = U + iV below N/2 and its mirror
+            // above (impl.go:405-413)
+            const float2 *ur = row_ptr(p, k, 0), *vr = row_ptr(p, k, 1);
+            // the member's extrema so far, used at the line's end
+            const bool posted = LEAN && bnd && k == cn - 1 && (MODE == TABLE || p < NL);
+            uint2 keys = make_uint2(0u, 0u);
+            if (posted) {
+                keys.x = *reinterpret_cast<const volatile unsigned int *>(bnd);
+                keys.y = *reinterpret_cast<const volatile unsigned int *>(bnd + 1);
+            }
+#pragma unroll
+            for (int q = 0; q < 16 / R1; q++) {
+                const int k0 = lt + q * G;
+                float2 z[R1];
+                constexpr int LR1 = R1 == 16 ? 4 : 3;
+#pragma unroll
+                for (int i = 0; i < R1 / 2; i++) {
+                    const float2 u = __ldg(ur + k0 + K1 * i), v = __ldg(vr + k0 + K1 * i);
+                    z[brevk(i, LR1)] = make_float2(__fsub_rn(u.x, v.y), __fadd_rn(u.y, v.x));
+                }
+#pragma unroll
+                for (int i = R1 / 2; i < R1; i++) {
+                    const int n = K1 * (R1 - i) - k0;
+                    const float2 u = __ldg(ur + n);
+                    float2 v = __ldg(vr + n);
+                    float uy = u.y;
+                    if (i == R1 / 2 && k0 == 0) {  // N/2 itself: the direct form
+                        uy = -uy;
+                        v.y = -v.y;
+                    }
+                    z[brevk(i, LR1)] = make_float2(__fadd_rn(u.x, v.y), __fsub_rn(v.x, uy));
+                }
+                if constexpr (R1 == 16)
+                    math16<true, 1, FAST>(z, triW);
+                else
+                    math_head<true, FAST>(z, triW);
+                // the previous pair's last pass has read the line
+                if (q == 0) group_sync<G>(mask);
+#pragma unroll
+                for (int i = 0; i < R1; i++) ln[i * PITCH + k0] = z[i];
+            }
+            if (k + 1 < cn || p + NL < P) prefetch(k + 1 < cn ? p : p + NL, k + 1 < cn ? k + 1 : 0);
+            group_sync<G>(mask);
+            float2 z[16];
+            {
+                // pass 2: unit (b, j); lanes run over the blocks first
+                // (NB = 4: even columns, then odd ones, in groups of eight,
+                // keep the half-warps on distinct banks)
+                const int bb = lt & (NB - 1), jl = lt / NB;
+                const int j = NB == 4 ? (jl & 8) | ((jl & 3) << 1) | ((jl >> 2) & 1) : jl;
+                float2 *q = ln + j * PITCH + bb;
+#pragma unroll
+                for (int i = 0; i < 16; i++) z[i] = q[brevk(i, 4) * NB];
+                math16<true, S::H2, FAST>(z, triW + tw_off(L, S::H2) + j);
+                if constexpr (NB > 1) {
+#pragma unroll
+                    for (int i = 0; i < 16; i++) q[i * NB] = z[i];
+                }
+            }
+            const bool last = k == cn - 1;
+            const bool odd = 2 * (pair0 + p) + 1 < bh;  // the imaginary part's row exists
+            const int y0 = tb.y0 + 2 * (pair0 + p);
+            const long long row0 = (long long)y0 * rw + tb.x0;
+            const int blockRow = MODE == TABLE ? ((2 * p) >> lgy) * nbx : 0;  // of both rows
+            // den (and t) of the thread's results, unit it
+            float den[AHEAD ? NU : 1][BOTH ? 2 : 1][RL], tt[BOTH ? 2 : 1][FAST ? 1 : RL];
+            auto load_den = [&](int it, int h) {
+                const int jj = lt + it * G, is = AHEAD ? it : 0, hs = BOTH ? h : 0;
+                const long long row = row0 + h * rw;
+                const int xe = h == 0 || odd ? bw : 0;
+#pragma unroll
+                for (int i = 0; i < RL; i++) {
+                    const int x = jj + HL * i;
+                    if constexpr (MODE == TABLE) {
+                        den[is][hs][i] = lbs[blockRow + (min(x, bw - 1) >> lgx)];  // its bound
+                    } else {
+                        float2 td = make_float2(0.f, 0.f);
+                        if constexpr (FAST)
+                            td.y = x < xe ? ld_once(dens + row + x) : 0.f;
+                        else if (x < xe)
+                            td = ld_once(lanes + row + x);
+                        if constexpr (!FAST) tt[hs][i] = td.x;
+                        den[is][hs][i] = td.y;
+                    }
+                }
+            };
+            if constexpr (AHEAD) {
+                // every unit's, in flight together while the barrier gathers the line
+#pragma unroll
+                for (int it = 0; it < NU; it++) {
+                    load_den(it, 0);
+                    load_den(it, 1);
+                }
+            }
+            if (LEAN && last && posted) warm = cut_keys(t, keys.x, keys.y) || warm;
+            if constexpr (NB > 1) group_sync<G>(mask);
+#pragma unroll
+            for (int it = 0; it < NU; it++) {
+                // last-pass unit jj: results x = jj + HL * i of the two rows
+                const int jj = lt + it * G;
+                if (last && !AHEAD) {
+                    load_den(it, 0);
+                    if (BOTH && MODE != TABLE) load_den(it, 1);
+                }
+                float2 *o = z;
+                float2 zu[NB == 1 ? 1 : RL];
+                if constexpr (NB > 1) {
+                    const float4 *q = reinterpret_cast<const float4 *>(ln + (jj & (R1 - 1)) * PITCH + (jj / R1) * NB);
+#pragma unroll
+                    for (int i = 0; i < NB / 2; i++) {
+                        const float4 w = q[i];
+                        // block b sits at brev(b)
+                        zu[brevk(2 * i, ilog2k(NB))] = make_float2(w.x, w.y);
+                        zu[brevk(2 * i + 1, ilog2k(NB))] = make_float2(w.z, w.w);
+                    }
+                    if constexpr (NB == 16)
+                        math16<true, HL, FAST>(zu, triW + tw_off(L, HL) + jj);
+                    else
+                        math4<true, HL, FAST>(zu, triW + tw_off(L, HL) + jj);
+                    o = zu;
+                }
+                if (!FAST && !last) {
+                    // the channels' sum, in channel order (impl.go:425-443)
+#pragma unroll
+                    for (int i = 0; i < RL; i++) {
+                        float2 &s = acc[FAST ? 0 : it * RL + i];
+                        s = k == 0 ? o[i] : make_float2(__fadd_rn(s.x, o[i].x), __fadd_rn(s.y, o[i].y));
+                    }
+                    continue;
+                }
+                // cuts on either side of 0, or none: a lower bound of den needs
+                // them so, and a zero den is then the score 0 between them
+                const float hp = t.hi > 0.f ? t.hi : -INFINITY, lp = t.lo < 0.f ? t.lo : INFINITY;
+                const float zero = MODE == LANES && t.hi > 0.f && t.lo < 0.f ? 0.f : -1.f;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    if (h == 1 && !odd) break;
+                    if (h == 1 && !BOTH && MODE != TABLE) load_den(it, 1);
+                    const bool rowIn = y0 + h >= roiY0 && y0 + h < roiY1;
+#pragma unroll
+                    for (int i = 0; i < RL; i++) {
+                        const int x = jj + HL * i, l = (2 * p + h) * N + x;
+                        float num = h ? o[i].y : o[i].x;
+                        if constexpr (!FAST) {
+                            const float2 s = acc[it * RL + i];
+                            if (cn > 1) num = __fadd_rn(h ? s.y : s.x, num);
+                            num = __fsub_rn(num, tt[BOTH ? h : 0][i]);
+                        }
+                        const float d = den[AHEAD ? it : 0][BOTH && MODE != TABLE ? h : 0][i];
+                        const bool cand = x < bw && d != zero && !(num < hp * d && num > lp * d);
+                        if constexpr (MODE == TABLE) {
+                            if (cand) t = score_table(t, num, a.ms, m, Pm, y0 + h, tb.x0 + x, denFlat, l);
+                        } else if constexpr (LEAN) {
+                            if (cand) t = score_track<FAST>(t, num, d, denFlat, l);
+                        } else if (x < bw) {
+                            const float sc = FAST ? score_fast(num, d, denFlat) : score_exact(num, d);
+                            if (map) map[row0 + h * rw + x] = sc;
+                            if (rowIn && x >= xlo && x < xhi) track(t, sc, l);
+                        }
+                    }
+                }
+                if (LEAN && it == 0 && !warm) {
+                    cut_share(t, mask);
+                    warm = true;
+                }
+            }
+            // new extrema at once to the member's other CTAs: without a
+            // cut every result forms its den
+            if (MODE == TABLE && __any_sync(mask, t.maxV > postV || t.minV < postN)) {
+                const unsigned int kx = __reduce_max_sync(mask, ordered_key(t.maxV));
+                const unsigned int kn = __reduce_max_sync(mask, ordered_key(-t.minV));
+                postV = from_key(kx);
+                postN = -from_key(kn);
+                t.hi = fmaxf(t.hi, below(postV));
+                t.lo = fminf(t.lo, above(postN));
+                if ((lt & 31) == 0) {
+                    atomicMax(bnd, kx);
+                    atomicMax(bnd + 1, kn);
+                }
+            }
+        }
+    // widen: CTA-local (row, x) -> the member's raster index
+    auto widen = [&](int l) {
+        return l == INT_MAX ? LLONG_MAX
+                            : (long long)(tb.y0 + 2 * pair0 + (l >> L)) * m.rw + tb.x0 + (l & (N - 1));
+    };
+    e.minV = t.minV;
+    e.maxV = t.maxV;
+    e.minI = widen(t.minL);
+    e.maxI = widen(t.maxL);
+    return e;
+}
+
+template <int L, bool FAST, Keep MODE>
+__global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, MODE)) k_inv_lines(const __grid_constant__ InvArgs a) {
+    griddep_wait();
+    using S = Lines<L>;
     extern __shared__ __align__(16) float2 smem[];
     __shared__ Ext shExt[S::CTA / 32];
     __shared__ int isLast;
     const FftClass &fc = a.fc;
     // members vary fastest: a member's CTAs spread over the whole launch, so
     // all but its first start from the extrema of earlier ones (a.bounds)
-    const int slot = blockIdx.x;
-    const int tileLocal = blockIdx.z;
+    const int slot = blockIdx.x, tileLocal = blockIdx.z;
     const int tile = fc.tileFirst + tileLocal;
     const DevMember &m = member_of(a.ms, slot);
     const DevParams &Pm = a.ms.params[m.pIdx];
@@ -196,7 +469,7 @@ __global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, LEAN)) k_in
     // the CTA's row pairs; none when its results all lie outside the
     // member's region of interest (no transform, no extrema)
     int P = 2 * pair0 < bh ? min(a.pairsPerCta, (bh - 2 * pair0 + 1) >> 1) : 0;
-    if (!LEAN && P > 0 && a.ms.anyRoi) {
+    if (MODE == ALL && P > 0 && a.ms.anyRoi) {
         const int ya = tb.y0 + 2 * pair0, yb = tb.y0 + min(2 * (pair0 + P), bh);
         if (ya >= m.roiY1 || yb <= m.roiY0 || tb.x0 >= m.roiX1 || tb.x0 + bw <= m.roiX0) P = 0;
     }
@@ -216,218 +489,7 @@ __global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, LEAN)) k_in
             }
         }
     } else if (P > 0) {
-        const int g = tid / G, lt = tid - g * G;          // the thread's group and its place in it
-        const unsigned int mask = G >= 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((tid & 31) / G * G);
-        float2 *ln = smem + (size_t)g * S::LINE;
-        const int hwp = fc.hwp, log2H = fc.log2H;
-        const int cn = FAST ? 1 : Pm.cn;
-        const size_t chanStride = (size_t)fc.dftH * hwp;
-        const float2 *scr = a.ms.scratch[a.cls] + (size_t)slot * a.ms.scratchStride[a.cls] +
-                            (size_t)tileLocal * a.cnS * chanStride;
-        const float2 *lanes = a.ms.lanes + (size_t)slot * a.ms.lanesStride;
-        const float *dens = reinterpret_cast<const float *>(lanes);
-        const float denFlat = near_flat_den(m.tw, m.th, Pm.templNorm);  // fast form: near-flat windows below it
-        float *map = LEAN ? nullptr : a.ms.map;
-        const float denLow = FAST ? fmaxf(denFlat, kCutDen) : kCutDen;
-        const bool ownStats = FAST && !LEAN && a.ms.sat != nullptr;
-        const int rw = m.rw, xlo = m.roiX0 - tb.x0, xhi = m.roiX1 - tb.x0, roiY0 = m.roiY0, roiY1 = m.roiY1;
-        const float2 *triW = fc.triW;
-        bool warm = false;                                // the cuts have been shared once
-        Track t = {FLT_MAX, -FLT_MAX, -INFINITY, INFINITY, INT_MAX, INT_MAX};
-        // rows r and r + 1 of channel k
-        auto row_ptr = [&](int p, int k, int h) {
-            return scr + (size_t)k * chanStride + (size_t)brev_bits(2 * (pair0 + p) + h, log2H) * hwp;
-        };
-        // towards L2, one 128-byte line per thread and step: the two rows
-        // and (last channel) their den
-        auto prefetch = [&](int p, int k) {
-            for (int o = lt; o < 2 * (N / 32 + 1); o += G) {
-                const int h = o > N / 32, c = h ? o - (N / 32 + 1) : o;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(row_ptr(p, k, h) + 16 * c));
-            }
-            if (k == cn - 1 && !ownStats) {
-                constexpr int EB = FAST ? 4 : 8;
-                const int r = 2 * (pair0 + p);
-                for (int h = 0; h < 2 && r + h < bh; h++) {
-                    const char *q = reinterpret_cast<const char *>(lanes) +
-                                    ((long long)(tb.y0 + r + h) * rw + tb.x0) * EB;
-                    for (int o = lt * 128; o < bw * EB; o += G * 128)
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
-                }
-            }
-        };
-        float2 acc[FAST ? 1 : 16];                        // the earlier channels' sum, the thread's results
-        for (int p = g; p < P; p += NL)
-#pragma unroll 1
-            for (int k = 0; k < cn; k++) {
-                // pass 1: unit k0's elements are Z[k0 + K1 * brev(i)]
-                // (bit-reversed input), Z = U + iV below N/2 and its mirror
-                // above (impl.go:405-413)
-                const float2 *ur = row_ptr(p, k, 0), *vr = row_ptr(p, k, 1);
-#pragma unroll
-                for (int q = 0; q < 16 / R1; q++) {
-                    const int k0 = lt + q * G;
-                    float2 z[R1];
-                    constexpr int LR1 = R1 == 16 ? 4 : 3;
-#pragma unroll
-                    for (int i = 0; i < R1 / 2; i++) {
-                        const float2 u = __ldg(ur + k0 + K1 * i), v = __ldg(vr + k0 + K1 * i);
-                        z[brevk(i, LR1)] = make_float2(__fsub_rn(u.x, v.y), __fadd_rn(u.y, v.x));
-                    }
-#pragma unroll
-                    for (int i = R1 / 2; i < R1; i++) {
-                        const int n = K1 * (R1 - i) - k0;
-                        const float2 u = __ldg(ur + n);
-                        float2 v = __ldg(vr + n);
-                        float uy = u.y;
-                        if (i == R1 / 2 && k0 == 0) {  // N/2 itself: the direct form
-                            uy = -uy;
-                            v.y = -v.y;
-                        }
-                        z[brevk(i, LR1)] = make_float2(__fadd_rn(u.x, v.y), __fsub_rn(v.x, uy));
-                    }
-                    if constexpr (R1 == 16)
-                        math16<true, 1, FAST>(z, triW);
-                    else
-                        math_head<true, FAST>(z, triW);
-                    // the previous pair's last pass has read the line
-                    if (q == 0) group_sync<G>(mask);
-#pragma unroll
-                    for (int i = 0; i < R1; i++) ln[i * PITCH + k0] = z[i];
-                }
-                if (k + 1 < cn || p + NL < P) prefetch(k + 1 < cn ? p : p + NL, k + 1 < cn ? k + 1 : 0);
-                group_sync<G>(mask);
-                float2 z[16];
-                {
-                    // pass 2: unit (b, j); lanes run over the blocks first
-                    // (NB = 4: even columns, then odd ones, in groups of eight,
-                    // keep the half-warps on distinct banks)
-                    const int bb = lt & (NB - 1), jl = lt / NB;
-                    const int j = NB == 4 ? (jl & 8) | ((jl & 3) << 1) | ((jl >> 2) & 1) : jl;
-                    float2 *q = ln + j * PITCH + bb;
-#pragma unroll
-                    for (int i = 0; i < 16; i++) z[i] = q[brevk(i, 4) * NB];
-                    math16<true, S::H2, FAST>(z, triW + tw_off(L, S::H2) + j);
-                    if constexpr (NB > 1) {
-#pragma unroll
-                        for (int i = 0; i < 16; i++) q[i * NB] = z[i];
-                    }
-                }
-                const bool last = k == cn - 1;
-                const bool odd = 2 * (pair0 + p) + 1 < bh;  // the imaginary part's row exists
-                const int y0 = tb.y0 + 2 * (pair0 + p);
-                const long long row0 = (long long)y0 * rw + tb.x0;
-                // den (and t) of the thread's results, unit it
-                float den[AHEAD ? NU : 1][BOTH ? 2 : 1][RL], tt[BOTH ? 2 : 1][FAST ? 1 : RL];
-                auto load_den = [&](int it, int h) {
-                    const int jj = lt + it * G, is = AHEAD ? it : 0, hs = BOTH ? h : 0;
-                    const long long row = row0 + h * rw;
-                    const int xe = h == 0 || odd ? bw : 0;
-                    if (FAST && ownStats) {
-#pragma unroll
-                        for (int i = 0; i < RL; i++) {
-                            const int x = jj + HL * i;
-                            den[is][hs][i] = x < xe ? sat_den_call(a.ms, m, Pm, y0 + h, tb.x0 + x) : 0.f;
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < RL; i++) {
-                            const int x = jj + HL * i;
-                            if constexpr (FAST) {
-                                den[is][hs][i] = x < xe ? ld_once(dens + row + x) : 0.f;
-                            } else {
-                                const float2 td = x < xe ? ld_once(lanes + row + x) : make_float2(0.f, 0.f);
-                                tt[hs][i] = td.x;
-                                den[is][hs][i] = td.y;
-                            }
-                        }
-                    }
-                };
-                if constexpr (AHEAD) {
-                    // every unit's, in flight together while the barrier gathers the line
-#pragma unroll
-                    for (int it = 0; it < NU; it++) {
-                        load_den(it, 0);
-                        load_den(it, 1);
-                    }
-                }
-                if (LEAN && last && p < NL && bnd) warm = cut_load(t, bnd);
-                if constexpr (NB > 1) group_sync<G>(mask);
-#pragma unroll
-                for (int it = 0; it < NU; it++) {
-                    // last-pass unit jj: results x = jj + HL * i of the two rows
-                    const int jj = lt + it * G;
-                    if (last && !AHEAD) {
-                        load_den(it, 0);
-                        if (BOTH) load_den(it, 1);
-                    }
-                    float2 *o = z;
-                    float2 zu[NB == 1 ? 1 : RL];
-                    if constexpr (NB > 1) {
-                        const float4 *q = reinterpret_cast<const float4 *>(ln + (jj & (R1 - 1)) * PITCH + (jj / R1) * NB);
-#pragma unroll
-                        for (int i = 0; i < NB / 2; i++) {
-                            const float4 w = q[i];
-                            // block b sits at brev(b)
-                            zu[brevk(2 * i, ilog2k(NB))] = make_float2(w.x, w.y);
-                            zu[brevk(2 * i + 1, ilog2k(NB))] = make_float2(w.z, w.w);
-                        }
-                        if constexpr (NB == 16)
-                            math16<true, HL, FAST>(zu, triW + tw_off(L, HL) + jj);
-                        else
-                            math4<true, HL, FAST>(zu, triW + tw_off(L, HL) + jj);
-                        o = zu;
-                    }
-                    if (!FAST && !last) {
-                        // the channels' sum, in channel order (impl.go:425-443)
-#pragma unroll
-                        for (int i = 0; i < RL; i++) {
-                            float2 &s = acc[FAST ? 0 : it * RL + i];
-                            s = k == 0 ? o[i] : make_float2(__fadd_rn(s.x, o[i].x), __fadd_rn(s.y, o[i].y));
-                        }
-                        continue;
-                    }
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        if (h == 1 && !odd) break;
-                        if (h == 1 && !BOTH) load_den(it, 1);
-                        const bool rowIn = y0 + h >= roiY0 && y0 + h < roiY1;
-#pragma unroll
-                        for (int i = 0; i < RL; i++) {
-                            const int x = jj + HL * i, l = (2 * p + h) * N + x;
-                            float num = h ? o[i].y : o[i].x;
-                            if constexpr (!FAST) {
-                                const float2 s = acc[it * RL + i];
-                                if (cn > 1) num = __fadd_rn(h ? s.y : s.x, num);
-                                num = __fsub_rn(num, tt[BOTH ? h : 0][i]);
-                            }
-                            const float d = den[AHEAD ? it : 0][BOTH ? h : 0][i];
-                            // (the results of zero and, in the fast form, near-flat dens take the ladder)
-                            const bool cand = x < bw && !(d >= denLow && num < t.hi * d && num > t.lo * d);
-                            if constexpr (LEAN) {
-                                if (cand) t = score_track<FAST>(t, num, d, denFlat, l);
-                            } else if (x < bw) {
-                                const float sc = FAST ? score_fast(num, d, denFlat) : score_exact(num, d);
-                                if (map) map[row0 + h * rw + x] = sc;
-                                if (rowIn && x >= xlo && x < xhi) track(t, sc, l);
-                            }
-                        }
-                    }
-                    if (LEAN && it == 0 && !warm) {
-                        cut_share(t, mask);
-                        warm = true;
-                    }
-                }
-            }
-        // widen: CTA-local (row, x) -> the member's raster index
-        auto widen = [&](int l) {
-            return l == INT_MAX ? LLONG_MAX
-                                : (long long)(tb.y0 + 2 * pair0 + (l >> L)) * m.rw + tb.x0 + (l & (N - 1));
-        };
-        e.minV = t.minV;
-        e.maxV = t.maxV;
-        e.minI = widen(t.minL);
-        e.maxI = widen(t.maxL);
+        e = line_pairs<L, FAST, MODE>(a, smem, m, Pm, tb, bw, bh, pair0, P, bnd);
     }
     // a CTA none of whose results passed its member's cuts has nothing to reduce
     if (__syncthreads_or(e.minI != LLONG_MAX || e.maxI != LLONG_MAX)) ext_block_reduce(e, shExt);
@@ -462,19 +524,22 @@ __global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, LEAN)) k_in
     if (tid == 0) ext_store_result(e, m.rw, a.out + m.outIdx);
 }
 
-template <int L, bool FAST, bool LEAN>
+template <int L, bool FAST, Keep MODE>
 void lines_one(const InvArgs &a, dim3 grid, cudaStream_t st) {
-    set_smem(k_inv_lines<L, FAST, LEAN>, Lines<L>::SMEM);
-    launch_k(k_inv_lines<L, FAST, LEAN>, grid, dim3(Lines<L>::CTA), Lines<L>::SMEM, st, a);
+    const size_t smem = Lines<L>::SMEM + (MODE == TABLE ? kBlocksMax * sizeof(float) : 0);
+    set_smem(k_inv_lines<L, FAST, MODE>, smem);
+    launch_k(k_inv_lines<L, FAST, MODE>, grid, dim3(Lines<L>::CTA), smem, st, a);
 }
 
 template <int L>
 void lines_form(const InvArgs &a, dim3 grid, cudaStream_t st) {
-    const bool lean = !a.ms.map && !a.ms.anyRoi && !a.ms.sat;
-    if (a.ms.form)
-        lean ? lines_one<L, true, true>(a, grid, st) : lines_one<L, true, false>(a, grid, st);
+    const bool all = a.ms.map || a.ms.anyRoi;
+    if (!a.ms.form)
+        all ? lines_one<L, false, ALL>(a, grid, st) : lines_one<L, false, LANES>(a, grid, st);
+    else if (a.ms.sat)
+        lines_one<L, true, TABLE>(a, grid, st);
     else
-        lean ? lines_one<L, false, true>(a, grid, st) : lines_one<L, false, false>(a, grid, st);
+        all ? lines_one<L, true, ALL>(a, grid, st) : lines_one<L, true, LANES>(a, grid, st);
 }
 
 }  // namespace

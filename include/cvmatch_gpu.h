@@ -355,18 +355,20 @@ int cvm_fleet_set_overlap(cvm_fleet *f, int on);
 
 /* Where a fleet's window statistics are formed (no counterpart in the
  * reference, which computes them in normalizeBandGo, impl.go:708-805).
- * CVM_STATS_KERNEL (the default): the statistics kernel writes each
- * window's den, which the inverse-rows epilogue reads back.
- * CVM_STATS_EPILOGUE: fast-form buckets without regions of interest whose
- * every member satisfies area * cn * 16256 < 2^32 (colour members up to
- * 66,052 px, gray up to 264,208 px) form each window's den inside the
- * inverse-rows epilogue from the frame's summed-area table, with no
- * statistics launch and no den written or read; other buckets, and every
- * exact- or mixed-form bucket, still run the statistics kernel.  Results
- * are the same bits either way.  The epilogue form measured slower on a
- * GB300 (256 RGBA templates on a 2560x1440 frame: 10.3 against 9.5 ms per
- * FindAll), hence not the default.  Not to be called while a FindAll on
- * the same fleet runs. */
+ * CVM_STATS_KERNEL: the statistics kernel writes each window's den, which
+ * the inverse rows read back.  CVM_STATS_EPILOGUE: fast-form buckets without
+ * regions of interest whose rows have 128 to 2048 points and whose every
+ * member satisfies (w + 15) * (h + 15) * cn * 16256 < 2^32 form den inside
+ * the inverse rows, from the frame's summed-area table, for the windows that
+ * may hold an extremum (a lower bound of den over blocks of results rules
+ * out the rest), with no statistics launch and no den written or read; other
+ * buckets, and every exact- or mixed-form bucket, still run the statistics
+ * kernel.  Results are the same bits either way.  A fleet on which this was
+ * never called chooses by itself on its first frame of a size (256 RGBA
+ * templates on a 2560x1440 frame: 5.6 ms per FindAll with the epilogue, 7.8
+ * with the kernel; small templates on flat panels with thin strokes are
+ * faster with the kernel).  Not to be called while a FindAll on the same
+ * fleet runs. */
 #define CVM_STATS_KERNEL 0
 #define CVM_STATS_EPILOGUE 1
 int cvm_fleet_set_stats(cvm_fleet *f, int mode);
