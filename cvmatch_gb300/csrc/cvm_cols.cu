@@ -283,6 +283,60 @@ __device__ __forceinline__ void middle_sweep(float2 *smem, const LDX &ldx, const
     __syncthreads();
 }
 
+// ------------------------------------------------ 512 rows in two passes
+// A fast-form fleet's 512-row inverse (mode 3) regroups the cascade's five
+// stages as 32 x 16 points: the head, its h = 2 stage and the h = 8 stage on
+// 32 rows in registers, straight from the spectral product, then the h = 32
+// and h = 128 stages as one radix-16 unit, straight to global memory -- one
+// trip through shared memory instead of two.  The same butterflies on the
+// same operands: the same bits.  (128
+// registers, two CTAs per SM: the stored spectra's loads from L2 bind it, 256
+// templates on 2560x1440 3.13 -> 3.04 ms.  The exact form's one channel at a
+// time gains no load for its registers: 0.84 -> 0.86 ms, it keeps three
+// passes.)
+
+// The first three stages on 32 contiguous logical slots.
+__device__ __forceinline__ void math32_inv(float2 *e, const float2 *__restrict__ tri) {
+#pragma unroll
+    for (int g = 0; g < 4; g++) math_head<true, true>(e + 8 * g, tri);
+    const float2 *t = tri + tw_off(9, 8);
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        if (j == 0)
+            bfly4_one<true>(&e[0], &e[8], &e[16], &e[24]);
+        else
+            bfly4<true, true>(&e[j], &e[8 + j], &e[16 + j], &e[24 + j], __ldg(t + j), __ldg(t + 8 + j), __ldg(t + 16 + j));
+    }
+}
+
+// x[c'] is row B + 16 * c' of the product; st stores the last pass.
+template <int LSC, typename LDX, typename STF>
+__device__ __forceinline__ void inverse_512(float2 *smem, const LDX &ldx, const STF &stf,
+                                            const float2 *__restrict__ tri) {
+    constexpr int L = 9, SC = 1 << LSC;
+    for (int u = threadIdx.x; u < (16 << LSC); u += blockDim.x) {
+        const int c = u & (SC - 1), B = u >> LSC;
+        float2 x[32], e[32];
+        ldx(x, c, B);
+        // logical 32a + t <-> row B + 16 * brev5(t)
+#pragma unroll
+        for (int t = 0; t < 32; t++) e[t] = x[brevk(t, 5)];
+        math32_inv(e, tri);
+        float2 *sp = smem + (B << LSC) + c;
+#pragma unroll
+        for (int t = 0; t < 32; t++) sp[(16 * brevk(t, 5)) << LSC] = e[t];
+    }
+    __syncthreads();
+    const SmemRev<L, LSC> sr{smem};
+    for (int u = threadIdx.x; u < (32 << LSC); u += blockDim.x) {
+        const int c = u & (SC - 1), j = u >> LSC;
+        float2 e[16];
+        sr.template load<16, 32>(e, c, j);
+        math16<true, 32, true>(e, tri + tw_off(L, 32) + j);
+        stf.template store<16, 32>(e, c, j);
+    }
+}
+
 // ------------------------------------------------ mode 4: fused channels
 // The fast form of one colour match: every channel of a column strip in
 // one CTA (channel k's [N x SC] strip at smem + k*(N << LSC)).  The
@@ -408,7 +462,7 @@ __global__ void __launch_bounds__(256, 3) k_cols_sum_t(ColsArgs a) {
 }
 
 template <int MODE, int L>
-__global__ void __launch_bounds__(256, 3) k_cols_t(ColsArgs a) {
+__global__ void __launch_bounds__(256, MODE == 3 && L == 9 ? 2 : 3) k_cols_t(ColsArgs a) {
     griddep_wait();
     griddep_launch();
     constexpr int N = 1 << L, NP = npass(L);
@@ -462,7 +516,15 @@ __global__ void __launch_bounds__(256, 3) k_cols_t(ColsArgs a) {
     if (MODE != 0) {
         const float2 *ts = m->tspec[a.cls] + (size_t)k * chanStride + c0;
         constexpr int PL = NP - 1;
-        constexpr int M = ((L & 1) && pass_kind(L, PL) == K4) ? 8 : 16, S = N / M;
+        constexpr bool TWO = MODE == 3 && L == 9;  // two passes of 32 x 16 points
+        constexpr int M = TWO ? 32 : (((L & 1) && pass_kind(L, PL) == K4) ? 8 : 16), S = N / M;
+        auto inv_out = [&]() {
+            const int ty = tile / a.g.ntx;
+            const int bh = (ty == a.g.nty - 1) ? m->rh - b.y0 : a.g.blockH;
+            const size_t scrOff = MODE == 3 ? (size_t)tileLocal * chanStride : ((size_t)tileLocal * a.cnS + k) * chanStride;
+            return GlobalInv<L>{a.ms.scratch[a.cls] + (size_t)slot * a.ms.scratchStride[a.cls] + scrOff + c0, hwp, wv,
+                                min(N, (bh + 1) & ~1)};
+        };
         if (MODE == 1) {
             auto ldx = [&](float2 *x, int c, int B) {
                 const float2 *p = smem + (B << LSC) + c;
@@ -485,6 +547,7 @@ __global__ void __launch_bounds__(256, 3) k_cols_t(ColsArgs a) {
             // the sum into the strip first measured 3.63 against 3.50 ms per
             // 256-member 2560x1440 frame: the strip's extra store and load
             // are shared-memory traffic in a kernel bound by it.)
+            const GlobalInv<L> gi = inv_out();
             const float2 *fr = a.in + (size_t)tileLocal * a.cnS * chanStride + c0;
             const float2 *tq = m->tspec[a.cls] + c0;
             // The channel sum formed in the registers of the inverse's first
@@ -524,15 +587,15 @@ __global__ void __launch_bounds__(256, 3) k_cols_t(ColsArgs a) {
                     for (int kk = 0; kk < cn; kk++) chan(kk);
                 }
             };
-            middle_sweep<false, L, LSC, decltype(ldx), false, true>(smem, ldx, nullptr, hwp, wv, tri);
+            if constexpr (TWO) {
+                inverse_512<LSC>(smem, ldx, gi, tri);
+                return;
+            } else {
+                middle_sweep<false, L, LSC, decltype(ldx), false, true>(smem, ldx, nullptr, hwp, wv, tri);
+            }
         }
-        const int ty = tile / a.g.ntx;
-        const int bh = (ty == a.g.nty - 1) ? m->rh - b.y0 : a.g.blockH;
-        const size_t scrOff = MODE == 3 ? (size_t)tileLocal * chanStride : ((size_t)tileLocal * a.cnS + k) * chanStride;
-        const GlobalInv<L> gi{a.ms.scratch[a.cls] + (size_t)slot * a.ms.scratchStride[a.cls] + scrOff + c0, hwp, wv,
-                              min(N, (bh + 1) & ~1)};
         col_passes<true, L, 1, NP - 1, LSC, MODE == 3>(sr, tri);
-        col_pass<true, L, NP - 1, LSC, MODE == 3>(sr, gi, tri);
+        col_pass<true, L, NP - 1, LSC, MODE == 3>(sr, inv_out(), tri);
     }
 }
 
