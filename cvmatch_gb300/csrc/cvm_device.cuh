@@ -136,6 +136,7 @@ struct FwdRowsArgs {
     // i * 256 * 2 pairsPerCta; 0 = plain loads
     int tma;
     unsigned int tmaSmemOff;
+    int chanPer;             // 2^7 .. 2^11 points: channels of a grid layer (grid z)
 };
 
 // The row transforms specialised on dftW = 2^5 .. 2^12 (cvm_rows.cu).
@@ -145,6 +146,9 @@ bool rows_fixed_length(int log2n);
 int rows_fast_wave_elems(int log2n);
 void launch_fwd_rows_fixed(const FwdRowsArgs &a, const CUtensorMap &map, dim3 grid, int threads, size_t smem,
                            cudaStream_t st);
+// Shared memory of a CTA's line buffers in the kernels with a thread group
+// per line (2^7 .. 2^11 points; inv_lines_cta lines at a time).
+size_t fwd_lines_smem(int log2n);
 // Encodes a 2-D tensor map over w x h bytes at img (row stride istride)
 // with boxes of 256 bytes x boxRows rows; false when the driver entry point
 // or the encoding is unavailable.

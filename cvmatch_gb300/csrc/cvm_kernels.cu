@@ -2130,8 +2130,17 @@ cudaError_t launch_fwd_rows(const uint8_t *img, long long istride, int step, int
     // few rows (a small template or frame): fewer pairs per CTA until the
     // launch has a CTA per SM, so the rows are spread over the SMs
     while (P > 1 && (long long)((pairs + P - 1) / P) * fc.ntiles < 152) P >>= 1;
-    dim3 grid((pairs + P - 1) / P, fc.ntiles);
-    const size_t smem = (size_t)P * group * padded_len(fc.n) * sizeof(float2);
+    // rows with a thread group per line: a CTA takes the pairs it holds at a
+    // time, and the channels get a grid layer each while the launch has CTAs
+    // to spare
+    const bool lines = inv_lines_length(fc.log2n);
+    int layers = 1;
+    if (lines) {
+        P = inv_lines_cta(fc.log2n);
+        if ((long long)((pairs + P - 1) / P) * fc.ntiles < 8 * 152) layers = group;
+    }
+    dim3 grid((pairs + P - 1) / P, fc.ntiles, layers);
+    const size_t smem = lines ? fwd_lines_smem(fc.log2n) : (size_t)P * group * padded_len(fc.n) * sizeof(float2);
     // as many threads as a radix-16 pass has units (a multiple of 32 in
     // 64..256), so no thread idles in those passes; a device-chosen colour
     // count is 3 unless an alpha plane varies, so size for that
@@ -2146,6 +2155,7 @@ cudaError_t launch_fwd_rows(const uint8_t *img, long long istride, int step, int
         a.chanCount = chanCount;
         a.cnDev = cnDev;
         a.chanGroup = group;
+        a.chanPer = (group + layers - 1) / layers;
         a.g = g;
         a.fc = fc;
         a.spec = spec;

@@ -32,13 +32,8 @@
 // of reading each value twice from L1 measured 2.62 ms: 17 KB per line
 // leaves the twiddles no L1.
 //
-// Layout of the line buffer: pass 1's unit of natural index k0 (logical
-// block v = brev(k0)) stores output i at i * PITCH + k0.  Pass 2's unit
-// (block b, column j) reads its 16 elements at j * PITCH + brev4(i) * NB +
-// brev(b) and stores them in place, output i at j * PITCH + i * NB +
-// brev(b); pass 3's unit jj = j + R1 * i then reads NB consecutive
-// elements.  PITCH keeps the three access patterns free of bank conflicts.
-#include "cvm_device.cuh"
+// (Line buffer: cvm_lines.cuh.)
+#include "cvm_lines.cuh"
 
 namespace cvm {
 namespace {
@@ -137,32 +132,6 @@ __device__ __noinline__ Track score_table(Track t, float num, const MemberSet &m
     return t;
 }
 
-template <int L>
-struct Lines {
-    static constexpr int N = 1 << L;
-    static constexpr int R1 = (L & 1) ? 8 : 16;           // pass 1: the head, or radix 16 at quarter 1
-    static constexpr int K1 = N / R1;                     // its units
-    static constexpr int NB = N / (16 * R1);              // blocks of pass 2 = pass 3's radix (1: no pass 3)
-    static constexpr int H2 = R1, H3 = 16 * R1;           // quarters of passes 2 and 3
-    // line pitch: conflict-free for pass 2's reads (8-byte words of NB-wide
-    // blocks) and pass 3's 16-byte reads over consecutive columns
-    static constexpr int PITCH = NB == 1 ? K1 + 1 : (NB == 4 ? K1 + 6 : K1 + 2);
-    static constexpr int LINE = (R1 * PITCH + 1) & ~1;    // elements
-    static constexpr int G = N / 16;                      // threads of a line
-    static constexpr int CTA = G > 64 ? G : 64;
-    static constexpr int NL = CTA / G;                    // lines of a CTA at a time
-    static constexpr size_t SMEM = (size_t)NL * LINE * sizeof(float2);  // + TABLE's bounds
-};
-
-// The barrier of a line's threads: the CTA (one line at a time) or the
-// group's lanes of its warp.
-template <int G>
-__device__ __forceinline__ void group_sync(unsigned int mask) {
-    if constexpr (G <= 32)
-        __syncwarp(mask);
-    else
-        __syncthreads();
-}
 
 // CTAs per SM the registers are budgeted for: 96 registers hold a fast-form
 // thread's 32 den values ahead of the last pass (12 CTAs spill: 2.13 against
@@ -209,6 +178,8 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
     float *map = LEAN ? nullptr : a.ms.map;
     const int rw = m.rw, xlo = m.roiX0 - tb.x0, xhi = m.roiX1 - tb.x0, roiY0 = m.roiY0, roiY1 = m.roiY1;
     const float2 *triW = fc.triW;
+    int j2, b2;
+    pass2_unit<L>(lt, j2, b2);
     bool warm = false;                                // the cuts have been shared once
     float postV = -FLT_MAX, postN = FLT_MAX;          // TABLE: the extrema the warp has posted
     float *lbs = reinterpret_cast<float *>(smem + (size_t)NL * S::LINE);
@@ -298,21 +269,7 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
             if (k + 1 < cn || p + NL < P) prefetch(k + 1 < cn ? p : p + NL, k + 1 < cn ? k + 1 : 0);
             group_sync<G>(mask);
             float2 z[16];
-            {
-                // pass 2: unit (b, j); lanes run over the blocks first
-                // (NB = 4: even columns, then odd ones, in groups of eight,
-                // keep the half-warps on distinct banks)
-                const int bb = lt & (NB - 1), jl = lt / NB;
-                const int j = NB == 4 ? (jl & 8) | ((jl & 3) << 1) | ((jl >> 2) & 1) : jl;
-                float2 *q = ln + j * PITCH + bb;
-#pragma unroll
-                for (int i = 0; i < 16; i++) z[i] = q[brevk(i, 4) * NB];
-                math16<true, S::H2, FAST>(z, triW + tw_off(L, S::H2) + j);
-                if constexpr (NB > 1) {
-#pragma unroll
-                    for (int i = 0; i < 16; i++) q[i * NB] = z[i];
-                }
-            }
+            pass2<L, true, FAST>(ln, j2, b2, z, triW);
             const bool last = k == cn - 1;
             const bool odd = 2 * (pair0 + p) + 1 < bh;  // the imaginary part's row exists
             const int y0 = tb.y0 + 2 * (pair0 + p);
@@ -361,18 +318,7 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                 float2 *o = z;
                 float2 zu[NB == 1 ? 1 : RL];
                 if constexpr (NB > 1) {
-                    const float4 *q = reinterpret_cast<const float4 *>(ln + (jj & (R1 - 1)) * PITCH + (jj / R1) * NB);
-#pragma unroll
-                    for (int i = 0; i < NB / 2; i++) {
-                        const float4 w = q[i];
-                        // block b sits at brev(b)
-                        zu[brevk(2 * i, ilog2k(NB))] = make_float2(w.x, w.y);
-                        zu[brevk(2 * i + 1, ilog2k(NB))] = make_float2(w.z, w.w);
-                    }
-                    if constexpr (NB == 16)
-                        math16<true, HL, FAST>(zu, triW + tw_off(L, HL) + jj);
-                    else
-                        math4<true, HL, FAST>(zu, triW + tw_off(L, HL) + jj);
+                    pass3<L, true, FAST>(ln, jj, zu, triW);
                     o = zu;
                 }
                 if (!FAST && !last) {

@@ -11,7 +11,7 @@
 // one per element.  Other lengths run the generic kernels.
 #include <cudaTypedefs.h>
 
-#include "cvm_device.cuh"
+#include "cvm_lines.cuh"
 
 namespace cvm {
 namespace {
@@ -276,6 +276,235 @@ __device__ __noinline__ void tma_stage_rows(const CUtensorMap *map, unsigned cha
     }
 }
 
+// The sample offsets of a launch (FwdRowsArgs::sub and its device-side forms).
+__device__ __forceinline__ void sample_offsets(const FwdRowsArgs &a, const TileBox &b, float *subv) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const long long istride = a.istride;
+    if (a.selfSums) {
+        // the template's own channel sums (this launch's one tile is the
+        // whole template): exact integers, reduced per warp then per CTA
+        __shared__ unsigned long long ssum[4];
+        if (tid < 4) ssum[tid] = 0ull;
+        __syncthreads();
+        unsigned long long sv[4] = {0ull, 0ull, 0ull, 0ull};
+        const uint8_t *t0 = a.img + (long long)b.y0 * istride + (long long)b.x0 * a.step;
+        const int npx = b.loadW * b.loadH;
+        if (a.pix32) {
+            unsigned int s4[4] = {0u, 0u, 0u, 0u};  // at most npx * 255 < 2^32
+#pragma unroll 4
+            for (int i = tid; i < npx; i += nt) {
+                const int y = i / b.loadW, x = i - y * b.loadW;
+                const unsigned int w = __ldg(reinterpret_cast<const unsigned int *>(t0 + (long long)y * istride) + x);
+#pragma unroll
+                for (int c = 0; c < 4; c++) s4[c] += (w >> (8 * c)) & 255u;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; c++) sv[c] = s4[c];
+        } else {
+            for (int i = tid; i < npx; i += nt) {
+                const int y = i / b.loadW, x = i - y * b.loadW;
+                const uint8_t *q = t0 + (long long)y * istride + (long long)x * a.step;
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (c < a.step) sv[c] += q[c];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sv[c] += __shfl_down_sync(0xffffffffu, sv[c], o);
+            if ((tid & 31) == 0 && sv[c]) atomicAdd(&ssum[c], sv[c]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < 4; c++) subv[c] = __fdiv_rn(__ull2float_rn(ssum[c]), a.subDiv);
+    } else {
+#pragma unroll
+        for (int g = 0; g < 4; g++)
+            subv[g] = a.subSums ? __fdiv_rn(__ull2float_rn(a.subSums[g]), a.subDiv) : a.sub[g];
+    }
+}
+
+// forwardRowPair (impl.go:301-344) with N/16 threads per line (N = 2^7 ..
+// 2^11): the same packing, butterflies and untangle as k_fwd_rows_t, so the
+// same bits.  A thread group holds a row pair's pixels -- every channel of
+// the 16 samples its first pass takes -- in registers and transforms the
+// launch's channels (or, in a launch with CTAs to spare, the one of its grid
+// layer) one after another; the line buffer takes two trips instead of the
+// scatter into bit-reversed order (four-way bank conflicts), two passes and
+// the last; barriers span two warps instead of eight.  A
+// 2560x1440 RGBA frame's 12 tiles of 1024 x 512: 85 -> 67 us; a 3840x2160 gray
+// frame beside its other chains 76 -> 55 us; a 1920x1080 RGBA frame likewise,
+// exact, 73 -> 38 us.  (Loads under per-sample conditions, instead of clamped
+// ones: 72 us, and 47 against 35 us on a 1366x767 frame without TMA.)
+template <int L, bool F>
+__global__ void __launch_bounds__(Lines<L>::CTA, L == 11 ? 4 : 8) k_fwd_lines(FwdRowsArgs a,
+                                                                             const __grid_constant__ CUtensorMap map) {
+    griddep_wait();
+    griddep_launch();
+    using S = Lines<L>;
+    constexpr int N = S::N, R1 = S::R1, K1 = S::K1, NB = S::NB, G = S::G, NL = S::NL, HALF = N / 2;
+    constexpr int LR1 = R1 == 16 ? 4 : 3;
+    extern __shared__ __align__(16) float2 smem[];
+    const FftClass &fc = a.fc;
+    const int tile = fc.tileFirst + blockIdx.y;
+    const TileBox b = tile_box(a.g, tile);
+    const int nrows = min(b.loadH, fc.dftH);
+    const int pair0 = blockIdx.x * a.pairsPerCta;
+    if (2 * pair0 >= nrows) return;
+    const int cnEff = a.cnDev ? min(*a.cnDev, a.chanCount) : a.chanCount;
+    const int cn = min(cnEff - a.chanFirst, a.chanGroup);  // channels of this launch's group
+    const int kA = blockIdx.z * a.chanPer, kB = min(cn, kA + a.chanPer);
+    if (kA >= kB) return;
+    const int P = min(a.pairsPerCta, (nrows - 2 * pair0 + 1) >> 1);
+    const int tid = threadIdx.x, g = tid / G, lt = tid - g * G;
+    const unsigned int mask = G >= 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((tid & 31) / G * G);
+    const long long istride = a.istride;
+    const uint8_t *img0 = a.img + (long long)(b.y0 + 2 * pair0) * istride + (long long)b.x0 * a.step;
+    float subv[4];
+    sample_offsets(a, b, subv);
+    // TMA: the CTA's rows land in shared memory first (box i holds bytes
+    // [xbase + 256 i, +256) of each of the box's rows)
+    __shared__ __align__(8) uint64_t tmaBar;
+    const int boxRows = 2 * a.pairsPerCta;
+    const unsigned char *stage = reinterpret_cast<const unsigned char *>(
+        (reinterpret_cast<uintptr_t>(smem) + a.tmaSmemOff + 127) & ~uintptr_t(127));
+    int tmaOff = 0;
+    if (a.tma) {
+        const int xbyte = b.x0 * a.step, xbase = xbyte & ~15;
+        tmaOff = xbyte - xbase;
+        const int nb = (tmaOff + b.loadW * a.step + 255) >> 8;
+        tma_stage_rows(&map, const_cast<unsigned char *>(stage), &tmaBar, xbase, b.y0 + 2 * pair0, nb, boxRows);
+    }
+    float2 *ln = smem + (size_t)g * S::LINE;
+    const float2 *tri = fc.triW;
+    const int hwp = fc.hwp, log2H = fc.log2H;
+    const size_t chanStride = (size_t)fc.dftH * hwp;
+    float2 *tbase = a.spec + (size_t)(tile - fc.tileFirst) * a.cnS * chanStride;
+    int j2, b2;
+    pass2_unit<L>(lt, j2, b2);
+    for (int p = g; p < P; p += NL) {
+        const int r = 2 * (pair0 + p);
+        const bool two = r + 1 < b.loadH;
+        // the pair's pixels at the thread's samples, channel chanFirst + c in
+        // byte c; samples beyond the row and a missing second row read a pixel
+        // that is there (pass 1 puts zeros in their place)
+        unsigned int wa[16], wb[16];
+        auto sample = [&](int n) { return min(lt + (n / R1) * G + K1 * (n % R1), b.loadW - 1); };
+        const uint8_t *pa = img0 + (long long)(2 * p) * istride, *pb = two ? pa + istride : pa;
+        if (a.tma) {
+            const unsigned char *st = stage + (size_t)(2 * p) * 256;
+            const int down = two ? 256 : 0;
+#pragma unroll
+            for (int n = 0; n < 16; n++) {
+                const int o = tmaOff + sample(n) * a.step, at = (o & ~255) * boxRows + (o & 255);
+                if (a.pix32) {
+                    wa[n] = *reinterpret_cast<const unsigned int *>(st + at) >> (8 * a.chanFirst);
+                    wb[n] = *reinterpret_cast<const unsigned int *>(st + at + down) >> (8 * a.chanFirst);
+                } else {  // gray
+                    wa[n] = st[at];
+                    wb[n] = st[at + down];
+                }
+            }
+        } else if (a.pix32) {
+#pragma unroll
+            for (int n = 0; n < 16; n++) {
+                const int x = sample(n);
+                wa[n] = __ldg(reinterpret_cast<const unsigned int *>(pa) + x) >> (8 * a.chanFirst);
+                wb[n] = __ldg(reinterpret_cast<const unsigned int *>(pb) + x) >> (8 * a.chanFirst);
+            }
+        } else {
+#pragma unroll
+            for (int n = 0; n < 16; n++) wa[n] = wb[n] = 0u;
+            for (int c = 0; c < cn; c++) {
+#pragma unroll
+                for (int n = 0; n < 16; n++) {
+                    const long long x = (long long)sample(n) * a.step + a.chanFirst + c;
+                    wa[n] |= (unsigned int)pa[x] << (8 * c);
+                    wb[n] |= (unsigned int)pb[x] << (8 * c);
+                }
+            }
+        }
+#pragma unroll 1
+        for (int k = kA; k < kB; k++) {
+            const float sg = subv[(a.chanFirst + k) & 3];
+            // pass 1: unit k0's elements are samples k0 + K1 * brev(i)
+            // (bit-reversed input); pixel * mul - sub is exact for the
+            // integers used; padding and a missing second row stay zero
+#pragma unroll
+            for (int q = 0; q < 16 / R1; q++) {
+                const int k0 = lt + q * G;
+                float2 z[R1];
+#pragma unroll
+                for (int i = 0; i < R1; i++) {
+                    const int x = k0 + K1 * i, n = q * R1 + i;
+                    const float va = (float)((wa[n] >> (8 * k)) & 255u), vb = (float)((wb[n] >> (8 * k)) & 255u);
+                    z[brevk(i, LR1)] = make_float2(x < b.loadW ? __fsub_rn(__fmul_rn(va, a.mul), sg) : 0.f,
+                                                   x < b.loadW && two ? __fsub_rn(__fmul_rn(vb, a.mul), sg) : 0.f);
+                }
+                if constexpr (R1 == 16)
+                    math16<false, 1, F>(z, tri);
+                else
+                    math_head<false, F>(z, tri);
+                // the previous channel's untangle has read the line
+                if (q == 0) group_sync<G>(mask);
+#pragma unroll
+                for (int i = 0; i < R1; i++) ln[i * S::PITCH + k0] = z[i];
+            }
+            group_sync<G>(mask);
+            float2 z[16];
+            pass2<L, false, F>(ln, j2, b2, z, tri);
+            group_sync<G>(mask);
+            // untangle (impl.go:331-341) into the two real-row spectra at
+            // their bit-reversed column-transform slots
+            float2 *cb = tbase + (size_t)(a.chanFirst + k) * chanStride;
+            float2 *ra = cb + (size_t)brev_bits(r, log2H) * hwp, *rb = cb + (size_t)brev_bits(r + 1, log2H) * hwp;
+            auto emit = [&](int kk, float2 zk, float2 n) {
+                ra[kk] = make_float2(__fmul_rn(0.5f, __fadd_rn(zk.x, n.x)), __fmul_rn(0.5f, __fsub_rn(zk.y, n.y)));
+                rb[kk] = make_float2(__fmul_rn(0.5f, __fadd_rn(zk.y, n.y)), __fmul_rn(0.5f, __fsub_rn(n.x, zk.x)));
+            };
+            if constexpr (NB == 4) {
+                // the last pass with it: the mirrors of unit j's outputs lie
+                // in unit H - j (j = 0 and H / 2 are their own)
+                constexpr int H = S::H3;
+                for (int j = lt; j <= H / 2; j += G) {
+                    float2 za[4];
+                    pass3<L, false, F>(ln, j, za, tri);
+                    if (j == 0) {
+                        emit(0, za[0], za[0]);
+                        emit(H, za[1], za[3]);
+                        emit(HALF, za[2], za[2]);
+                    } else if (j == H / 2) {
+                        emit(j, za[0], za[3]);
+                        emit(j + H, za[1], za[2]);
+                    } else {
+                        const int jp = H - j;
+                        float2 zb[4];
+                        pass3<L, false, F>(ln, jp, zb, tri);
+                        emit(j, za[0], zb[3]);
+                        emit(j + H, za[1], zb[2]);
+                        emit(jp, zb[0], za[3]);
+                        emit(jp + H, zb[1], za[2]);
+                    }
+                }
+            } else {
+                // the last pass's outputs back to the line in natural order
+                if constexpr (NB == 1) {
+#pragma unroll
+                    for (int i = 0; i < 16; i++) ln[j2 + S::H2 * i] = z[i];
+                } else {
+                    pass3<L, false, F>(ln, lt, z, tri);
+                    group_sync<G>(mask);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) ln[lt + S::H3 * i] = z[i];
+                }
+                group_sync<G>(mask);
+                for (int kk = lt; kk <= HALF; kk += G) emit(kk, ln[kk], ln[(N - kk) & (N - 1)]);
+            }
+        }
+    }
+}
+
 template <int LOG2N, bool F>
 __global__ void __launch_bounds__(256) k_fwd_rows_t(FwdRowsArgs a, const __grid_constant__ CUtensorMap map) {
     griddep_wait();
@@ -297,36 +526,7 @@ __global__ void __launch_bounds__(256) k_fwd_rows_t(FwdRowsArgs a, const __grid_
     const long long istride = a.istride;
     const uint8_t *img0 = a.img + (long long)(b.y0 + 2 * pair0) * istride + (long long)b.x0 * a.step;
     float subv[4];
-    if (a.selfSums) {
-        // the template's own channel sums (this launch's one tile is the
-        // whole template): exact integers, reduced per warp then per CTA
-        __shared__ unsigned long long ssum[4];
-        if (tid < 4) ssum[tid] = 0ull;
-        __syncthreads();
-        unsigned long long sv[4] = {0ull, 0ull, 0ull, 0ull};
-        const uint8_t *t0 = a.img + (long long)b.y0 * istride + (long long)b.x0 * a.step;
-        const int npx = b.loadW * b.loadH;
-        for (int i = tid; i < npx; i += nt) {
-            const int y = i / b.loadW, x = i - y * b.loadW;
-            const uint8_t *q = t0 + (long long)y * istride + (long long)x * a.step;
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (c < a.step) sv[c] += q[c];
-        }
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sv[c] += __shfl_down_sync(0xffffffffu, sv[c], o);
-            if ((tid & 31) == 0 && sv[c]) atomicAdd(&ssum[c], sv[c]);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < 4; c++) subv[c] = __fdiv_rn(__ull2float_rn(ssum[c]), a.subDiv);
-    } else {
-#pragma unroll
-        for (int g = 0; g < 4; g++)
-            subv[g] = a.subSums ? __fdiv_rn(__ull2float_rn(a.subSums[g]), a.subDiv) : a.sub[g];
-    }
+    sample_offsets(a, b, subv);
     // TMA: the CTA's rows land in shared memory first (box i holds bytes
     // [xbase + 256 i, +256) of each of the box's rows)
     __shared__ __align__(8) uint64_t tmaBar;
@@ -783,6 +983,17 @@ __global__ void __launch_bounds__(256, FAST ? (last_pass_r(LOG2N) == 16 ? 2 : 4)
 }
 
 template <int L>
+void fwd_lines(const FwdRowsArgs &a, const CUtensorMap &map, dim3 grid, size_t smem, cudaStream_t st) {
+    if (a.fma) {
+        set_smem(k_fwd_lines<L, true>, smem);
+        launch_k(k_fwd_lines<L, true>, grid, dim3(Lines<L>::CTA), smem, st, a, map);
+    } else {
+        set_smem(k_fwd_lines<L, false>, smem);
+        launch_k(k_fwd_lines<L, false>, grid, dim3(Lines<L>::CTA), smem, st, a, map);
+    }
+}
+
+template <int L>
 void fwd_one(const FwdRowsArgs &a, const CUtensorMap &map, dim3 grid, int threads, size_t smem, cudaStream_t st) {
     if (a.fma) {
         set_smem(k_fwd_rows_t<L, true>, smem);
@@ -826,12 +1037,22 @@ void launch_fwd_rows_fixed(const FwdRowsArgs &a, const CUtensorMap &map, dim3 gr
     switch (a.fc.log2n) {
         case 5: fwd_one<5>(a, map, grid, threads, smem, st); break;
         case 6: fwd_one<6>(a, map, grid, threads, smem, st); break;
-        case 7: fwd_one<7>(a, map, grid, threads, smem, st); break;
-        case 8: fwd_one<8>(a, map, grid, threads, smem, st); break;
-        case 9: fwd_one<9>(a, map, grid, threads, smem, st); break;
-        case 10: fwd_one<10>(a, map, grid, threads, smem, st); break;
-        case 11: fwd_one<11>(a, map, grid, threads, smem, st); break;
+        case 7: fwd_lines<7>(a, map, grid, smem, st); break;
+        case 8: fwd_lines<8>(a, map, grid, smem, st); break;
+        case 9: fwd_lines<9>(a, map, grid, smem, st); break;
+        case 10: fwd_lines<10>(a, map, grid, smem, st); break;
+        case 11: fwd_lines<11>(a, map, grid, smem, st); break;
         default: fwd_one<12>(a, map, grid, threads, smem, st); break;
+    }
+}
+
+size_t fwd_lines_smem(int log2n) {
+    switch (log2n) {
+        case 7: return Lines<7>::SMEM;
+        case 8: return Lines<8>::SMEM;
+        case 9: return Lines<9>::SMEM;
+        case 10: return Lines<10>::SMEM;
+        default: return Lines<11>::SMEM;
     }
 }
 
