@@ -382,7 +382,14 @@ struct SoloJob {
     int frameOnSide;  // the frame arrives on the second side stream (its frame event)
     int form;         // CVM_FORM_EXACT, _FAST or _MIXED (cached spectra must be of this form)
     const Plan *plan; // the tile plan (one-shot; nullptr: the tuned plan, or newGoPlan)
+    void *work;       // the workspace, its head cleared (nullptr: taken from the pool for the call)
+    size_t *need;     // report the workspace's size and queue nothing
 };
+
+// The head of a one-shot call's workspace that is cleared first: DevParams and
+// DevFrame, 256 bytes each.
+constexpr size_t kSoloZero = 512;
+static_assert(sizeof(DevParams) <= 256 && sizeof(DevFrame) <= 256, "the head of the workspace");
 
 int run_solo(const SoloJob &J, cudaStream_t st);
 
@@ -433,7 +440,7 @@ int solo_plan(const SoloJob &J, cudaStream_t st, Plan *out) {
         }
     }
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    if (!J.img || cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return CVM_OK;
     }
@@ -534,10 +541,14 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
         if (fastSum) bytes += Arena::bytes(spec_elems(G->fc[c], 1), sizeof(float2));
         if (!J.cachedP) bytes += Arena::bytes(tspec_elems(G->fc[c], cnS), sizeof(float2));
     }
+    if (J.need) {
+        *J.need = bytes;
+        return CVM_OK;
+    }
     PoolBuf buf;
-    CVM_TRY(pool_alloc(buf, bytes, st));
+    if (!J.work) CVM_TRY(pool_alloc(buf, bytes, st));
     Arena A;
-    A.base = static_cast<char *>(buf.p);
+    A.base = static_cast<char *>(J.work ? J.work : buf.p);
     DevParams *P = A.take<DevParams>(1);
     DevFrame *F = A.take<DevFrame>(1);
     Partial *parts = A.take<Partial>(nparts);
@@ -555,11 +566,8 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
             ts[c] = tsOwn[c];
         }
     }
-    CVM_CUDA(cudaMemsetAsync(F, 0, sizeof(DevFrame), st));
-    if (J.cachedP)
-        CVM_CUDA(cudaMemcpyAsync(P, J.cachedP, sizeof(DevParams), cudaMemcpyDeviceToDevice, st));
-    else
-        CVM_CUDA(cudaMemsetAsync(P, 0, sizeof(DevParams), st));
+    // P and F, adjacent, in one
+    if (!J.work) CVM_CUDA(cudaMemsetAsync(P, 0, kSoloZero, st));
     MemberSet ms;
     memset(&ms, 0, sizeof ms);
     ms.solo.tspec[0] = ts[0];
@@ -597,9 +605,19 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     // flight the same early chain measured slower end to end, with the
     // ingest kernel and with the copy engine alike: host-buffer calls keep
     // the template behind the frame.)
-    const bool early = !J.frameOnSide && !J.cachedP && J.mode == 1 && (long long)J.tw * J.th <= 65536;
+    // (A 640x480 gray match from RGBA, replayed: 92 -> 84 us.)
+    // A call whose channel count is fixed needs k_prep's results only in the
+    // vertical pass of its statistics and from its columns on: k_prep takes a
+    // stream of its own, and the frame's rows, the horizontal sums and the
+    // template's spectrum (the fast form's sums its own samples) all start at
+    // once.
+    const bool known = J.mode == 0;
+    // (every CTA of the row kernel sums the template: small ones)
+    const bool early = !J.cachedP && (known ? !fast || (long long)J.tw * J.th <= 8192
+                                            : !J.frameOnSide && (long long)J.tw * J.th <= 65536);
+    if (known && J.frameOnSide) CVM_CUDA(cudaStreamWaitEvent(st, ss.frame, 0));
+    if (known || early) CVM_CUDA(cudaEventRecord(ss.fork, st));  // the inputs, P and F zeroed, the pool's buffers
     if (early) {
-        CVM_CUDA(cudaEventRecord(ss.fork, st));  // the template and the pool's spectrum buffers
         CVM_CUDA(cudaStreamWaitEvent(ss.st, ss.fork, 0));
         CVM_TRY(build_tspec(*G, J.tpl, J.tstride, J.step, J.tw, J.th, cnS, nullptr, tsOwn[0], tsOwn[1], ss.st,
                             nullptr, nullptr, fast ? 1 : 0));
@@ -611,7 +629,7 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     // priority, so they fill the SMs the transforms leave instead of
     // displacing the row transform; otherwise the statistics start after
     // k_prep, above it.
-    const bool statsLate = fastSum && J.th <= 64;
+    const bool statsLate = !known && fastSum && J.th <= 64;
     // Otherwise, on a frame of 2^20 pixels or more, the frame's row
     // transform of every channel the alpha scans cannot drop (all but a
     // colour match's alpha plane) runs on the rows stream (the caller's
@@ -624,15 +642,20 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     // template 92.8 -> 96.6 us in the fast form; the same match in the exact
     // form 118.5 -> 113 us, a 3840x2160 gray match with a 256x256 template
     // 209.6 -> 202.7 us in the fast form.)
-    const bool split = !statsLate && (long long)J.iw * J.ih >= (1LL << 20);
-    if (J.frameOnSide) CVM_CUDA(cudaStreamWaitEvent(st, ss.frame, 0));
+    const bool split = !known && !statsLate && (long long)J.iw * J.ih >= (1LL << 20);
+    if (!known && J.frameOnSide) CVM_CUDA(cudaStreamWaitEvent(st, ss.frame, 0));
+    cudaStream_t pst = known ? ss.stats : st;  // k_prep's stream
+    if (known) {
+        CVM_CUDA(cudaStreamWaitEvent(ss.stats, ss.fork, 0));
+        CVM_CUDA(cudaStreamWaitEvent(ss.st2, ss.fork, 0));
+    }
     if (split) {
         CVM_CUDA(cudaEventRecord(ss.fork, st));  // the frame, P and F zeroed, the pool's buffers
         CVM_CUDA(cudaStreamWaitEvent(ss.stats, ss.fork, 0));
     }
     CVM_CUDA(launch_prep(J.cachedP ? nullptr : J.tpl, J.tstride, J.tw, J.th, J.step, cnS,
                          J.mode == 1 ? J.img : nullptr, J.istride, J.iw, J.ih, P, 1, J.cachedP ? 0 : 1, J.mode,
-                         J.cnFixed, F, st));
+                         J.cnFixed, F, pst, J.cachedP));
     // the fast form transforms the frame offset by -128 (zero-mean templates)
     const float off[4] = {128.f, 128.f, 128.f, 128.f};
     if (split) {
@@ -642,13 +665,13 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
         CVM_CUDA(cudaEventRecord(ss.rows, ss.stats));
     }
     cudaStream_t sst = statsLate ? ss.stats : ss.st2;
-    CVM_CUDA(cudaEventRecord(ss.prep, st));
+    CVM_CUDA(cudaEventRecord(ss.prep, pst));
     if (!early) CVM_CUDA(cudaStreamWaitEvent(ss.st, ss.prep, 0));
-    CVM_CUDA(cudaStreamWaitEvent(sst, ss.prep, 0));
+    if (!known) CVM_CUDA(cudaStreamWaitEvent(sst, ss.prep, 0));
     if (!statsLate) {
         CVM_CUDA(launch_sep_stats(J.img, J.istride, J.step, J.iw, J.ih, ms, 1, J.tw, rw, sg,
                                   J.mode == 1 ? 3 : J.cnFixed, J.mode == 1 ? 4 : J.cnFixed, H, 0, sst, 0, nullptr,
-                                  nullptr, blk));
+                                  nullptr, blk, known ? J.cnFixed : 0, known ? ss.prep : nullptr));
         CVM_CUDA(cudaEventRecord(ss.joinStats, sst));
     }
     if (!J.cachedP && !early)
@@ -667,9 +690,10 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
         // launch)
         PdlScope pdl(statsLate);
         for (int c = 0; c < G->nclass; c++)
-            CVM_CUDA(launch_fwd_rows(J.img, J.istride, J.step, cnS, &P->cn, G->g, G->fc[c], spec[c], cnS, st, 0,
-                                     nullptr, 1.0f, fast ? off : nullptr));
+            CVM_CUDA(launch_fwd_rows(J.img, J.istride, J.step, cnS, known ? nullptr : &P->cn, G->g, G->fc[c], spec[c],
+                                     cnS, st, 0, nullptr, 1.0f, fast ? off : nullptr));
     }
+    if (known) CVM_CUDA(cudaStreamWaitEvent(st, ss.prep, 0));
     if (statsLate) {
         // the horizontal sums at the caller's priority, the vertical pass
         // (which gates the inverse rows) back above it on the second side stream
@@ -882,12 +906,205 @@ cvm_result *host_result_slot(cvm_result **dev) {
     return s.h;
 }
 
+// What a call wants of its device map: the map, or its occurrences.
+int map_results(const float *dMap, int rw, int rh, float *map, const PeakReq *pk, PoolBuf &bp, cudaStream_t st) {
+    if (map) CVM_CUDA(cudaMemcpyAsync(map, dMap, (size_t)rw * rh * sizeof(float), cudaMemcpyDeviceToHost, st));
+    if (pk) {
+        const size_t nsc = peaks_scratch_ints(rw, rh);
+        const size_t xyBytes = (size_t)std::max(pk->maxPeaks, 0) * 2 * sizeof(int32_t);
+        CVM_TRY(pool_alloc(bp, (nsc + 1) * sizeof(int) + xyBytes, st));
+        int *scr = static_cast<int *>(bp.p), *dCount = scr + nsc;
+        int32_t *dXY = reinterpret_cast<int32_t *>(dCount + 1);
+        CVM_CUDA(launch_peaks(dMap, rw, rh, pk->thresh, pk->rx, pk->ry, scr, dXY, pk->maxPeaks, dCount, st));
+        CVM_CUDA(cudaMemcpyAsync(pk->count, dCount, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        if (xyBytes) CVM_CUDA(cudaMemcpyAsync(pk->xy, dXY, xyBytes, cudaMemcpyDeviceToHost, st));
+    }
+    return CVM_OK;
+}
+
+// A repeated one-shot call as a CUDA graph.  A small host-buffer call queued
+// launch by launch -- some thirty runtime calls over four streams -- is bound
+// by the host: 84 us for a 320x200 gray match, 104 for a 640x480 one from
+// RGBA; replayed 45 and 57 us (GB300, Grace host).  From the kGraphCalls-th call of a shape on, a thread
+// replays its launches as one graph: the inputs by one kernel that takes the
+// caller's addresses from mapped page-locked memory (so the graph holds no
+// caller's pointer), then run_solo's launches on a workspace of the graph's
+// own.  Inputs of up to kGraphStage bytes are copied behind those addresses by
+// the host first: 64 KB in 3 us, where the device takes 15 us to translate and
+// read a few pageable pages.  A thread keeps the kGraphs shapes it used last, each of at most
+// kGraphBytes, until other shapes take their places or the thread ends.  Where
+// the device cannot read the caller's memory, under the profiler, or when the
+// capture fails, the call is queued launch by launch.
+constexpr int kGraphs = 4, kGraphCalls = 3;
+constexpr size_t kGraphBytes = size_t(256) << 20, kGraphStage = size_t(192) << 10;
+
+struct SoloKey {
+    int iw, ih, tw, th, mode, cn, step, gray, form, tune, map;
+    bool operator==(const SoloKey &o) const {
+        return std::tie(iw, ih, tw, th, mode, cn, step, gray, form, tune, map) ==
+               std::tie(o.iw, o.ih, o.tw, o.th, o.mode, o.cn, o.step, o.gray, o.form, o.tune, o.map);
+    }
+};
+
+struct SoloGraph {
+    SoloKey key{};
+    int calls = 0;       // of the shape so far
+    bool failed = false;
+    uint64_t used = 0;
+    void *mem = nullptr;  // frame, template, map, workspace
+    float *map = nullptr;
+    SoloSource *src = nullptr;  // mapped page-locked, and the staged inputs behind it
+    uint8_t *stage[2] = {nullptr, nullptr}, *stageDev[2] = {nullptr, nullptr};  // frame, template (nullptr: read in place)
+    cvm_result *res = nullptr;  // likewise
+    cudaGraphExec_t exec = nullptr;
+    unsigned launches = 0;
+    void drop() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (mem) cudaFree(mem);
+        if (src) cudaFreeHost(src);
+        if (res) cudaFreeHost(res);
+        *this = SoloGraph();
+    }
+};
+
+// The calling thread's entry for a shape (its least recently used one given
+// up for a new shape).
+SoloGraph *solo_graph(const SoloKey &key) {
+    struct Set {
+        SoloGraph g[kGraphs];
+        uint64_t tick = 0;
+        ~Set() {
+            for (SoloGraph &e : g) e.drop();
+        }
+    };
+    thread_local Set s;
+    SoloGraph *hit = nullptr;
+    for (SoloGraph &e : s.g)
+        if (e.calls > 0 && e.key == key) hit = &e;
+    if (!hit) {
+        hit = &s.g[0];
+        for (SoloGraph &e : s.g)
+            if (e.used < hit->used) hit = &e;
+        hit->drop();
+        hit->key = key;
+    }
+    hit->calls++;
+    hit->used = ++s.tick;
+    return hit;
+}
+
+// Captures the shape's launches; false when it cannot be done.
+bool solo_capture(SoloGraph &g, SoloJob J, cudaStream_t st) {
+    const SoloKey &k = g.key;
+    const int bpp = k.gray ? 4 : k.step;
+    const long long ip = (long long)align_up((size_t)k.iw * k.step, 128), tp = (long long)align_up((size_t)k.tw * k.step, 128);
+    const size_t mapBytes = k.map ? (size_t)(k.iw - k.tw + 1) * (k.ih - k.th + 1) * sizeof(float) : 0;
+    size_t work = 0;
+    J.need = &work;
+    if (run_solo(J, st) != CVM_OK) return false;
+    J.need = nullptr;
+    const size_t oTpl = align_up((size_t)ip * k.ih, 256), oMap = oTpl + align_up((size_t)tp * k.th, 256);
+    const size_t oWork = oMap + align_up(mapBytes, 256), total = oWork + work;
+    if (total > kGraphBytes) return false;
+    const size_t bImg = align_up((size_t)k.iw * bpp, 16) * k.ih, bTpl = align_up((size_t)k.tw * bpp, 16) * k.th;
+    const size_t sImg = bImg <= kGraphStage ? align_up(bImg, 256) : 0, sTpl = bTpl <= kGraphStage ? bTpl : 0;
+    void *dSrc = nullptr, *dRes = nullptr;
+    if (cudaMalloc(&g.mem, total) != cudaSuccess ||
+        cudaHostAlloc(reinterpret_cast<void **>(&g.src), 256 + sImg + sTpl, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostAlloc(reinterpret_cast<void **>(&g.res), sizeof(cvm_result), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&dSrc, g.src, 0) != cudaSuccess ||
+        cudaHostGetDevicePointer(&dRes, g.res, 0) != cudaSuccess)
+        return false;
+    uint8_t *dImg = static_cast<uint8_t *>(g.mem), *dTpl = dImg + oTpl;
+    for (int i = 0; i < 2; i++)
+        if (i ? sTpl : sImg) {
+            g.stage[i] = reinterpret_cast<uint8_t *>(g.src) + 256 + (i ? sImg : 0);
+            g.stageDev[i] = static_cast<uint8_t *>(dSrc) + 256 + (i ? sImg : 0);
+        }
+    g.map = k.map ? reinterpret_cast<float *>(dImg + oMap) : nullptr;
+    J.img = dImg;
+    J.istride = ip;
+    J.tpl = dTpl;
+    J.tstride = tp;
+    J.map = g.map;
+    J.out = static_cast<cvm_result *>(dRes);
+    J.work = dImg + oWork;
+    J.frameOnSide = 0;
+    if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) != cudaSuccess) return false;
+    const uint64_t l0 = g_launches.load();
+    bool ok = launch_ingest_solo(static_cast<const SoloSource *>(dSrc), dImg, ip, k.iw, k.ih, dTpl, tp, k.tw, k.th, bpp,
+                                 k.gray, static_cast<unsigned int *>(J.work), (int)(kSoloZero / 4), st) == cudaSuccess;
+    ok = ok && run_solo(J, st) == CVM_OK;
+    g.launches = (unsigned)(g_launches.load() - l0);
+    cudaGraph_t graph = nullptr;
+    ok = cudaStreamEndCapture(st, &graph) == cudaSuccess && ok && graph;
+    ok = ok && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
+    if (graph) cudaGraphDestroy(graph);
+    return ok;
+}
+
+// The shape's graph when there is one by now (nullptr: queue the call).
+SoloGraph *replayable(const SoloKey &key, const SoloJob &J, cudaStream_t st) {
+    if (!dev().pageable || profile_on()) return nullptr;
+    SoloGraph *g = solo_graph(key);
+    if (g->exec) return g;
+    if (g->failed || g->calls < kGraphCalls) return nullptr;
+    // (a caller's own stream capture on this thread is left alone)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool ok = solo_capture(*g, J, st);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (ok) return g;
+    cudaGetLastError();
+    const int calls = g->calls;
+    const uint64_t used = g->used;
+    g->drop();
+    g->key = key;
+    g->calls = calls;
+    g->used = used;
+    g->failed = true;
+    return nullptr;
+}
+
 int host_solo(const uint8_t *img, long long istride, int iw, int ih, const uint8_t *tpl, long long tstride,
               int tw, int th, int mode, int cnFixed, int step, int grayFromRgba, float *map,
               cvm_result *out, const PeakReq *pk = nullptr) {
     CVM_TRY(ensure_device());
     cudaStream_t st = thread_stream();
     SideStream &ss = side_stream();
+    const int rw = iw - tw + 1, rh = ih - th + 1;
+    SoloJob J;
+    memset(&J, 0, sizeof J);
+    J.form = solo_form();
+    J.iw = iw;
+    J.ih = ih;
+    J.step = step;
+    J.mode = mode;
+    J.cnFixed = cnFixed;
+    J.tw = tw;
+    J.th = th;
+    const SoloKey key{iw, ih, tw, th, mode, cnFixed, step, grayFromRgba, J.form, g_autotune.load(), map || pk ? 1 : 0};
+    if (SoloGraph *g = replayable(key, J, st)) {
+        const int bpp = grayFromRgba ? 4 : step;
+        SoloSource in[2] = {{img, istride}, {tpl, tstride}};
+        for (int i = 0; i < 2; i++)
+            if (g->stage[i]) {
+                const size_t row = (size_t)(i ? tw : iw) * bpp, pitch = align_up(row, 16);
+                const uint8_t *p = i ? tpl : img;
+                for (int y = 0; y < (i ? th : ih); y++)
+                    memcpy(g->stage[i] + y * pitch, p + (long long)y * (i ? tstride : istride), row);
+                in[i] = SoloSource{g->stageDev[i], (long long)pitch};
+            }
+        memcpy(g->src, in, sizeof in);
+        CVM_CUDA(cudaGraphLaunch(g->exec, st));
+        count_launches(g->launches);
+        PoolBuf bp;
+        CVM_TRY(map_results(g->map, rw, rh, map, pk, bp, st));
+        bp.release(st);
+        CVM_CUDA(cudaStreamSynchronize(st));
+        *out = *g->res;
+        return CVM_OK;
+    }
     PoolBuf bi, bt, gi, gt, bm, bo;
     long long ip, tp;
     const int bpp = grayFromRgba ? 4 : step;
@@ -912,7 +1129,6 @@ int host_solo(const uint8_t *img, long long istride, int iw, int ih, const uint8
         ip = gp;
         tp = gtp;
     }
-    const int rw = iw - tw + 1, rh = ih - th + 1;
     float *dMap = nullptr;
     if (map || pk) {
         CVM_TRY(pool_alloc(bm, (size_t)rw * rh * sizeof(float), st));
@@ -923,36 +1139,16 @@ int host_solo(const uint8_t *img, long long istride, int iw, int ih, const uint8
         CVM_TRY(pool_alloc(bo, sizeof(cvm_result), st));
         dOut = static_cast<cvm_result *>(bo.p);
     }
-    SoloJob J;
-    memset(&J, 0, sizeof J);
-    J.form = solo_form();
     J.img = dImg;
     J.istride = ip;
-    J.iw = iw;
-    J.ih = ih;
-    J.step = step;
-    J.mode = mode;
-    J.cnFixed = cnFixed;
     J.tpl = dTpl;
     J.tstride = tp;
-    J.tw = tw;
-    J.th = th;
     J.map = dMap;
     J.out = dOut;
     J.frameOnSide = !grayFromRgba;
     CVM_TRY(run_solo(J, st));
-    if (map) CVM_CUDA(cudaMemcpyAsync(map, dMap, (size_t)rw * rh * sizeof(float), cudaMemcpyDeviceToHost, st));
     PoolBuf bp;
-    if (pk) {
-        const size_t nsc = peaks_scratch_ints(rw, rh);
-        const size_t xyBytes = (size_t)std::max(pk->maxPeaks, 0) * 2 * sizeof(int32_t);
-        CVM_TRY(pool_alloc(bp, (nsc + 1) * sizeof(int) + xyBytes, st));
-        int *scr = static_cast<int *>(bp.p), *dCount = scr + nsc;
-        int32_t *dXY = reinterpret_cast<int32_t *>(dCount + 1);
-        CVM_CUDA(launch_peaks(dMap, rw, rh, pk->thresh, pk->rx, pk->ry, scr, dXY, pk->maxPeaks, dCount, st));
-        CVM_CUDA(cudaMemcpyAsync(pk->count, dCount, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        if (xyBytes) CVM_CUDA(cudaMemcpyAsync(pk->xy, dXY, xyBytes, cudaMemcpyDeviceToHost, st));
-    }
+    CVM_TRY(map_results(dMap, rw, rh, map, pk, bp, st));
     if (!hOut) CVM_CUDA(cudaMemcpyAsync(out, bo.p, sizeof(cvm_result), cudaMemcpyDeviceToHost, st));
     // the device buffers go back to the pool in stream order now, so the
     // host's frees overlap the device work instead of following the wait
@@ -1451,12 +1647,11 @@ int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw
     DevMember *T = A.take<DevMember>(tab.size());
     int *dPoor = A.take<int>(1), poor = 0;
     unsigned int *sat = A.take<unsigned int>(lanes), *blk = A.take<unsigned int>(sat_scratch_elems(ph, hp, np));
-    CVM_CUDA(cudaMemcpyAsync(P, f->dP, n * sizeof(DevParams), cudaMemcpyDeviceToDevice, ts));
     CVM_CUDA(cudaMemsetAsync(F, 0, sizeof(DevFrame), ts));
     CVM_CUDA(cudaMemsetAsync(dPoor, 0, sizeof(int), ts));
     CVM_CUDA(cudaMemcpyAsync(T, tab.data(), tab.size() * sizeof(DevMember), cudaMemcpyHostToDevice, ts));
     CVM_CUDA(launch_prep(nullptr, 0, 0, 0, f->step, 0, f->step == 4 ? dParent : nullptr, pstride, pw, ph, P, n, 0, 0, 0,
-                         F, ts));
+                         F, ts, f->dP));
     CVM_CUDA(launch_sat(dParent, pstride, pw, ph, hp, np, &F->cnMax, blk, sat, ts));
     MemberSet ms;
     memset(&ms, 0, sizeof ms);
@@ -1716,11 +1911,10 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
             }
         }
     } sideJoin{ss, st};
-    CVM_CUDA(cudaMemcpyAsync(P, f->dP, n * sizeof(DevParams), cudaMemcpyDeviceToDevice, st));
-    CVM_CUDA(cudaMemsetAsync(F, 0, sizeof(DevFrame), st));
-    CVM_CUDA(cudaMemsetAsync(bounds, 0, (size_t)3 * n * sizeof(int), st));
+    // F and the extrema and counters behind it, in one
+    CVM_CUDA(cudaMemsetAsync(F, 0, Arena::bytes(1, sizeof(DevFrame)) + (size_t)3 * n * sizeof(int), st));
     CVM_CUDA(launch_prep(nullptr, 0, 0, 0, f->step, 0, f->step == 4 ? dParent : nullptr, pstride, pw, ph, P, n, 0, 0,
-                         0, F, st));
+                         0, F, st, f->dP));
     if (sat) CVM_CUDA(launch_sat(dParent, pstride, pw, ph, hpP, cnP == 4 ? 4 : 2, &F->cnMax, satBlk, sat, st));
     if (anyStatsKernel) CVM_CUDA(launch_row_prefix(dParent, pstride, f->step, pw, ph, cnP, prefix, hpP, st));
     if (prefixBlk) CVM_CUDA(launch_vblock(prefix, prefixBlk, ph / 16, prefixRow, st));

@@ -144,7 +144,8 @@ cudaError_t launch_alpha_scan(const uint8_t *img, long long stride, int w, int h
 // F must be zeroed, or hold cached template sums, before the launch.
 cudaError_t launch_prep(const uint8_t *tpl, long long tstride, int tw, int th, int tstep, int cnStats,
                         const uint8_t *parent, long long pstride, int pw, int ph, DevParams *P, int n,
-                        int setInit, int initMode, int initCnFixed, DevFrame *F, cudaStream_t st);
+                        int setInit, int initMode, int initCnFixed, DevFrame *F, cudaStream_t st,
+                        const DevParams *cached = nullptr);
 // Forward row pass of every tile of `fc` (or of a template: geometry with
 // one 1x1 block whose loads are the template's tw x th).
 // Channels [chanFirst, min(chanCount, *cnDev)) are transformed.
@@ -227,12 +228,15 @@ SepGrid sep_grid(int rwMax, int rhMax);
 // (optional): k_vstats runs on vst, ordered after k_hsum by the event vev.
 // blk (optional): one match, (ih/16) x hp x stat_pitch(cnMax) u32 for the
 // 16-row block sums of H, from which each band starts (tall templates),
-// built here; a fleet (sharedPrefix), the block sums of the prefix's main
+// built here; cnKnown: the match's channel count when it is fixed (k_hsum then
+// reads no params), and prepared an event that k_vstats waits for, after which
+// the params hold; a fleet (sharedPrefix), the block sums of the prefix's main
 // block built by launch_vblock.
 cudaError_t launch_sep_stats(const uint8_t *img, long long istride, int step, int iw, int ih, const MemberSet &ms,
                              int nmembers, int soloTw, int soloRw, const SepGrid &sg, int cnMin, int cnMax,
                              unsigned int *H, size_t slotStride, cudaStream_t st, int sharedPrefix = 0,
-                             cudaStream_t vst = nullptr, cudaEvent_t vev = nullptr, unsigned int *blk = nullptr);
+                             cudaStream_t vst = nullptr, cudaEvent_t vev = nullptr, unsigned int *blk = nullptr,
+                             int cnKnown = 0, cudaEvent_t prepared = nullptr);
 // The 16-row block sums of rows of rowElems u32 (block b = rows 16b ..
 // 16b+15, the rows' layout), nblk blocks: a vertical slide starts from them.
 cudaError_t launch_vblock(const unsigned int *H, unsigned int *B, int nblk, size_t rowElems, cudaStream_t st);
@@ -264,6 +268,18 @@ cudaError_t upload_bytes(void *dst, const void *src, size_t n, cudaStream_t st);
 // at src into device memory, by a kernel reading over the host link.
 cudaError_t launch_ingest(void *dst, size_t dpitch, const void *src, size_t spitch, size_t rowBytes, int rows,
                           cudaStream_t st);
+// A one-shot call's inputs by one kernel: the frame and the template, from
+// device-accessible host memory at the addresses and row strides that arg[0]
+// and arg[1] (mapped page-locked memory) hold when the kernel runs, into
+// device planes of the given pitches; gray: RGBA inputs, stored as rgbToGray's
+// bytes.  Also clears zeroWords words at zero.
+struct alignas(16) SoloSource {
+    const uint8_t *pix;
+    long long stride;
+};
+cudaError_t launch_ingest_solo(const SoloSource *arg, uint8_t *dImg, long long ipitch, int iw, int ih, uint8_t *dTpl,
+                               long long tpitch, int tw, int th, int bpp, int gray, unsigned int *zero, int zeroWords,
+                               cudaStream_t st);
 cudaError_t launch_shrink_gather(const float2 *src, int dftH, float2 *dst, int dh2, int hwp, int cnS,
                                  cudaStream_t st);
 
@@ -306,6 +322,7 @@ void set_error_message(const char *msg);
 
 // per-kernel event timing (exported by cvm_profile_enable/cvm_profile_read)
 void profile_enable(int on);
+bool profile_on();
 int profile_read(int i, char *name, size_t len, double *ms, unsigned long long *count);
 int profile_span(int i, char *name, size_t len, double *t0, double *t1);
 

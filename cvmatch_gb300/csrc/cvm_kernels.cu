@@ -320,6 +320,7 @@ struct PrepArgs {
     int pw, ph, parentCtas;
     int pvec16;              // parent rows 16-byte aligned: scan with vector loads
     DevParams *P;
+    const DevParams *cached; // the template statistics when they are not accumulated in P (nullptr: P's)
     int n;                   // params to finalize
     int setInit;             // store mode/cnFixed/tw/th of `init` into P[0] first
     int initMode, initCnFixed;
@@ -437,7 +438,7 @@ __global__ void k_prep(PrepArgs a) {
     F.alphaMismatch = ((volatile DevFrame *)a.F)->alphaMismatch;
     for (int i = tid; i < a.n; i += nt) {
         DevParams p;
-        const volatile DevParams *src = a.P + i;
+        const volatile DevParams *src = (a.cached ? a.cached : a.P) + i;
         for (int k = 0; k < 4; k++) {
             p.tsum[k] = src->tsum[k];
             p.tsq[k] = src->tsq[k];
@@ -1319,6 +1320,7 @@ struct HsumArgs {
     int first;
     const DevParams *params;
     int pIdx;                 // solo member params index
+    int cn;                   // the channel count when it is fixed (0: in the params)
 };
 
 template <int CN>
@@ -1518,10 +1520,11 @@ __global__ void __launch_bounds__(256) k_hsum(HsumArgs a) {
         pIdx = m.pIdx;
     }
     const DevParams &Pm = a.params[pIdx];
-    if (Pm.flat) return;
-    if (Pm.cn == CNA)
+    if (!a.cn && Pm.flat) return;
+    const int cn = a.cn ? a.cn : Pm.cn;
+    if (cn == CNA)
         hsum_row<CNA>(a, slot, tw, rw, sp, wsum);
-    else if (CNB != CNA && Pm.cn == CNB)
+    else if (CNB != CNA && cn == CNB)
         hsum_row<CNB>(a, slot, tw, rw, sp, wsum);
 }
 
@@ -2021,6 +2024,93 @@ __global__ void k_ingest(unsigned char *__restrict__ dst, size_t dpitch, const u
     }
 }
 
+// One plane of a one-shot call's inputs, rows of w pixels of BPP bytes; GRAY:
+// RGBA to gray on the way.  Sixteen-byte items where the source allows them.
+template <typename V, int PER, bool GRAY>
+__device__ __forceinline__ void ingest_items(const uint8_t *src, long long spitch, uint8_t *dst, long long dpitch,
+                                             int perRow, int rows, int cta, int ctas) {
+    const long long items = (long long)perRow * rows, stride = (long long)ctas * blockDim.x;
+    for (long long i0 = (long long)cta * blockDim.x + threadIdx.x; i0 < items; i0 += 4 * stride) {
+        V v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const long long i = i0 + k * stride;
+            if (i < items) {
+                const long long y = i / perRow;
+                v[k] = reinterpret_cast<const V *>(src + y * spitch)[i - y * perRow];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const long long i = i0 + k * stride;
+            if (i >= items) continue;
+            const long long y = i / perRow, x = i - y * perRow;
+            if constexpr (GRAY) {
+                const unsigned int *c = reinterpret_cast<const unsigned int *>(&v[k]);
+#pragma unroll
+                for (int q = 0; q < PER; q++)
+                    dst[y * dpitch + x * PER + q] = (uint8_t)((4899u * (c[q] & 255u) + 9617u * ((c[q] >> 8) & 255u) +
+                                                               1868u * ((c[q] >> 16) & 255u) + 8192u) >> 14);
+            } else {
+                reinterpret_cast<V *>(dst + y * dpitch)[x] = v[k];
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void ingest_plane(const uint8_t *src, long long spitch, uint8_t *dst, long long dpitch, int w,
+                                             int rows, int bpp, int gray, int cta, int ctas) {
+    const unsigned long long a = reinterpret_cast<unsigned long long>(src) | (unsigned long long)spitch |
+                                 (unsigned long long)(w * bpp);
+    if (gray) {
+        // (RGBA pixels at any byte address)
+        if ((a & 15) == 0) {
+            ingest_items<uint4, 4, true>(src, spitch, dst, dpitch, w / 4, rows, cta, ctas);
+        } else if ((a & 3) == 0) {
+            ingest_items<unsigned int, 1, true>(src, spitch, dst, dpitch, w, rows, cta, ctas);
+        } else {
+            const long long items = (long long)w * rows, stride = (long long)ctas * blockDim.x;
+            for (long long i = (long long)cta * blockDim.x + threadIdx.x; i < items; i += stride) {
+                const long long y = i / w, x = i - y * w;
+                const uint8_t *p = src + y * spitch + 4 * x;
+                dst[y * dpitch + x] = (uint8_t)((4899u * p[0] + 9617u * p[1] + 1868u * p[2] + 8192u) >> 14);
+            }
+        }
+    } else if ((a & 15) == 0) {
+        ingest_items<uint4, 1, false>(src, spitch, dst, dpitch, w * bpp / 16, rows, cta, ctas);
+    } else if ((a & 3) == 0) {
+        ingest_items<unsigned int, 1, false>(src, spitch, dst, dpitch, w * bpp / 4, rows, cta, ctas);
+    } else {
+        ingest_items<unsigned char, 1, false>(src, spitch, dst, dpitch, w * bpp, rows, cta, ctas);
+    }
+}
+
+// The first kIngestTpl CTAs take the template (and clear `zero`), the others
+// the frame: every CTA waits for the host twice, for its addresses and for its
+// pixels, and both planes wait at the same time.
+constexpr int kIngestTpl = 8;
+
+__global__ void __launch_bounds__(256) k_ingest_solo(const SoloSource *arg, uint8_t *dImg, long long ipitch, int iw,
+                                                     int ih, uint8_t *dTpl, long long tpitch, int tw, int th, int bpp,
+                                                     int gray, unsigned int *zero, int zeroWords) {
+    __shared__ ulonglong2 a;
+    const bool tpl = (int)blockIdx.x < kIngestTpl;
+    if (threadIdx.x == 0) {
+        // (address, row stride) in one 16-byte read of mapped host memory
+        const SoloSource *p = arg + (tpl ? 1 : 0);
+        asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(a.x), "=l"(a.y) : "l"(p));
+    }
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < zeroWords; i += 256) zero[i] = 0u;
+    __syncthreads();
+    const uint8_t *src = reinterpret_cast<const uint8_t *>(a.x);
+    if (tpl)
+        ingest_plane(src, (long long)a.y, dTpl, tpitch, tw, th, bpp, gray, blockIdx.x, kIngestTpl);
+    else
+        ingest_plane(src, (long long)a.y, dImg, ipitch, iw, ih, bpp, gray, blockIdx.x - kIngestTpl,
+                     gridDim.x - kIngestTpl);
+}
+
 // Small host values to device memory through kernel arguments.
 struct UploadBlob {
     unsigned char bytes[3072];
@@ -2078,7 +2168,7 @@ cudaError_t launch_alpha_scan(const uint8_t *img, long long stride, int w, int h
 
 cudaError_t launch_prep(const uint8_t *tpl, long long tstride, int tw, int th, int tstep, int cnStats,
                         const uint8_t *parent, long long pstride, int pw, int ph, DevParams *P, int n,
-                        int setInit, int initMode, int initCnFixed, DevFrame *F, cudaStream_t st) {
+                        int setInit, int initMode, int initCnFixed, DevFrame *F, cudaStream_t st, const DevParams *cached) {
     PrepArgs a;
     a.tpl = tpl;
     a.tstride = tstride;
@@ -2099,6 +2189,7 @@ cudaError_t launch_prep(const uint8_t *tpl, long long tstride, int tw, int th, i
     a.parentCtas = parent ? (ph < 304 ? ph : 304) : 0;
     a.pvec16 = parent && (reinterpret_cast<uintptr_t>(parent) & 15) == 0 && (pstride & 15) == 0;
     a.P = P;
+    a.cached = cached;
     a.n = n;
     a.setInit = setInit;
     a.initMode = initMode;
@@ -2234,11 +2325,9 @@ cudaError_t launch_cols(int mode, const float2 *in, float2 *out, int cnS, const 
     if (SC < 1) SC = 1;
     a.SC = SC;
     a.logSC = ilog2i(SC);
-    // the generic kernels take (strip, channel, tile x member); the fixed
-    // heights' fleet modes take (tile x member, channel, strip)
-    const int strips = (fc.hw + SC - 1) / SC;
-    dim3 grid(strips, chanCount, fc.ntiles * (mode == 0 ? 1 : nmembers));
-    if (mode >= 2 && cols_fixed_length(fc.log2H)) grid = dim3(fc.ntiles * nmembers, mode == 3 ? 1 : chanCount, strips);
+    // the generic kernels take (strip, channel, tile x member)
+    const int strips = (fc.hw + SC - 1) / SC, targets = fc.ntiles * (mode == 0 ? 1 : nmembers);
+    const dim3 grid(strips, chanCount, targets);
     const size_t smem = (size_t)fc.dftH * SC * sizeof(float2);
     ProfScope ps(label ? label
                        : (mode == 0 ? "k_cols_fwd"
@@ -2258,7 +2347,7 @@ cudaError_t launch_cols(int mode, const float2 *in, float2 *out, int cnS, const 
         return cudaGetLastError();
     }
     if (cols_fixed_length(fc.log2H)) {
-        launch_cols_fixed(a, grid, smem, st);
+        launch_cols_fixed(a, chanCount, targets, st);
     } else if ((fc.log2H & 1) == 0 && fc.dftH >= 4) {
         if (mode == 0) {
             set_smem(k_cols_even<0>, smem);
@@ -2442,7 +2531,7 @@ static int vstat_band(const SepGrid &sg, int nmembers) {
 cudaError_t launch_sep_stats(const uint8_t *img, long long istride, int step, int iw, int ih, const MemberSet &ms,
                              int nmembers, int soloTw, int soloRw, const SepGrid &sg, int cnMin, int cnMax,
                              unsigned int *H, size_t slotStride, cudaStream_t st, int sharedPrefix,
-                             cudaStream_t vst, cudaEvent_t vev, unsigned int *blk) {
+                             cudaStream_t vst, cudaEvent_t vev, unsigned int *blk, int cnKnown, cudaEvent_t prepared) {
     // a shared 4-channel prefix keeps its (s3, alpha squares) block after
     // the ih x hp x 4 main block (launch_row_prefix)
     HsumArgs h;
@@ -2460,6 +2549,7 @@ cudaError_t launch_sep_stats(const uint8_t *img, long long istride, int step, in
     h.first = ms.first;
     h.params = ms.params;
     h.pIdx = ms.solo.pIdx;
+    h.cn = cnKnown;
     VstatArgs v;
     v.H = H;
     v.slotStride = slotStride;
@@ -2512,6 +2602,10 @@ cudaError_t launch_sep_stats(const uint8_t *img, long long istride, int step, in
         if (e == cudaSuccess) e = cudaStreamWaitEvent(vst, vev, 0);
         if (e != cudaSuccess) return e;
         st = vst;
+    }
+    if (prepared) {
+        const cudaError_t e = cudaStreamWaitEvent(st, prepared, 0);
+        if (e != cudaSuccess) return e;
     }
     if (sharedPrefix) v.blk = blk;  // a fleet's block sums, built once per frame (launch_vblock)
     if (v.blk && !sharedPrefix) {
@@ -2673,6 +2767,19 @@ cudaError_t upload_bytes(void *dst, const void *src, size_t n, cudaStream_t st) 
     return cudaSuccess;
 }
 
+cudaError_t launch_ingest_solo(const SoloSource *arg, uint8_t *dImg, long long ipitch, int iw, int ih, uint8_t *dTpl,
+                               long long tpitch, int tw, int th, int bpp, int gray, unsigned int *zero, int zeroWords,
+                               cudaStream_t st) {
+    // a CTA per 4 KB of the frame (four 16-byte items a thread would leave
+    // most of the SMs without any), up to four per SM
+    const long long want = ((long long)iw * ih * bpp + 4095) / 4096;
+    const int ctas = (int)std::max(1LL, std::min(4LL * 152, want));
+    k_ingest_solo<<<kIngestTpl + ctas, 256, 0, st>>>(arg, dImg, ipitch, iw, ih, dTpl, tpitch, tw, th, bpp, gray, zero,
+                                                     zeroWords);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_shrink_gather(const float2 *src, int dftH, float2 *dst, int dh2, int hwp, int cnS,
                                  cudaStream_t st) {
     const long long total = (long long)cnS * dh2 * hwp;
@@ -2694,6 +2801,11 @@ void profile_enable(int on) {
         if (prof::origin) cudaEventDestroy(prof::origin);
         prof::origin = nullptr;
     }
+}
+
+bool profile_on() {
+    std::lock_guard<std::mutex> lk(prof::mu);
+    return prof::on;
 }
 
 int profile_span(int i, char *name, size_t len, double *t0, double *t1) {

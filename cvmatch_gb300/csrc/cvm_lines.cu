@@ -140,14 +140,15 @@ __device__ __noinline__ Track score_table(Track t, float num, const MemberSet &m
 // CTAs spill: 1.17 against 0.84 ms).
 __host__ __device__ constexpr int lines_ctas(int L, bool fast, int mode) {
     return mode == 2 ? (L == 11 ? 4 : (L <= 8 ? 8 : 9))
-                     : (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 7) : (fast ? 10 : 8))) * (mode ? 4 : 3) / 4;
+                     : (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 5) : (fast ? 10 : 8))) * (mode ? 4 : 3) / 4;
 }
 
 // What a launch keeps of its results.  ALL: every score may be wanted (a
 // score map, regions of interest).  LANES: the extrema alone, den (and t)
 // from the statistics kernel's lanes.  TABLE: a fast-form fleet's extrema,
-// den on demand.
-enum Keep { ALL, LANES, TABLE };
+// den on demand.  SOLO: LANES for a single match, whose CTAs all start at once
+// with no extrema of earlier ones to cut by (fleets keep their registers).
+enum Keep { ALL, LANES, TABLE, SOLO };
 
 // The extrema (and scores) of the CTA's row pairs.
 template <int L, bool FAST, Keep MODE>
@@ -268,8 +269,6 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
             }
             if (k + 1 < cn || p + NL < P) prefetch(k + 1 < cn ? p : p + NL, k + 1 < cn ? k + 1 : 0);
             group_sync<G>(mask);
-            float2 z[16];
-            pass2<L, true, FAST>(ln, j2, b2, z, triW);
             const bool last = k == cn - 1;
             const bool odd = 2 * (pair0 + p) + 1 < bh;  // the imaginary part's row exists
             const int y0 = tb.y0 + 2 * (pair0 + p);
@@ -297,6 +296,8 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                     }
                 }
             };
+            float2 z[16];
+            pass2<L, true, FAST>(ln, j2, b2, z, triW);
             if constexpr (AHEAD) {
                 // every unit's, in flight together while the barrier gathers the line
 #pragma unroll
@@ -330,10 +331,46 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                     }
                     continue;
                 }
+                // the correlation of result i of row h, the earlier channels' sum
+                // and t applied (the exact form)
+                auto numer = [&](int h, int i) {
+                    float num = h ? o[i].y : o[i].x;
+                    if constexpr (!FAST) {
+                        const float2 s = acc[it * RL + i];
+                        if (cn > 1) num = __fadd_rn(h ? s.y : s.x, num);
+                        num = __fsub_rn(num, tt[BOTH ? h : 0][i]);
+                    }
+                    return num;
+                };
+                if (MODE == SOLO && it == 0 && !warm) {
+                    // No extrema to start from (a single match's CTAs all start
+                    // at once): the largest and smallest quotients of the warp's
+                    // first unit, by the hardware division, as cuts -- within
+                    // 2^-22 of scores that are there, cut at 2^-18.  (Without
+                    // them nearly all its results took the ladder, 2000 of the
+                    // 2500 instructions of a 128-point line's warp.)
+                    float qx = -FLT_MAX, qn = FLT_MAX;
+#pragma unroll
+                    for (int h = 0; h < (BOTH ? 2 : 1); h++)
+#pragma unroll
+                        for (int i = 0; i < RL; i++) {
+                            const float num = numer(h, i), d = den[AHEAD ? it : 0][BOTH ? h : 0][i];
+                            const float q = __fdividef(num, d);
+                            if (jj + HL * i < bw && fabsf(num) < d) {
+                                qx = fmaxf(qx, q);
+                                qn = fminf(qn, q);
+                            }
+                        }
+                    qx = from_key(__reduce_max_sync(mask, ordered_key(qx)));
+                    qn = -from_key(__reduce_max_sync(mask, ordered_key(-qn)));
+                    if (qx > -FLT_MAX) t.hi = fmaxf(t.hi, qx - (fabsf(qx) * 3.814697265625e-06f + 1e-15f));
+                    if (qn < FLT_MAX) t.lo = fminf(t.lo, qn + (fabsf(qn) * 3.814697265625e-06f + 1e-15f));
+                    warm = true;
+                }
                 // cuts on either side of 0, or none: a lower bound of den needs
                 // them so, and a zero den is then the score 0 between them
                 const float hp = t.hi > 0.f ? t.hi : -INFINITY, lp = t.lo < 0.f ? t.lo : INFINITY;
-                const float zero = MODE == LANES && t.hi > 0.f && t.lo < 0.f ? 0.f : -1.f;
+                const float zero = MODE != TABLE && t.hi > 0.f && t.lo < 0.f ? 0.f : -1.f;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     if (h == 1 && !odd) break;
@@ -342,12 +379,7 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
 #pragma unroll
                     for (int i = 0; i < RL; i++) {
                         const int x = jj + HL * i, l = (2 * p + h) * N + x;
-                        float num = h ? o[i].y : o[i].x;
-                        if constexpr (!FAST) {
-                            const float2 s = acc[it * RL + i];
-                            if (cn > 1) num = __fadd_rn(h ? s.y : s.x, num);
-                            num = __fsub_rn(num, tt[BOTH ? h : 0][i]);
-                        }
+                        const float num = numer(h, i);
                         const float d = den[AHEAD ? it : 0][BOTH && MODE != TABLE ? h : 0][i];
                         const bool cand = x < bw && d != zero && !(num < hp * d && num > lp * d);
                         if constexpr (MODE == TABLE) {
@@ -361,7 +393,7 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                         }
                     }
                 }
-                if (LEAN && it == 0 && !warm) {
+                if (LEAN && MODE != SOLO && it == 0 && !warm) {
                     cut_share(t, mask);
                     warm = true;
                 }
@@ -479,13 +511,15 @@ void lines_one(const InvArgs &a, dim3 grid, cudaStream_t st) {
 
 template <int L>
 void lines_form(const InvArgs &a, dim3 grid, cudaStream_t st) {
-    const bool all = a.ms.map || a.ms.anyRoi;
+    const Keep k = a.ms.map || a.ms.anyRoi ? ALL : (a.ms.table ? LANES : SOLO);
     if (!a.ms.form)
-        all ? lines_one<L, false, ALL>(a, grid, st) : lines_one<L, false, LANES>(a, grid, st);
+        k == ALL ? lines_one<L, false, ALL>(a, grid, st)
+                 : (k == SOLO ? lines_one<L, false, SOLO>(a, grid, st) : lines_one<L, false, LANES>(a, grid, st));
     else if (a.ms.sat)
         lines_one<L, true, TABLE>(a, grid, st);
     else
-        all ? lines_one<L, true, ALL>(a, grid, st) : lines_one<L, true, LANES>(a, grid, st);
+        k == ALL ? lines_one<L, true, ALL>(a, grid, st)
+                 : (k == SOLO ? lines_one<L, true, SOLO>(a, grid, st) : lines_one<L, true, LANES>(a, grid, st));
 }
 
 }  // namespace
