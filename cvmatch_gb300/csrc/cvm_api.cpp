@@ -623,28 +623,29 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
                             nullptr, nullptr, fast ? 1 : 0));
         CVM_CUDA(cudaEventRecord(ss.join, ss.st));
     }
-    // A fast-form colour match with a short template (the fused column pass
-    // dominates; the statistics have slack until the inverse rows) queues its
+    // A fast-form colour match of a small frame and a short template queues its
     // horizontal sums behind the frame's row transform, at the caller's
-    // priority, so they fill the SMs the transforms leave instead of
-    // displacing the row transform; otherwise the statistics start after
-    // k_prep, above it.
-    const bool statsLate = !known && fastSum && J.th <= 64;
-    // Otherwise, on a frame of 2^20 pixels or more, the frame's row
-    // transform of every channel the alpha scans cannot drop (all but a
-    // colour match's alpha plane) runs on the rows stream (the caller's
-    // priority) from before k_prep, which only the alpha plane's transform,
-    // the statistics and the template chain wait for; k_prep, ready at once
-    // on the caller's stream, still places its CTAs first.  (A small frame
-    // or a late statistics chain loses more to the extra cross-stream
-    // waits and the side chains it exposes: a 640x480 gray match with a
-    // 64x48 template 70.3 -> 73.4 us, a 1920x1080 colour match with a 96x32
-    // template 92.8 -> 96.6 us in the fast form; the same match in the exact
-    // form 118.5 -> 113 us, a 3840x2160 gray match with a 256x256 template
-    // 209.6 -> 202.7 us in the fast form.)
-    const bool split = !known && !statsLate && (long long)J.iw * J.ih >= (1LL << 20);
+    // priority, so they fill the SMs the transforms leave instead of displacing
+    // the row transform (1280x720 with a 57x41 template: 56.7 us, 59.9 with the
+    // statistics after k_prep, above it); on a frame of 2^20 pixels or more the
+    // late vertical pass ends after the columns (1920x1080 with 96x32: 85.2 us,
+    // 84.1 the other way).
+    const bool large = (long long)J.iw * J.ih >= (1LL << 20);
+    const bool statsLate = !known && fastSum && J.th <= 64 && !large;
+    // A colour frame of 2^20 pixels or more: the row transform of every channel
+    // the alpha scans cannot drop (all but the alpha plane) runs on the rows
+    // stream (the caller's priority) from before k_prep, which only the alpha
+    // plane's transform, the statistics and the template chain wait for; k_prep,
+    // ready at once on the caller's stream, still places its CTAs first.  (A
+    // 1920x1080 match with a 96x32 template, exact: 118.5 -> 113 us; a small
+    // frame or a late statistics chain loses more to the extra cross-stream
+    // waits and the side chains it exposes.)
+    const bool split = !known && !statsLate && large;
     if (!known && J.frameOnSide) CVM_CUDA(cudaStreamWaitEvent(st, ss.frame, 0));
-    cudaStream_t pst = known ? ss.stats : st;  // k_prep's stream
+    // k_prep's stream, and the statistics': a large frame with a fixed channel
+    // count runs them at the caller's priority, beside its rows instead of above
+    // them (3840x2160 gray with 256x256: 202.5 -> 190.8 us)
+    cudaStream_t pst = known ? (large ? ss.st2 : ss.stats) : st;
     if (known) {
         CVM_CUDA(cudaStreamWaitEvent(ss.stats, ss.fork, 0));
         CVM_CUDA(cudaStreamWaitEvent(ss.st2, ss.fork, 0));
@@ -664,7 +665,7 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
                                      spec[c], cnS, ss.stats, 0, nullptr, 1.0f, fast ? off : nullptr));
         CVM_CUDA(cudaEventRecord(ss.rows, ss.stats));
     }
-    cudaStream_t sst = statsLate ? ss.stats : ss.st2;
+    cudaStream_t sst = statsLate || (known && large) ? ss.stats : ss.st2;
     CVM_CUDA(cudaEventRecord(ss.prep, pst));
     if (!early) CVM_CUDA(cudaStreamWaitEvent(ss.st, ss.prep, 0));
     if (!known) CVM_CUDA(cudaStreamWaitEvent(sst, ss.prep, 0));

@@ -626,6 +626,22 @@ __device__ __forceinline__ void ldv(unsigned int *o, const unsigned int *p) {
     }
 }
 
+// The same from shared memory (NP = 2 or 4).
+template <int NP>
+__device__ __forceinline__ void lds(unsigned int *o, const unsigned int *p) {
+    if constexpr (NP == 2) {
+        const uint2 t = *reinterpret_cast<const uint2 *>(p);
+        o[0] = t.x;
+        o[1] = t.y;
+    } else {
+        const uint4 t = *reinterpret_cast<const uint4 *>(p);
+        o[0] = t.x;
+        o[1] = t.y;
+        o[2] = t.z;
+        o[3] = t.w;
+    }
+}
+
 template <int NP>
 __device__ __forceinline__ void stv(unsigned int *p, const unsigned int *v) {
     if constexpr (NP == 2) {
