@@ -38,6 +38,8 @@
 #include <algorithm>
 #include <cstring>
 
+#include <type_traits>
+
 #include "cvm_device.cuh"
 
 namespace cvm {
@@ -870,12 +872,12 @@ __device__ __forceinline__ unsigned long long rn_bits(unsigned long long a, int 
 // u32->f32 rounding, and the exponent is then adjusted exactly.
 __device__ __forceinline__ float u64_to_f32_rn(unsigned long long a) {
     const unsigned int hi = (unsigned int)(a >> 32), lo = (unsigned int)a;
-    if (hi == 0) return __uint2float_rn(lo);
-    const int sh = 32 - __clz(hi);  // bits above the low word, 1..32
-    const unsigned int t = (unsigned int)(a >> sh);
-    const unsigned int dropped = sh == 32 ? lo : (lo & ((1u << sh) - 1u));
-    const float f = __uint2float_rn(t | (dropped != 0u));
-    return __int_as_float(__float_as_int(f) + (sh << 23));
+    const int sh = 32 - __clz(hi);  // bits above the low word, 0..32
+    const unsigned int t = __funnelshift_rc(lo, hi, sh);
+    unsigned int dropped;           // lo's low sh bits, at the top (the shift clamps at 32)
+    asm("shl.b32 %0, %1, %2;" : "=r"(dropped) : "r"(lo), "r"(32 - sh));
+    const float f = __uint2float_rn(t | min(dropped, 1u));
+    return __int_as_float(__float_as_int(f) + (sh << 23));  // (0 + 0 when a is 0)
 }
 
 // float32(float64(v)) (impl.go:902-1009): the conversion to float64 rounds
@@ -1874,7 +1876,16 @@ __global__ void __launch_bounds__(256) k_den_poor(const __grid_constant__ Member
 // FAST (the fleet's fast form, zero-mean template spectra): the
 // correlation already is the numerator, so only den is stored, one float
 // per result (the first half of the member's lanes slot).
-template <int CN, bool PRE, int PCN, bool FAST = false>
+// SMALL: every squared window sum fits 32 bits (area * cn * 255^2 < 2^32: up to
+// 22,016 RGB pixels), hence also every cross and variance numerator 53: the
+// 64-bit products and the reference's two-step conversion shrink to one
+// multiply and one rounding.  (The exact form's statistics are bound by their
+// instructions.  64 RGB templates of 24..96 pixels a side on 1920x1080: 172
+// instructions a result before, 99 now, and with the 128-row bands 790 -> 472
+// us; the same bands without SMALL 577, with its one rounding but a 64-bit
+// squared sum 573.  A 53-bit middle step, larger templates with one rounding,
+// gains nothing on RGB, so there is none.)
+template <int CN, bool PRE, int PCN, bool FAST, bool SMALL>
 __device__ __forceinline__ void vstat_cols(const VstatArgs &a, const DevMember &m, const DevParams &Pm) {
     constexpr int NP = PRE ? (PCN == 4 ? 4 : stat_pitch_c(PCN)) : stat_pitch_c(CN);
     // PRE (a fleet wave): members vary fastest across the grid, so the
@@ -1925,7 +1936,7 @@ __device__ __forceinline__ void vstat_cols(const VstatArgs &a, const DevMember &
         }
     };
     unsigned int s[CN];
-    unsigned long long q = 0;
+    typename std::conditional<SMALL, unsigned int, unsigned long long>::type q = 0;
 #pragma unroll
     for (int k = 0; k < CN; k++) s[k] = 0u;
     int dy0 = 0;
@@ -1951,7 +1962,7 @@ __device__ __forceinline__ void vstat_cols(const VstatArgs &a, const DevMember &
         for (int k = 0; k < CN; k++) s[k] += hv[k];
         q += hv[CN];
     }
-    const unsigned long long area = (unsigned long long)m.tw * th;
+    const unsigned int area = (unsigned int)m.tw * th;
     const unsigned int t0 = (unsigned int)Pm.tsum[0], t1 = (unsigned int)Pm.tsum[1];
     const unsigned int t2 = (unsigned int)Pm.tsum[2], t3 = (unsigned int)Pm.tsum[3];
     const float eps = 1.1920928955078125e-06f;  // 10 * 2^-23
@@ -1961,13 +1972,14 @@ __device__ __forceinline__ void vstat_cols(const VstatArgs &a, const DevMember &
     // A fleet's prefix differences (two loads per row) keep RB = 1: the
     // batch's registers cost more occupancy than its loads in flight gain.
     constexpr int RB = PRE ? 1 : 4;
-    for (int yb = Y0; yb < Y0 + Bv; yb += RB) {
+    const unsigned int *pin = H + (size_t)(Y0 + th) * rp, *pout = H + (size_t)Y0 * rp;
+    for (int yb = Y0; yb < Y0 + Bv; yb += RB, pin += RB * rp, pout += RB * rp) {
         unsigned int hinB[RB][CN + 1], houtB[RB][CN + 1];
 #pragma unroll
         for (int r = 0; r < RB; r++)
             if (yb + r + 1 < Y0 + Bv) {
-                rowvals(H + (size_t)(yb + r + th) * rp, hinB[r]);
-                rowvals(H + (size_t)(yb + r) * rp, houtB[r]);
+                rowvals(pin + r * rp, hinB[r]);
+                rowvals(pout + r * rp, houtB[r]);
             }
 #pragma unroll
         for (int r = 0; r < RB; r++) {
@@ -1993,10 +2005,11 @@ __device__ __forceinline__ void vstat_cols(const VstatArgs &a, const DevMember &
             // FAST: the exact variance numerator from its two 32-bit halves
             // (within 1.5 ulp; the reference's two-step float64 -> float32
             // conversion is kept otherwise)
-            const unsigned long long idv = area * q - sq;
+            const unsigned long long idv = (unsigned long long)area * q - sq;
+            auto exact = [](unsigned long long v) { return SMALL ? u64_to_f32_rn(v) : f32_via_f64((long long)v); };
             const float id = FAST ? fmaf(__uint2float_rn((unsigned int)(idv >> 32)), 4294967296.0f,
                                          __uint2float_rn((unsigned int)idv))
-                                  : f32_via_f64((long long)idv);
+                                  : exact(idv);
             const float diff2 = __fmul_rn(id, Pm.varScale);
             float lim = 0.5f;
             if (q < (1ull << 24)) {
@@ -2010,13 +2023,14 @@ __device__ __forceinline__ void vstat_cols(const VstatArgs &a, const DevMember &
             if (FAST) {
                 dens[(size_t)y * m.rw] = den;
             } else {
-                const float l0 = CN == 1 ? __uint2float_rn(s[0]) : f32_via_f64((long long)cross);
+                const float l0 = CN == 1 ? __uint2float_rn(s[0]) : exact(cross);
                 lanes[(size_t)y * m.rw] = make_float2(__fmul_rn(l0, Pm.numScale), den);
             }
             if (more) {
 #pragma unroll
                 for (int k = 0; k < CN; k++) s[k] += hin[k] - hout[k];
-                q += (unsigned long long)hin[CN] - (unsigned long long)hout[CN];
+                q += hin[CN];
+                q -= hout[CN];
             }
         }
     }
@@ -2027,10 +2041,18 @@ __global__ void __launch_bounds__(256) k_vstats(VstatArgs a) {
     const DevMember &m = member_of(a.ms, PRE ? blockIdx.x : blockIdx.z);
     const DevParams &Pm = a.ms.params[m.pIdx];
     if (Pm.flat) return;
-    if (Pm.cn == CNA)
-        vstat_cols<CNA, PRE, CNB, FAST>(a, m, Pm);
-    else if (CNB != CNA && Pm.cn == CNB)
-        vstat_cols<CNB, PRE, CNB, FAST>(a, m, Pm);
+    const bool small = (unsigned long long)m.tw * m.th * Pm.cn * 65025ull < (1ull << 32);
+    if (Pm.cn == CNA) {
+        if (small)
+            vstat_cols<CNA, PRE, CNB, FAST, true>(a, m, Pm);
+        else
+            vstat_cols<CNA, PRE, CNB, FAST, false>(a, m, Pm);
+    } else if (CNB != CNA && Pm.cn == CNB) {
+        if (small)
+            vstat_cols<CNB, PRE, CNB, FAST, true>(a, m, Pm);
+        else
+            vstat_cols<CNB, PRE, CNB, FAST, false>(a, m, Pm);
+    }
 }
 
 // Frame ingest from page-locked host memory: the GPU reads the caller's
@@ -2556,13 +2578,16 @@ SepGrid sep_grid(int rwMax, int rhMax) {
 
 // Band height of the vertical slide: every band first sums th rows, so
 // taller bands amortise that start over more results; the band stays at 16
-// rows unless the launch has CTAs to spare (~6 per SM at the taller band),
-// and at most 256 (a 78-member wave of 2560x1440 statistics: bands of 128
-// rows 3.03 ms, 256 rows 2.91, 512 rows 3.09, 1024 rows 3.61 -- the
-// tallest leave too few CTAs per SM).
+// rows unless the launch has CTAs to spare (~6 per SM at the taller band, and
+// for the step from 128 to 256 rows ~24: with fewer the last wave of CTAs
+// costs more than the starts; 64 RGB members on 1920x1080, 2048 CTAs at 256
+// rows: 539 us, at 128: 472), and at most 256 (a 78-member wave of 2560x1440
+// statistics, 4680 CTAs at 256 rows: bands of 128 rows 3.03 ms, 256 rows
+// 2.91, 512 rows 3.09, 1024 rows 3.61 -- the tallest leave too few CTAs per SM).
 static int vstat_band(const SepGrid &sg, int nmembers) {
     int BV = 16;
-    while (BV < 256 && (long long)sg.ncx * ((sg.rhMax + 2 * BV - 1) / (2 * BV)) * nmembers >= 6 * 152) BV *= 2;
+    while (BV < 256 && (long long)sg.ncx * ((sg.rhMax + 2 * BV - 1) / (2 * BV)) * nmembers >= (BV < 128 ? 6 : 24) * 152)
+        BV *= 2;
     return BV;
 }
 
