@@ -137,10 +137,17 @@ __device__ __noinline__ Track score_table(Track t, float num, const MemberSet &m
 // thread's 32 den values ahead of the last pass (12 CTAs spill: 2.13 against
 // 2.01 ms; without them 14 CTAs 2.00 at the same 4096 elements per CTA); the
 // exact form keeps the channel sum of its 16 results, 128 registers (nine
-// CTAs spill: 1.17 against 0.84 ms).
+// CTAs spill: 1.17 against 0.84 ms).  With every score (mode 0) the quotients
+// of all results are in flight: three quarters of the CTAs, but all of them
+// for the fast form's 2048 points (a 4K gray map: three CTAs 56.6 us, four
+// 50.6, five 46.9, six 48.4) and six for the exact form's 256 points (1280x800
+// with 32x32, RGB: three 27.6 us, six 22.7, seven 24.8; 128 points: three
+// 32.9, six 35.0).
 __host__ __device__ constexpr int lines_ctas(int L, bool fast, int mode) {
-    return mode == 2 ? (L == 11 ? 4 : (L <= 8 ? 8 : 9))
-                     : (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 5) : (fast ? 10 : 8))) * (mode ? 4 : 3) / 4;
+    return mode == 2                   ? (L == 11 ? 4 : (L <= 8 ? 8 : 9))
+           : mode == 0 && L == 8 && !fast ? 6
+                                       : (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 5) : (fast ? 10 : 8))) *
+                                             (mode || (L == 11 && fast) ? 4 : 3) / 4;
 }
 
 // What a launch keeps of its results.  ALL: every score may be wanted (a
