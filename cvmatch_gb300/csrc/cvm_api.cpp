@@ -627,11 +627,12 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     // horizontal sums behind the frame's row transform, at the caller's
     // priority, so they fill the SMs the transforms leave instead of displacing
     // the row transform (1280x720 with a 57x41 template: 56.7 us, 59.9 with the
-    // statistics after k_prep, above it); on a frame of 2^20 pixels or more the
+    // statistics after k_prep, above it).  On a frame of 2^20 pixels or more the
     // late vertical pass ends after the columns (1920x1080 with 96x32: 85.2 us,
-    // 84.1 the other way).
+    // 84.1 the other way), unless a queued call's frame still has to arrive
+    // (from host memory 159 us, 166 the other way).
     const bool large = (long long)J.iw * J.ih >= (1LL << 20);
-    const bool statsLate = !known && fastSum && J.th <= 64 && !large;
+    const bool statsLate = !known && fastSum && J.th <= 64 && (!large || J.frameOnSide);
     // A colour frame of 2^20 pixels or more: the row transform of every channel
     // the alpha scans cannot drop (all but the alpha plane) runs on the rows
     // stream (the caller's priority) from before k_prep, which only the alpha
@@ -947,6 +948,14 @@ struct SoloKey {
     }
 };
 
+// Allocations, frees and captures of this scope are this thread's own affair: a
+// caller's capture, on this thread or another, neither refuses nor sees them.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 struct SoloGraph {
     SoloKey key{};
     int calls = 0;       // of the shape so far
@@ -960,6 +969,7 @@ struct SoloGraph {
     cudaGraphExec_t exec = nullptr;
     unsigned launches = 0;
     void drop() {
+        RelaxedCapture relaxed;
         if (exec) cudaGraphExecDestroy(exec);
         if (mem) cudaFree(mem);
         if (src) cudaFreeHost(src);
@@ -1050,12 +1060,10 @@ SoloGraph *replayable(const SoloKey &key, const SoloJob &J, cudaStream_t st) {
     SoloGraph *g = solo_graph(key);
     if (g->exec) return g;
     if (g->failed || g->calls < kGraphCalls) return nullptr;
-    // (a caller's own stream capture on this thread is left alone)
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const bool ok = solo_capture(*g, J, st);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (ok) return g;
+    {
+        RelaxedCapture relaxed;
+        if (solo_capture(*g, J, st)) return g;
+    }
     cudaGetLastError();
     const int calls = g->calls;
     const uint64_t used = g->used;
