@@ -636,8 +636,7 @@ def _workload_config(key, ws, args):
         return {"workload": f"Fleet.FindAll, {args.templates} RGBA templates 16..192 x 16..128 (70% a*x+b shifted "
                             "crops, 30% absent) on a 2560x1440 RGBA frame", "parent": [2560, 1440],
                 "templates": args.templates, "channels": "RGBA (cn=3 after the alpha scans)", "l2": l2,
-                "parallelism": par, **({"stats": "inverse-rows epilogue"} if getattr(args, "stats", "kernel")
-                                       == "epilogue" else {}),
+                "parallelism": par, **({"stats": args.stats} if getattr(args, "stats", "auto") != "auto" else {}),
                 **({"overlap": "off"} if getattr(args, "overlap", "on") == "off" else {}),
                 **({"wave": args.wave} if getattr(args, "wave", 0) else {})}
     if key == "match":
@@ -1087,8 +1086,8 @@ def run_gpu(args):
     key = args.workload
     if key == "fleet":
         W = FleetWorkload(cvm, torch, dev, stream, count=args.templates)
-        if args.stats == "epilogue":
-            W.fleet.SetStats(cvm.STATS_EPILOGUE)
+        if args.stats != "auto":
+            W.fleet.SetStats(cvm.STATS_EPILOGUE if args.stats == "epilogue" else cvm.STATS_KERNEL)
         W.overlap = args.overlap == "on"
         W.fleet.SetOverlap(W.overlap)
         W.fleet.SetWave(args.wave)
@@ -1288,9 +1287,10 @@ def main():
     ap.add_argument("--timeline", action="store_true", help="print one profiled step's launch spans to stderr")
     ap.add_argument("--autotune", default="on", choices=["on", "off"],
                     help="the fast forms' tile-plan autotuner (cvm_set_autotune); off runs newGoPlan's plans")
-    ap.add_argument("--stats", default="kernel", choices=["kernel", "epilogue"],
-                    help="--workload fleet: window statistics from the statistics kernel (default) or formed in "
-                         "the inverse-rows epilogue from the frame's summed-area table (cvm_fleet_set_stats)")
+    ap.add_argument("--stats", default="auto", choices=["auto", "kernel", "epilogue"],
+                    help="--workload fleet: window statistics from the statistics kernel, or formed in the "
+                         "inverse-rows epilogue from the frame's summed-area table (cvm_fleet_set_stats); auto: "
+                         "the library chooses on its first frame")
     ap.add_argument("--wave", type=int, default=0,
                     help="--workload fleet: member tails per wave (cvm_fleet_set_wave; 0: the workspace budget's)")
     ap.add_argument("--overlap", default="on", choices=["on", "off"],

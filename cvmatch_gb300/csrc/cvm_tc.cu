@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_selftest(const TcTables *_
 
 // --------------------------------------------------------- inverse rows
 
-// The fast form's fused inverse rows (k_inv_rows_t<10, true> with the
+// The fast form's fused inverse rows (k_inv_lines<10, true> with the
 // radix-4 cascade replaced): four row pairs per MMA tile, pairsPerCta row
 // pairs per CTA (the same grid and partial records as the FP32 kernel).
 __global__ void __launch_bounds__(kTcThreads, 4) k_inv_rows_tc(InvArgs a) {
