@@ -313,7 +313,9 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                     load_den(it, 1);
                 }
             }
-            if (LEAN && last && posted) warm = cut_keys(t, keys.x, keys.y) || warm;
+            // `warm` gates collectives of the group's lanes, and other CTAs
+            // post while the lanes read: one answer for all of them
+            if (LEAN && last && posted) warm = __all_sync(mask, cut_keys(t, keys.x, keys.y)) || warm;
             if constexpr (NB > 1) group_sync<G>(mask);
 #pragma unroll
             for (int it = 0; it < NU; it++) {
