@@ -383,6 +383,7 @@ struct SoloJob {
     int form;         // CVM_FORM_EXACT, _FAST or _MIXED (cached spectra must be of this form)
     const Plan *plan; // the tile plan (one-shot; nullptr: the tuned plan, or newGoPlan)
     void *work;       // the workspace, its head cleared (nullptr: taken from the pool for the call)
+    size_t workBytes; // its size
     size_t *need;     // report the workspace's size and queue nothing
 };
 
@@ -424,23 +425,30 @@ std::mutex g_tuneMu;
 std::map<TuneKey, TuneEntry> g_tune;
 std::atomic<int> g_autotune{1};
 
+TuneKey tune_key(const SoloJob &J) {
+    return TuneKey{J.iw, J.ih, J.tw, J.th, J.mode, J.mode == 1 ? 0 : J.cnFixed, J.step, J.form};
+}
+
+// The plan of J's shape when nothing is left to measure for it: newGoPlan's in
+// the exact form or with tuning off, or the tuned one.
+bool settled_plan(const SoloJob &J, int autotune, Plan *out) {
+    *out = make_plan(J.tw, J.th, J.iw - J.tw + 1, J.ih - J.th + 1);
+    if (J.form == CVM_FORM_EXACT || !autotune) return true;
+    std::lock_guard<std::mutex> lk(g_tuneMu);
+    auto it = g_tune.find(tune_key(J));
+    if (it == g_tune.end()) return false;
+    *out = it->second.plan;
+    return true;
+}
+
 // The plan a fast-form one-shot match of J's shape runs (tuning it first
 // when needed); *out = newGoPlan's plan when tuning is off or not possible.
 int solo_plan(const SoloJob &J, cudaStream_t st, Plan *out) {
     const int rw = J.iw - J.tw + 1, rh = J.ih - J.th + 1;
-    *out = make_plan(J.tw, J.th, rw, rh);
-    if (J.form == CVM_FORM_EXACT || !g_autotune.load()) return CVM_OK;
-    const TuneKey key{J.iw, J.ih, J.tw, J.th, J.mode, J.mode == 1 ? 0 : J.cnFixed, J.step, J.form};
-    {
-        std::lock_guard<std::mutex> lk(g_tuneMu);
-        auto it = g_tune.find(key);
-        if (it != g_tune.end()) {
-            *out = it->second.plan;
-            return CVM_OK;
-        }
-    }
+    if (settled_plan(J, g_autotune.load(), out)) return CVM_OK;
+    const TuneKey key = tune_key(J);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (!J.img || cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return CVM_OK;
     }
@@ -545,6 +553,7 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
         *J.need = bytes;
         return CVM_OK;
     }
+    if (J.work && bytes > J.workBytes) return fail(CVM_ERR_ARGS, "cvmatch_gpu: workspace too small");
     PoolBuf buf;
     if (!J.work) CVM_TRY(pool_alloc(buf, bytes, st));
     Arena A;
@@ -1004,13 +1013,16 @@ SoloGraph *solo_graph(const SoloKey &key) {
     return hit;
 }
 
-// Captures the shape's launches; false when it cannot be done.
-bool solo_capture(SoloGraph &g, SoloJob J, cudaStream_t st) {
+// Captures the shape's launches on the given plan; false when it cannot be
+// done.  (One plan for the workspace's size and for the launches in it: other
+// threads may switch the autotuner or tune the shape meanwhile.)
+bool solo_capture(SoloGraph &g, SoloJob J, const Plan &plan, cudaStream_t st) {
     const SoloKey &k = g.key;
     const int bpp = k.gray ? 4 : k.step;
     const long long ip = (long long)align_up((size_t)k.iw * k.step, 128), tp = (long long)align_up((size_t)k.tw * k.step, 128);
     const size_t mapBytes = k.map ? (size_t)(k.iw - k.tw + 1) * (k.ih - k.th + 1) * sizeof(float) : 0;
     size_t work = 0;
+    J.plan = &plan;
     J.need = &work;
     if (run_solo(J, st) != CVM_OK) return false;
     J.need = nullptr;
@@ -1040,6 +1052,7 @@ bool solo_capture(SoloGraph &g, SoloJob J, cudaStream_t st) {
     J.map = g.map;
     J.out = static_cast<cvm_result *>(dRes);
     J.work = dImg + oWork;
+    J.workBytes = work;
     J.frameOnSide = 0;
     if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) != cudaSuccess) return false;
     const uint64_t l0 = g_launches.load();
@@ -1059,10 +1072,11 @@ SoloGraph *replayable(const SoloKey &key, const SoloJob &J, cudaStream_t st) {
     if (!dev().pageable || profile_on()) return nullptr;
     SoloGraph *g = solo_graph(key);
     if (g->exec) return g;
-    if (g->failed || g->calls < kGraphCalls) return nullptr;
+    Plan plan;
+    if (g->failed || g->calls < kGraphCalls || !settled_plan(J, key.tune, &plan)) return nullptr;
     {
         RelaxedCapture relaxed;
-        if (solo_capture(*g, J, st)) return g;
+        if (solo_capture(*g, J, plan, st)) return g;
     }
     cudaGetLastError();
     const int calls = g->calls;
