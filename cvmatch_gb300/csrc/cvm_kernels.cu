@@ -1328,20 +1328,22 @@ struct HsumArgs {
 
 // A warp owns a span of the row's columns and scans it 128 at a time, four
 // adjacent columns a thread (one load of 16 bytes where the row allows it);
-// the exclusive prefixes go to shared memory, one 16-byte slot per column (a
-// spare slot every eight keeps the strided stores off each other's banks), and
-// every output takes two of them.  (Each thread prefixed a segment of the row
+// the exclusive prefixes go to shared memory, one 16-byte slot per column (8
+// bytes up to two channels; a spare slot every eight keeps the strided stores off
+// each other's banks), and every output takes two of them.  (Each thread prefixed a segment of the row
 // in shared memory, one plane after another: alone, a 1920x1080 RGBA frame 18
 // us, 13 now; in whole calls, Find on 1280x720 60.0 -> 56.7 us, 1366x767 with
 // four channels 114 -> 109.)
 template <int CN>
 __device__ __forceinline__ void hsum_row(const HsumArgs &a, int slot, int tw, int rw, unsigned int *sp,
                                          unsigned int (*wsum)[5]) {
-    constexpr int NL = CN + 1, NM = CN == 1 ? 2 : 4, NP = stat_pitch_c(CN);
+    // (slots of two words: s and the squares, or two channels)
+    constexpr int NL = CN + 1, NM = CN <= 2 ? 2 : 4, NP = stat_pitch_c(CN);
+    constexpr bool EXT = NL > NM;
     const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     const int iw = a.iw, pad = a.padShift;
     const uint8_t *row = a.img + (long long)r * a.istride;
-    unsigned int *ext = sp + (size_t)NM * (iw + 1 + (iw >> pad));  // CN == 4: the squares' plane
+    unsigned int *ext = sp + (size_t)NM * (iw + 1 + (iw >> pad));  // EXT: the squares' plane
     const size_t align = reinterpret_cast<size_t>(row);
     const bool vec = a.step == 4 ? (align & 15) == 0 : (a.step == 1 && (align & 3) == 0);
     const bool words = a.step == 4 && (align & 3) == 0;
@@ -1432,7 +1434,7 @@ __device__ __forceinline__ void hsum_row(const HsumArgs &a, int slot, int tw, in
 #pragma unroll
                 for (int q = 0; q < NM; q++) m[q] = q < NL ? left[q < NL ? q : 0] : 0u;
                 stv<NM>(sp + (size_t)NM * (x + i + ((x + i) >> pad)), m);
-                if (CN == 4) ext[x + i] = left[CN];
+                if (EXT) ext[x + i] = left[CN];
             }
 #pragma unroll
             for (int q = 0; q < NL; q++) left[q] += v[i][q];
@@ -1448,7 +1450,7 @@ __device__ __forceinline__ void hsum_row(const HsumArgs &a, int slot, int tw, in
         lds<NM>(hi, sp + (size_t)NM * (e + (e >> pad)));
 #pragma unroll
         for (int q = 0; q < NP; q++) v[q] = q < NM && q < NL ? hi[q < NM ? q : 0] - lo[q < NM ? q : 0] : 0u;
-        if (CN == 4) v[CN < NP ? CN : 0] = ext[e] - ext[x];
+        if (EXT) v[CN < NP ? CN : 0] = ext[e] - ext[x];
         stv<NP>(H + (size_t)x * NP, v);
     }
 }
@@ -2642,7 +2644,8 @@ cudaError_t launch_sep_stats(const uint8_t *img, long long istride, int step, in
     }
     // the prefixes' slots (the widest rows do without the spare ones)
     const auto slots = [&](int pad) {
-        return ((size_t)(cnMax == 1 ? 2 : 4) * (iw + 1 + (iw >> pad)) + (cnMax == 4 ? iw + 1 : 0)) * sizeof(unsigned int);
+        return ((size_t)(cnMax <= 2 ? 2 : 4) * (iw + 1 + (iw >> pad)) + (cnMax == 2 || cnMax == 4 ? iw + 1 : 0)) *
+               sizeof(unsigned int);
     };
     h.padShift = slots(3) <= 200 * 1024 ? 3 : 31;
     const size_t smem = slots(h.padShift);
