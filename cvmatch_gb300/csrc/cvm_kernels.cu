@@ -1663,7 +1663,7 @@ __device__ __forceinline__ void sat_lanes(unsigned int c, unsigned int *v, unsig
 
 template <int NP>
 __global__ void __launch_bounds__(256) k_sat_cols(SatArgs a) {
-    const int x = blockIdx.x * 256 + threadIdx.x, y0 = blockIdx.y * kSatRows;
+    const int x = blockIdx.y * 256 + threadIdx.x, y0 = blockIdx.x * kSatRows;
     if (x >= a.iw) return;
     unsigned int v[NP] = {}, w[2] = {}, c[kSatRows];
 #pragma unroll
@@ -1678,7 +1678,7 @@ __global__ void __launch_bounds__(256) k_sat_cols(SatArgs a) {
         w[0] += pw[0];
         w[1] += pw[1];
     }
-    const size_t e = (size_t)blockIdx.y * a.hp + x;
+    const size_t e = (size_t)blockIdx.x * a.hp + x;
     stv<NP>(a.B + e * NP, v);
     if (NP == 4 && *a.cnMax == 4) stv<2>(a.Ba + e * 2, w);
 }
@@ -2761,7 +2761,7 @@ cudaError_t launch_sat(const uint8_t *img, long long istride, int iw, int ih, in
     a.Ba = np == 4 ? B + (size_t)a.nb * hp * 4 : nullptr;
     a.S = S;
     a.Sa = np == 4 ? S + (size_t)(ih + 1) * hp * 4 : nullptr;
-    const dim3 gc((iw + 255) / 256, a.nb);
+    const dim3 gc(a.nb, (iw + 255) / 256);  // (a grid's y ends at 65,535)
     const int gs = (iw * np + 31) / 32;
     ProfScope ps("k_sat", st);
     if (np == 4) {
