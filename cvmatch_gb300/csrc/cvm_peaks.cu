@@ -12,10 +12,10 @@
 //
 // Nearly every result is rejected by its score or by one of its eight
 // neighbours; what is left is a local maximum, and only those look at their
-// whole window, one after another, a warp's lanes along its rows.  (One
-// thread per result scanning its window from the corner, in the count and
-// again in the write: 90 + 86 us on a 1249 x 769 map with 33 x 33 windows and
-// the threshold 0.3; now 30 + 6.)
+// whole window.  A warp whose candidates are few takes them one after another,
+// its lanes along the window's rows; with many of them (small windows, plateaus
+// of equal scores) each lane scans its own.  kLaneScan has the line and its
+// figures.
 #include "cvm_device.cuh"
 
 namespace cvm {
@@ -23,27 +23,65 @@ namespace {
 
 constexpr int kPeakCols = 256;
 
+// A lane's own scan of its window costs the warp one load per window position;
+// a candidate taken by the warp one batch of eight loads per eight rows and 32
+// columns started, and the batch's latency: as long as kLaneScan positions.
+// Measured on 1249 x 769 maps with lines at 8, 16, 32 and 64: 17 x 17 windows
+// of noise 89, 82, 65 and 62 us, 33 x 33 of scattered equal peaks 308, 282, 229
+// and 261, 81 x 81 of noise 112, 112, 237 and 246.  Every candidate taken by
+// the warp: a plateau with 3 x 3 windows 406 us, with 9 x 9 735, 9 x 9 noise 85;
+// now 21, 49 and 43.
+constexpr int kLaneScan = 32;
+
 // The recipe's test, with its comparisons: a score that is not below the
 // threshold (NaN included) is a candidate, and any strictly greater
 // neighbour rejects it.  Every lane of the warp takes part.
 __device__ __forceinline__ unsigned int peak_bits(const float *__restrict__ m, int w, int h, int x, int y, float thresh,
                                                   int rx, int ry) {
     const int lane = threadIdx.x & 31;
-    bool cand = false;
     float v = 0.f;
+    bool cand = false;
     if (x < w) {
-        const float *p = m + (size_t)y * w + x;
-        v = *p;
+        v = m[(size_t)y * w + x];
         cand = !(v < thresh);
+    }
+    if (cand) {
+        // the neighbours inside the window and the map, all eight in flight
+        // (others stand in as the result itself, which rejects nothing)
+        const int xl = rx > 0 ? max(x - 1, 0) : x, xr = rx > 0 ? min(x + 1, w - 1) : x;
+        const int yu = ry > 0 ? max(y - 1, 0) : y, yd = ry > 0 ? min(y + 1, h - 1) : y;
+        const float *u = m + (size_t)yu * w, *c = m + (size_t)y * w, *d = m + (size_t)yd * w;
+        const bool g = (u[xl] > v) | (u[x] > v) | (u[xr] > v) | (c[xl] > v) | (c[xr] > v) | (d[xl] > v) | (d[x] > v) |
+                       (d[xr] > v);
+        cand = !g;
+    }
+    unsigned int left = __ballot_sync(0xffffffffu, cand);
+    if (rx <= 1 && ry <= 1) return left;  // the neighbours are the window
+    const long long batches = (long long)((2 * ry + 8) / 8) * ((2 * rx + 32) / 32);
+    if ((2 * rx + 1LL) * (2 * ry + 1) <= kLaneScan * batches * __popc(left)) {
         if (cand) {
-            const int x0 = rx > 0 && x > 0 ? -1 : 0, x1 = rx > 0 && x + 1 < w ? 1 : 0;
-            const int y0 = ry > 0 && y > 0 ? -1 : 0, y1 = ry > 0 && y + 1 < h ? 1 : 0;
-            for (int dy = y0; dy <= y1; dy++)
-                for (int dx = x0; dx <= x1; dx++) cand = cand && !(p[(long long)dy * w + dx] > v);
+            const int x0 = max(0, x - rx), x1 = min(w - 1, x + rx), y0 = max(0, y - ry), y1 = min(h - 1, y + ry);
+            // a row at a time, four of up to three columns
+            const int step = rx <= 1 ? 4 : 1;
+            for (int r = y0; r <= y1 && cand; r += step) {
+                bool g = false;
+                if (rx <= 1) {
+                    for (int c = x0; c <= x1; c++) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) g |= m[(size_t)min(r + i, y1) * w + c] > v;
+                    }
+                } else {
+                    const float *row = m + (size_t)r * w;
+#pragma unroll 4
+                    for (int c = x0; c <= x1; c++) g |= row[c] > v;
+                }
+                cand = !g;
+            }
         }
+        return __ballot_sync(0xffffffffu, cand);
     }
     unsigned int bits = 0u;
-    for (unsigned int left = __ballot_sync(0xffffffffu, cand); left; left &= left - 1) {
+    for (; left; left &= left - 1) {
         const int l = __ffs(left) - 1, cx = x - lane + l;
         const float cv = __shfl_sync(0xffffffffu, v, l);
         const int x0 = max(0, cx - rx), x1 = min(w - 1, cx + rx), y0 = max(0, y - ry), y1 = min(h - 1, y + ry);
@@ -105,21 +143,30 @@ __global__ void __launch_bounds__(1024) k_peaks_scan(int *counts, int n, int *to
     if (tid == 1023) *total = part[1023];
 }
 
-// One thread per 32 results.
+// A thread per 32 results finds their place; the warp writes the words that
+// have any one after another, a lane per result.
 __global__ void __launch_bounds__(256) k_peaks_write(const int *__restrict__ offsets,
                                                      const unsigned int *__restrict__ masks, int nxb, int words,
                                                      int32_t *xy, int maxPeaks) {
     constexpr int kWords = kPeakCols / 32;
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= words) return;
-    unsigned int b = masks[i];
-    if (!b) return;
+    const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31;
+    const unsigned int b = i < words ? masks[i] : 0u;
     const int block = i / kWords, word = i - block * kWords, y = block / nxb;
-    int idx = offsets[block];
-    for (int k = 0; k < word; k++) idx += __popc(masks[block * kWords + k]);
-    for (; b && idx < maxPeaks; b &= b - 1, idx++) {
-        xy[2 * idx] = (block - y * nxb) * kPeakCols + 32 * word + __ffs(b) - 1;
-        xy[2 * idx + 1] = y;
+    const int x = (block - y * nxb) * kPeakCols + 32 * word;
+    int idx = 0;
+    if (b) {
+        idx = offsets[block];
+        for (int k = 0; k < word; k++) idx += __popc(masks[block * kWords + k]);
+    }
+    for (unsigned int left = __ballot_sync(0xffffffffu, b && idx < maxPeaks); left; left &= left - 1) {
+        const int l = __ffs(left) - 1;
+        const unsigned int bl = __shfl_sync(0xffffffffu, b, l);
+        const int at = __shfl_sync(0xffffffffu, idx, l) + __popc(bl & ((1u << lane) - 1u));
+        const int xl = __shfl_sync(0xffffffffu, x, l) + lane, yl = __shfl_sync(0xffffffffu, y, l);
+        if ((bl >> lane & 1u) && at < maxPeaks) {
+            xy[2 * (size_t)at] = xl;
+            xy[2 * (size_t)at + 1] = yl;
+        }
     }
 }
 
