@@ -197,13 +197,24 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
         lgy = block_log2(m.th);
         nbx = (bw + (1 << lgx) - 1) >> lgx;
         const int rows = min(2 * P, bh - 2 * pair0), n = nbx * ((rows + (1 << lgy) - 1) >> lgy);
+        bool flat = true;
 #pragma unroll 1
         for (int i = tid; i < n; i += S::CTA) {
             const int by = i / nbx, x = (i - by * nbx) << lgx, y = by << lgy;
-            lbs[i] = block_bound(a.ms, m, Pm, tb.y0 + 2 * pair0 + y, tb.x0 + x, min(1 << lgx, bw - x),
-                                 min(1 << lgy, rows - y));
+            const float lb = block_bound(a.ms, m, Pm, tb.y0 + 2 * pair0 + y, tb.x0 + x, min(1 << lgx, bw - x),
+                                         min(1 << lgy, rows - y));
+            lbs[i] = lb;
+            flat = flat && lb == INFINITY;
         }
-        __syncthreads();
+        // No deviation in any window of the CTA (a black frame, a letterbox's
+        // bars): every den and so every score is 0, whatever the correlation.
+        // 64 templates on a black 1920x1080 frame: 1.81 ms with the
+        // transforms, 0.62 without; with den from the statistics kernel 1.32.
+        if (__syncthreads_and(flat)) {
+            ext_init(e);
+            if (tid == 0) ext_add(e, 0.f, (long long)(tb.y0 + 2 * pair0) * m.rw + tb.x0);
+            return e;
+        }
     }
     Track t = {FLT_MAX, -FLT_MAX, -INFINITY, INFINITY, INT_MAX, INT_MAX};
     // rows r and r + 1 of channel k
