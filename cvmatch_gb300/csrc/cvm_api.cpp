@@ -188,6 +188,21 @@ SideStream &side_stream() {
     return s;
 }
 
+// A host-buffer call that ends early waits for what it queued: the device may
+// still be reading the caller's pixels or the thread's staging, and using
+// buffers that the call's end gives back.  (Declared after the call's buffers,
+// so that it runs before they are released.)
+struct Settle {
+    cudaStream_t st;
+    bool done = false;  // the call has waited by itself
+    ~Settle() {
+        if (done) return;
+        SideStream &ss = side_stream();
+        for (cudaStream_t s : {st, ss.st, ss.st2, ss.stats, ss.waveRows}) cudaStreamSynchronize(s);
+        cudaGetLastError();
+    }
+};
+
 const float2 *dev_tri(int n) {
     DeviceState &d = dev();
     std::lock_guard<std::mutex> lk(d.triMu);
@@ -606,6 +621,24 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     // orders only the CTAs waiting for a slot), so k_prep is the launch
     // that is ready first.
     SideStream &ss = side_stream();
+    // An error return joins the side streams into st, in whose order the
+    // workspace goes back to the pool.
+    struct Join {
+        SideStream &ss;
+        cudaStream_t st;
+        bool done;
+        ~Join() {
+            if (done) return;
+            cudaStreamCaptureStatus a = cudaStreamCaptureStatusNone, b = a;
+            cudaStreamIsCapturing(st, &a);
+            for (cudaStream_t s : {ss.st, ss.st2, ss.stats})
+                if (cudaStreamIsCapturing(s, &b) == cudaSuccess && a == b) {
+                    cudaEventRecord(ss.join, s);
+                    cudaStreamWaitEvent(st, ss.join, 0);
+                }
+            cudaGetLastError();
+        }
+    } join{ss, st, false};
     // A one-shot colour match on a device-resident frame starts its template
     // spectrum at once, beside k_prep: all four channels (the frame's alpha
     // plane decides later whether the fourth is used) and, in the fast form,
@@ -748,6 +781,7 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     for (int c = 0; c < G->nclass; c++)
         CVM_CUDA(launch_inv_rows(G->g, G->fc[c], c, fast ? 1 : cnS, ms, 1, G->g.blockH, partOff[c], nparts, parts,
                                  &F->normDone, J.out, st, 0, F->bounds));
+    join.done = true;
     return CVM_OK;
 }
 
@@ -1119,16 +1153,19 @@ int host_solo(const uint8_t *img, long long istride, int iw, int ih, const uint8
                 in[i] = SoloSource{g->stageDev[i], (long long)pitch};
             }
         memcpy(g->src, in, sizeof in);
+        PoolBuf bp;
+        Settle settle{st};
         CVM_CUDA(cudaGraphLaunch(g->exec, st));
         count_launches(g->launches);
-        PoolBuf bp;
         CVM_TRY(map_results(g->map, rw, rh, map, pk, bp, st));
         bp.release(st);
         CVM_CUDA(cudaStreamSynchronize(st));
+        settle.done = true;
         *out = *g->res;
         return CVM_OK;
     }
-    PoolBuf bi, bt, gi, gt, bm, bo;
+    PoolBuf bi, bt, gi, gt, bm, bo, bp;
+    Settle settle{st};
     long long ip, tp;
     const int bpp = grayFromRgba ? 4 : step;
     // The frame moves in on the second side stream (the long transfer,
@@ -1170,7 +1207,6 @@ int host_solo(const uint8_t *img, long long istride, int iw, int ih, const uint8
     J.out = dOut;
     J.frameOnSide = !grayFromRgba;
     CVM_TRY(run_solo(J, st));
-    PoolBuf bp;
     CVM_TRY(map_results(dMap, rw, rh, map, pk, bp, st));
     if (!hOut) CVM_CUDA(cudaMemcpyAsync(out, bo.p, sizeof(cvm_result), cudaMemcpyDeviceToHost, st));
     // the device buffers go back to the pool in stream order now, so the
@@ -1183,6 +1219,7 @@ int host_solo(const uint8_t *img, long long istride, int iw, int ih, const uint8
     bp.release(st);
     bo.release(st);
     CVM_CUDA(cudaStreamSynchronize(st));
+    settle.done = true;
     if (hOut) *out = *hOut;
     return CVM_OK;
 }
@@ -2269,12 +2306,14 @@ int cvm_rgba_to_gray(const uint8_t *pix, int64_t stride, int w, int h, uint8_t *
     CVM_TRY(ensure_device());
     cudaStream_t st = thread_stream();
     PoolBuf bi, bo;
+    Settle settle{st};
     long long ip;
     CVM_TRY(upload_image(bi, pix, stride, w, h, 4, &ip, st));
     CVM_TRY(pool_alloc(bo, (size_t)w * h, st));
     CVM_CUDA(launch_gray(static_cast<const uint8_t *>(bi.p), ip, w, h, static_cast<uint8_t *>(bo.p), w, st));
     CVM_CUDA(cudaMemcpyAsync(out, bo.p, (size_t)w * h, cudaMemcpyDeviceToHost, st));
     CVM_CUDA(cudaStreamSynchronize(st));
+    settle.done = true;
     return CVM_OK;
 }
 
@@ -2295,6 +2334,7 @@ int cvm_alpha_const(const uint8_t *pix, int64_t stride, int w, int h, int *out) 
     CVM_TRY(ensure_device());
     cudaStream_t st = thread_stream();
     PoolBuf bi, bf;
+    Settle settle{st};
     long long ip;
     CVM_TRY(upload_image(bi, pix, stride, w, h, 4, &ip, st));
     CVM_TRY(pool_alloc(bf, sizeof(unsigned int), st));
@@ -2303,6 +2343,7 @@ int cvm_alpha_const(const uint8_t *pix, int64_t stride, int w, int h, int *out) 
     unsigned int mism = 0;
     CVM_CUDA(cudaMemcpyAsync(&mism, bf.p, sizeof mism, cudaMemcpyDeviceToHost, st));
     CVM_CUDA(cudaStreamSynchronize(st));
+    settle.done = true;
     *out = mism == 0;
     return CVM_OK;
 }
@@ -2374,12 +2415,14 @@ int cvm_matcher_find(cvm_matcher *m, const uint8_t *parent, int64_t pstride, int
     }
     cudaStream_t st = thread_stream();
     PoolBuf bi, bo;
+    Settle settle{st};
     long long ip;
     CVM_TRY(upload_image(bi, parent, pstride, pw, ph, m->step, &ip, st));
     CVM_TRY(pool_alloc(bo, sizeof(cvm_result), st));
     CVM_TRY(matcher_find_dev(m, static_cast<const uint8_t *>(bi.p), ip, pw, ph, static_cast<cvm_result *>(bo.p), st));
     CVM_CUDA(cudaMemcpyAsync(out, bo.p, sizeof(cvm_result), cudaMemcpyDeviceToHost, st));
     CVM_CUDA(cudaStreamSynchronize(st));
+    settle.done = true;
     return CVM_OK;
 }
 
@@ -2422,12 +2465,14 @@ int cvm_fleet_find_all(cvm_fleet *f, const uint8_t *parent, int64_t pstride, int
                         ph);
     cudaStream_t st = thread_stream();
     PoolBuf bi, bo;
+    Settle settle{st};
     long long ip;
     CVM_TRY(upload_image(bi, parent, pstride, pw, ph, f->step, &ip, st));
     CVM_TRY(pool_alloc(bo, n * sizeof(cvm_result), st));
     CVM_TRY(fleet_find_dev(f, static_cast<const uint8_t *>(bi.p), ip, pw, ph, static_cast<cvm_result *>(bo.p), st));
     CVM_CUDA(cudaMemcpyAsync(out, bo.p, n * sizeof(cvm_result), cudaMemcpyDeviceToHost, st));
     CVM_CUDA(cudaStreamSynchronize(st));
+    settle.done = true;
     return CVM_OK;
 }
 

@@ -45,6 +45,67 @@ void plan_changes_during_the_capture(bool off) {
     EXPECT(rows == std::set<int>{128});
 }
 
+// Every call that queues work fails once, in every host-buffer entry point:
+// an error return leaves nothing behind that still reads the caller's memory.
+void errors_wait() {
+    cvm_set_form(CVM_FORM_EXACT);
+    const int w = 700, h = 300, tw = 40, th = 30;
+    std::vector<float> map((size_t)(w - tw + 1) * (h - th + 1));
+    std::vector<uint8_t> gray((size_t)w * h);
+    cvm_matcher *m[2];
+    for (int i = 0; i < 2; i++) {
+        tpl[4 * i] = 7;
+        EXPECT(cvm_matcher_new(tpl.data(), 4 * tw, tw, th, 4, &m[i]) == CVM_OK);
+    }
+    cvm_fleet *f;
+    EXPECT(cvm_fleet_new(m, 2, &f) == CVM_OK);
+    cvm_result r[2];
+    int32_t xy[20], n;
+    int c;
+    const std::vector<std::function<int()>> entries = {
+        [&] { return call(w, h, tw, th); },
+        [&] { return cvm_match_gray_rgba(frame.data(), 4 * w, w, h, tpl.data(), 4 * tw, tw, th, r); },
+        [&] { return cvm_match_map(frame.data(), 4 * w, w, h, tpl.data(), 4 * tw, tw, th, map.data()); },
+        [&] { return cvm_match_map_peaks(frame.data(), 4 * w, w, h, tpl.data(), 4 * tw, tw, th, 0.5f, 2, 2, xy, 10, &n); },
+        [&] { return cvm_matcher_find(m[0], frame.data(), 4 * w, w, h, r); },
+        [&] { return cvm_fleet_find_all(f, frame.data(), 4 * w, w, h, r); },
+        [&] { return cvm_rgba_to_gray(frame.data(), 4 * w, w, h, gray.data()); },
+        [&] { return cvm_alpha_const(frame.data(), 4 * w, w, h, &c); },
+    };
+    auto &st = fake::state();
+    const std::set<std::string> reads = {"ingest", "ingest_solo", "cudaMemcpy2DAsync", "cudaGraphLaunch"};
+    int failed = 0;
+    for (const auto &entry : entries)
+        for (int replay = 0; replay < 2; replay++) {
+            for (int k = replay ? 3 : 1; k > 0; k--) EXPECT(entry() == CVM_OK);
+            for (int at = 0;; at++) {
+                int i = 0;
+                bool hit = false, reading = false;
+                st.on_call = [&](const std::string &name) {
+                    if (hit) return cudaSuccess;
+                    if (i++ == at) {
+                        hit = true;
+                        st.synced.clear();
+                        return cudaErrorUnknown;
+                    }
+                    reading = reading || reads.count(name);
+                    return cudaSuccess;
+                };
+                const int rc = entry();
+                st.on_call = nullptr;
+                if (!hit) {
+                    EXPECT(rc == CVM_OK);
+                    break;
+                }
+                if (rc != CVM_OK && reading) {
+                    failed++;
+                    EXPECT(st.synced.count(thread_stream()) && st.synced.count(side_stream().st2));
+                }
+            }
+        }
+    EXPECT(failed > 60);
+}
+
 }  // namespace
 
 namespace cvm {
@@ -57,6 +118,8 @@ int main(int argc, char **argv) {
         plan_changes_during_the_capture(true);
     else if (what == "plan_published")
         plan_changes_during_the_capture(false);
+    else if (what == "errors")
+        errors_wait();
     else
         return 2;
     return 0;

@@ -28,3 +28,8 @@ def replay(tmp_path_factory):
 def test_one_plan_for_the_size_and_the_launches(replay, event):
     r = subprocess.run([replay, event], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr
+
+
+def test_an_error_return_has_waited_for_what_reads_the_callers_memory(replay):
+    r = subprocess.run([replay, "errors"], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
