@@ -246,9 +246,16 @@ struct PoolBuf {
     }
 };
 
+bool give_back_idle();  // the memory of replayed calls' idle graphs (below), if any
+
 int pool_alloc(PoolBuf &b, size_t bytes, cudaStream_t st) {
     b.st = st;
-    CVM_CUDA(cudaMallocFromPoolAsync(&b.p, bytes ? bytes : 256, dev().pool, st));
+    cudaError_t e = cudaMallocFromPoolAsync(&b.p, bytes ? bytes : 256, dev().pool, st);
+    if (e == cudaErrorMemoryAllocation && give_back_idle()) {
+        cudaGetLastError();
+        e = cudaMallocFromPoolAsync(&b.p, bytes ? bytes : 256, dev().pool, st);
+    }
+    CVM_CUDA(e);
     return CVM_OK;
 }
 
@@ -970,18 +977,25 @@ int map_results(const float *dMap, int rw, int rh, float *map, const PeakReq *pk
 // A repeated one-shot call as a CUDA graph.  A small host-buffer call queued
 // launch by launch -- some thirty runtime calls over four streams -- is bound
 // by the host: 84 us for a 320x200 gray match, 104 for a 640x480 one from
-// RGBA; replayed 45 and 57 us (GB300, Grace host).  From the kGraphCalls-th call of a shape on, a thread
-// replays its launches as one graph: the inputs by one kernel that takes the
+// RGBA; replayed 45 and 57 us (GB300, Grace host).  From the kGraphCalls-th call of a shape on, by
+// whichever threads, its launches are replayed as one graph: the inputs by one kernel that takes the
 // caller's addresses from mapped page-locked memory (so the graph holds no
 // caller's pointer), then run_solo's launches on a workspace of the graph's
 // own.  Inputs of up to kGraphStage bytes are copied behind those addresses by
 // the host first: 64 KB in 3 us, where the device takes 15 us to translate and
-// read a few pageable pages.  A thread keeps the kGraphs shapes it used last, each of at most
-// kGraphBytes, until other shapes take their places or the thread ends.  Where
-// the device cannot read the caller's memory, under the profiler, or when the
-// capture fails, the call is queued launch by launch.
-constexpr int kGraphs = 4, kGraphCalls = 3;
-constexpr size_t kGraphBytes = size_t(256) << 20, kGraphStage = size_t(192) << 10;
+// read a few pageable pages.
+//
+// The process keeps up to kGraphs graphs and kGraphBytes of device memory for
+// them, each of at most kGraphBytesEach; a call has one to itself while it
+// runs, so threads that call one shape at once hold one each.  When a new graph
+// does not fit, those that none of the last kGraphStale calls used make room;
+// else the call is queued launch by launch, as it is where the device cannot
+// read the caller's memory, under the profiler, or when the capture fails.  (A
+// capture costs about 0.3 ms: shapes that only push each other out gain
+// nothing.)  A workspace allocation that fails gives all idle ones back.
+constexpr int kGraphs = 32, kGraphCalls = 3, kGraphShapes = 64;
+constexpr uint64_t kGraphStale = 256;
+constexpr size_t kGraphBytes = size_t(1) << 30, kGraphBytesEach = size_t(256) << 20, kGraphStage = size_t(192) << 10;
 
 struct SoloKey {
     int iw, ih, tw, th, mode, cn, step, gray, form, tune, map;
@@ -1001,97 +1015,161 @@ struct RelaxedCapture {
 
 struct SoloGraph {
     SoloKey key{};
-    int calls = 0;       // of the shape so far
-    bool failed = false;
     uint64_t used = 0;
-    void *mem = nullptr;  // frame, template, map, workspace
+    PoolBuf mem;          // frame, template, map, workspace
+    size_t bytes = 0;
     float *map = nullptr;
     SoloSource *src = nullptr;  // mapped page-locked, and the staged inputs behind it
     uint8_t *stage[2] = {nullptr, nullptr}, *stageDev[2] = {nullptr, nullptr};  // frame, template (nullptr: read in place)
     cvm_result *res = nullptr;  // likewise
     cudaGraphExec_t exec = nullptr;
     unsigned launches = 0;
-    void drop() {
+    ~SoloGraph() {
         RelaxedCapture relaxed;
         if (exec) cudaGraphExecDestroy(exec);
-        if (mem) cudaFree(mem);
         if (src) cudaFreeHost(src);
         if (res) cudaFreeHost(res);
-        *this = SoloGraph();
+        mem.release(thread_stream());  // (idle: its last call has waited for it)
+        cudaGetLastError();
     }
 };
 
-// The calling thread's entry for a shape (its least recently used one given
-// up for a new shape).
-SoloGraph *solo_graph(const SoloKey &key) {
-    struct Set {
-        SoloGraph g[kGraphs];
-        uint64_t tick = 0;
-        ~Set() {
-            for (SoloGraph &e : g) e.drop();
-        }
+struct SoloPool {
+    struct Shape {
+        SoloKey key{};
+        int calls = 0;
+        bool failed = false;
+        uint64_t used = 0;
     };
-    thread_local Set s;
-    SoloGraph *hit = nullptr;
-    for (SoloGraph &e : s.g)
-        if (e.calls > 0 && e.key == key) hit = &e;
-    if (!hit) {
-        hit = &s.g[0];
-        for (SoloGraph &e : s.g)
-            if (e.used < hit->used) hit = &e;
-        hit->drop();
-        hit->key = key;
+    std::mutex mu;
+    std::vector<std::unique_ptr<SoloGraph>> idle;
+    std::vector<Shape> shapes;  // the last kGraphShapes called
+    size_t bytes = 0;           // of all graphs, idle or not
+    int graphs = 0;
+    uint64_t tick = 0;
+
+    // The shape's record (mu held).
+    Shape &shape(const SoloKey &key) {
+        Shape *old = nullptr;
+        for (Shape &s : shapes) {
+            if (s.key == key) return s;
+            if (!old || s.used < old->used) old = &s;
+        }
+        if ((int)shapes.size() < kGraphShapes) {
+            shapes.emplace_back();
+            old = &shapes.back();
+        }
+        *old = Shape();
+        old->key = key;
+        return *old;
     }
-    hit->calls++;
-    hit->used = ++s.tick;
-    return hit;
+    // Room for one more graph of n bytes (mu held); the graphs that made room
+    // go to `out`, to be destroyed without the lock.
+    bool reserve(size_t n, std::vector<std::unique_ptr<SoloGraph>> &out) {
+        auto fits = [&]() { return graphs < kGraphs && bytes + n <= kGraphBytes; };
+        while (!fits()) {
+            size_t k = idle.size();
+            for (size_t i = 0; i < idle.size(); i++)
+                if (tick - idle[i]->used > kGraphStale && (k == idle.size() || idle[i]->used < idle[k]->used)) k = i;
+            if (k == idle.size()) return false;
+            take(k, out);
+        }
+        bytes += n;
+        graphs++;
+        return true;
+    }
+    void take(size_t k, std::vector<std::unique_ptr<SoloGraph>> &out) {
+        bytes -= idle[k]->bytes;
+        graphs--;
+        out.push_back(std::move(idle[k]));
+        idle.erase(idle.begin() + k);
+    }
+};
+
+// (never destroyed: calls may still end while the process does)
+SoloPool &solo_pool() {
+    static SoloPool *p = new SoloPool;
+    return *p;
+}
+
+bool give_back_idle() {
+    std::vector<std::unique_ptr<SoloGraph>> out;
+    SoloPool &p = solo_pool();
+    std::lock_guard<std::mutex> lk(p.mu);
+    while (!p.idle.empty()) p.take(p.idle.size() - 1, out);
+    return !out.empty();
+}
+
+// A call's hold on a graph: back to the idle ones at the call's end.
+struct SoloLease {
+    std::unique_ptr<SoloGraph> g;
+    SoloLease() = default;
+    SoloLease(SoloLease &&) = default;
+    ~SoloLease() {
+        if (!g) return;
+        SoloPool &p = solo_pool();
+        std::lock_guard<std::mutex> lk(p.mu);
+        g->used = p.tick;
+        p.idle.push_back(std::move(g));
+    }
+};
+
+// A graph's memory: the frame, the template, the map and the workspace.
+struct SoloLayout {
+    long long ip = 0, tp = 0;
+    size_t oTpl = 0, oMap = 0, oWork = 0, work = 0, total = 0;
+};
+
+bool solo_layout(const SoloKey &k, SoloJob J, const Plan &plan, cudaStream_t st, SoloLayout &l) {
+    const size_t mapBytes = k.map ? (size_t)(k.iw - k.tw + 1) * (k.ih - k.th + 1) * sizeof(float) : 0;
+    J.plan = &plan;
+    J.need = &l.work;
+    if (run_solo(J, st) != CVM_OK) return false;
+    l.ip = (long long)align_up((size_t)k.iw * k.step, 128);
+    l.tp = (long long)align_up((size_t)k.tw * k.step, 128);
+    l.oTpl = align_up((size_t)l.ip * k.ih, 256);
+    l.oMap = l.oTpl + align_up((size_t)l.tp * k.th, 256);
+    l.oWork = l.oMap + align_up(mapBytes, 256);
+    l.total = l.oWork + l.work;
+    return l.total <= kGraphBytesEach;
 }
 
 // Captures the shape's launches on the given plan; false when it cannot be
 // done.  (One plan for the workspace's size and for the launches in it: other
 // threads may switch the autotuner or tune the shape meanwhile.)
-bool solo_capture(SoloGraph &g, SoloJob J, const Plan &plan, cudaStream_t st) {
+bool solo_capture(SoloGraph &g, SoloJob J, const Plan &plan, const SoloLayout &l, cudaStream_t st) {
     const SoloKey &k = g.key;
     const int bpp = k.gray ? 4 : k.step;
-    const long long ip = (long long)align_up((size_t)k.iw * k.step, 128), tp = (long long)align_up((size_t)k.tw * k.step, 128);
-    const size_t mapBytes = k.map ? (size_t)(k.iw - k.tw + 1) * (k.ih - k.th + 1) * sizeof(float) : 0;
-    size_t work = 0;
-    J.plan = &plan;
-    J.need = &work;
-    if (run_solo(J, st) != CVM_OK) return false;
-    J.need = nullptr;
-    const size_t oTpl = align_up((size_t)ip * k.ih, 256), oMap = oTpl + align_up((size_t)tp * k.th, 256);
-    const size_t oWork = oMap + align_up(mapBytes, 256), total = oWork + work;
-    if (total > kGraphBytes) return false;
     const size_t bImg = align_up((size_t)k.iw * bpp, 16) * k.ih, bTpl = align_up((size_t)k.tw * bpp, 16) * k.th;
     const size_t sImg = bImg <= kGraphStage ? align_up(bImg, 256) : 0, sTpl = bTpl <= kGraphStage ? bTpl : 0;
     void *dSrc = nullptr, *dRes = nullptr;
-    if (cudaMalloc(&g.mem, total) != cudaSuccess ||
+    if (pool_alloc(g.mem, l.total, st) != CVM_OK ||
         cudaHostAlloc(reinterpret_cast<void **>(&g.src), 256 + sImg + sTpl, cudaHostAllocMapped) != cudaSuccess ||
         cudaHostAlloc(reinterpret_cast<void **>(&g.res), sizeof(cvm_result), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&dSrc, g.src, 0) != cudaSuccess ||
         cudaHostGetDevicePointer(&dRes, g.res, 0) != cudaSuccess)
         return false;
-    uint8_t *dImg = static_cast<uint8_t *>(g.mem), *dTpl = dImg + oTpl;
+    uint8_t *dImg = static_cast<uint8_t *>(g.mem.p), *dTpl = dImg + l.oTpl;
     for (int i = 0; i < 2; i++)
         if (i ? sTpl : sImg) {
             g.stage[i] = reinterpret_cast<uint8_t *>(g.src) + 256 + (i ? sImg : 0);
             g.stageDev[i] = static_cast<uint8_t *>(dSrc) + 256 + (i ? sImg : 0);
         }
-    g.map = k.map ? reinterpret_cast<float *>(dImg + oMap) : nullptr;
+    g.map = k.map ? reinterpret_cast<float *>(dImg + l.oMap) : nullptr;
     J.img = dImg;
-    J.istride = ip;
+    J.istride = l.ip;
     J.tpl = dTpl;
-    J.tstride = tp;
+    J.tstride = l.tp;
     J.map = g.map;
     J.out = static_cast<cvm_result *>(dRes);
-    J.work = dImg + oWork;
-    J.workBytes = work;
+    J.plan = &plan;
+    J.work = dImg + l.oWork;
+    J.workBytes = l.work;
     J.frameOnSide = 0;
     if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) != cudaSuccess) return false;
     const uint64_t l0 = g_launches.load();
-    bool ok = launch_ingest_solo(static_cast<const SoloSource *>(dSrc), dImg, ip, k.iw, k.ih, dTpl, tp, k.tw, k.th, bpp,
-                                 k.gray, static_cast<unsigned int *>(J.work), (int)(kSoloZero / 4), st) == cudaSuccess;
+    bool ok = launch_ingest_solo(static_cast<const SoloSource *>(dSrc), dImg, l.ip, k.iw, k.ih, dTpl, l.tp, k.tw, k.th,
+                                 bpp, k.gray, static_cast<unsigned int *>(J.work), (int)(kSoloZero / 4), st) == cudaSuccess;
     ok = ok && run_solo(J, st) == CVM_OK;
     g.launches = (unsigned)(g_launches.load() - l0);
     cudaGraph_t graph = nullptr;
@@ -1101,26 +1179,54 @@ bool solo_capture(SoloGraph &g, SoloJob J, const Plan &plan, cudaStream_t st) {
     return ok;
 }
 
-// The shape's graph when there is one by now (nullptr: queue the call).
-SoloGraph *replayable(const SoloKey &key, const SoloJob &J, cudaStream_t st) {
-    if (!dev().pageable || profile_on()) return nullptr;
-    SoloGraph *g = solo_graph(key);
-    if (g->exec) return g;
-    Plan plan;
-    if (g->failed || g->calls < kGraphCalls || !settled_plan(J, key.tune, &plan)) return nullptr;
+// A graph of the shape for this call (none: queue the call).
+SoloLease replayable(const SoloKey &key, const SoloJob &J, cudaStream_t st) {
+    SoloLease lease;
+    if (!dev().pageable || profile_on()) return lease;
+    SoloPool &p = solo_pool();
     {
-        RelaxedCapture relaxed;
-        if (solo_capture(*g, J, plan, st)) return g;
+        std::lock_guard<std::mutex> lk(p.mu);
+        SoloPool::Shape &s = p.shape(key);
+        s.used = ++p.tick;
+        s.calls = std::min(s.calls + 1, kGraphCalls);
+        size_t k = p.idle.size();
+        for (size_t i = 0; i < p.idle.size(); i++)
+            if (p.idle[i]->key == key && (k == p.idle.size() || p.idle[i]->used > p.idle[k]->used)) k = i;
+        if (k < p.idle.size()) {
+            lease.g = std::move(p.idle[k]);
+            p.idle.erase(p.idle.begin() + k);
+            return lease;
+        }
+        if (s.failed || s.calls < kGraphCalls) return lease;
     }
-    cudaGetLastError();
-    const int calls = g->calls;
-    const uint64_t used = g->used;
-    g->drop();
-    g->key = key;
-    g->calls = calls;
-    g->used = used;
-    g->failed = true;
-    return nullptr;
+    Plan plan;
+    if (!settled_plan(J, key.tune, &plan)) return lease;
+    RelaxedCapture relaxed;
+    SoloLayout l;
+    bool ok = solo_layout(key, J, plan, st, l), reserved = false;
+    if (ok) {
+        std::vector<std::unique_ptr<SoloGraph>> out;  // (destroyed before the new one allocates)
+        std::lock_guard<std::mutex> lk(p.mu);
+        reserved = p.reserve(l.total, out);
+        if (!reserved) return lease;
+    }
+    if (ok) {
+        auto g = std::make_unique<SoloGraph>();
+        g->key = key;
+        g->bytes = l.total;
+        ok = solo_capture(*g, J, plan, l, st);
+        if (ok) lease.g = std::move(g);
+    }
+    if (!ok) {
+        cudaGetLastError();
+        std::lock_guard<std::mutex> lk(p.mu);
+        p.shape(key).failed = true;
+        if (reserved) {
+            p.bytes -= l.total;
+            p.graphs--;
+        }
+    }
+    return lease;
 }
 
 int host_solo(const uint8_t *img, long long istride, int iw, int ih, const uint8_t *tpl, long long tstride,
@@ -1141,7 +1247,8 @@ int host_solo(const uint8_t *img, long long istride, int iw, int ih, const uint8
     J.tw = tw;
     J.th = th;
     const SoloKey key{iw, ih, tw, th, mode, cnFixed, step, grayFromRgba, J.form, g_autotune.load(), map || pk ? 1 : 0};
-    if (SoloGraph *g = replayable(key, J, st)) {
+    if (SoloLease lease = replayable(key, J, st); lease.g) {
+        SoloGraph *g = lease.g.get();
         const int bpp = grayFromRgba ? 4 : step;
         SoloSource in[2] = {{img, istride}, {tpl, tstride}};
         for (int i = 0; i < 2; i++)

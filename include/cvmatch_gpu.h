@@ -27,6 +27,13 @@
  *     call made with a different device current returns
  *     CVM_ERR_UNSUPPORTED before queueing anything.  (The fixed-scratch
  *     entry point keeps its own per-device set-up.)
+ *   - From its third call on, a host-buffer match of one shape (sizes,
+ *     channels, form) is replayed as a CUDA graph, by whichever threads make
+ *     the calls.  The process keeps up to 32 such graphs, with at most 1 GB of
+ *     device memory and 13 MB of page-locked memory in all; shapes that have
+ *     not been called lately make room for others, and a device allocation
+ *     that fails inside the library gives the idle ones' memory back.  No
+ *     caller's pointer is kept.
  *   - The computation is the reference's op sequence: scores are
  *     bit-identical to cvmatch's Go path on the same inputs.
  */

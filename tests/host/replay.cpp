@@ -1,4 +1,6 @@
 // Replayed one-shot host calls, on the stand-ins of fake_cuda.h.
+#include <thread>
+
 #include "fake_cuda.h"
 
 #include "../../cvmatch_gb300/csrc/cvm_api.cpp"
@@ -106,6 +108,72 @@ void errors_wait() {
     EXPECT(failed > 60);
 }
 
+long graph_launches() { return fake::state().calls["cudaGraphLaunch"]; }
+
+// Calls of one shape from ever new threads, one at a time: they share what is
+// kept, and from the fourth on a thread's first call replays.
+void threads_share() {
+    cvm_set_form(CVM_FORM_EXACT);
+    size_t after = 0;
+    for (int i = 0; i < 24; i++) {
+        std::thread([&] { EXPECT(call(700, 300, 40, 30) == CVM_OK); }).join();
+        if (i >= 3) EXPECT(graph_launches() == i - 1);
+        if (i == 3) after = fake::state().deviceBytes;
+    }
+    EXPECT(fake::state().calls["cudaGraphInstantiate"] == 1);
+    EXPECT(fake::state().deviceBytes == after);
+}
+
+// Threads inside calls of one shape at the same time, a graph each: bounded.
+void threads_bounded() {
+    cvm_set_form(CVM_FORM_EXACT);
+    for (int i = 0; i < 3; i++) EXPECT(call(1500, 700, 40, 30) == CVM_OK);
+    const size_t one = fake::state().deviceBytes;
+    std::vector<std::thread> t;
+    std::atomic<int> left{64};
+    for (int i = 0; i < 64; i++)
+        t.emplace_back([&] {
+            for (int k = 0; k < 4; k++) EXPECT(call(1500, 700, 40, 30) == CVM_OK);
+            left--;
+            while (left > 0) std::this_thread::yield();  // (a thread's end gives nothing back)
+        });
+    while (left > 0) std::this_thread::yield();
+    EXPECT(fake::state().deviceBytes <= (size_t(1) << 30) + (64 << 20));
+    for (auto &x : t) x.join();
+    EXPECT(one > (16 << 20));
+    EXPECT(fake::state().deviceBytes <= (size_t(1) << 30) + (64 << 20));
+}
+
+// More shapes than are kept, in turn: no capture pushes another out in vain;
+// shapes no longer called make room.
+void shapes_in_turn() {
+    cvm_set_form(CVM_FORM_EXACT);
+    for (int round = 0; round < 12; round++)
+        for (int k = 0; k < 40; k++) EXPECT(call(300 + 8 * k, 200, 20, 20) == CVM_OK);
+    EXPECT(fake::state().calls["cudaGraphInstantiate"] <= 40);
+    EXPECT(graph_launches() > 200);
+    for (int k = 0; k < 400; k++) EXPECT(call(300, 200, 20, 20) == CVM_OK);
+    const long n = fake::state().calls["cudaGraphInstantiate"];
+    for (int k = 0; k < 3; k++) EXPECT(call(1000, 200, 20, 20) == CVM_OK);
+    EXPECT(fake::state().calls["cudaGraphInstantiate"] == n + 1);
+    for (int k = 0; k < 200; k++)
+        for (int i = 0; i < 3; i++) EXPECT(call(640, 220 + k, 20, 20) == CVM_OK);
+    EXPECT(fake::state().deviceBytes <= (size_t(1) << 30) + (64 << 20));
+}
+
+// Device memory runs out: the idle graphs' goes to the call that needs it.
+void memory_given_back() {
+    cvm_set_form(CVM_FORM_EXACT);
+    for (int i = 0; i < 4; i++) EXPECT(call(700, 300, 40, 30) == CVM_OK);
+    EXPECT(graph_launches() == 2);
+    const size_t held = fake::state().deviceBytes;
+    fake::state().on_call = [&](const std::string &f) {
+        return f == "cudaMallocFromPoolAsync" && fake::state().deviceBytes >= held ? cudaErrorMemoryAllocation : cudaSuccess;
+    };
+    EXPECT(call(500, 300, 40, 30) == CVM_OK);
+    EXPECT(fake::state().deviceBytes < held);
+}
+
 }  // namespace
 
 namespace cvm {
@@ -120,6 +188,14 @@ int main(int argc, char **argv) {
         plan_changes_during_the_capture(false);
     else if (what == "errors")
         errors_wait();
+    else if (what == "threads_share")
+        threads_share();
+    else if (what == "threads_bounded")
+        threads_bounded();
+    else if (what == "shapes_in_turn")
+        shapes_in_turn();
+    else if (what == "memory_given_back")
+        memory_given_back();
     else
         return 2;
     return 0;

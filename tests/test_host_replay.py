@@ -33,3 +33,9 @@ def test_one_plan_for_the_size_and_the_launches(replay, event):
 def test_an_error_return_has_waited_for_what_reads_the_callers_memory(replay):
     r = subprocess.run([replay, "errors"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("event", ["threads_share", "threads_bounded", "shapes_in_turn", "memory_given_back"])
+def test_what_the_process_keeps_is_bounded_and_shared(replay, event):
+    r = subprocess.run([replay, event], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
