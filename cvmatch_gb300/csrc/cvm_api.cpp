@@ -1563,11 +1563,12 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
 // rest the frame's shared cost, and the bucket's cost is shared + n x
 // per-member.  newGoPlan's plan (fleet.go:356-365) is kept unless another
 // candidate beats it by more than 3 %.  Cached per (frame size, bucket
-// maxima, members, step, form) for the process.
+// maxima, members, step, form, den's source) for the process.
 struct FleetTuneKey {
-    int pw, ph, tw, th, step, form, n;
+    int pw, ph, tw, th, step, form, n, stats;  // stats: den's source in the trials (their cost differs)
     bool operator<(const FleetTuneKey &o) const {
-        return std::tie(pw, ph, tw, th, step, form, n) < std::tie(o.pw, o.ph, o.tw, o.th, o.step, o.form, o.n);
+        return std::tie(pw, ph, tw, th, step, form, n, stats) <
+               std::tie(o.pw, o.ph, o.tw, o.th, o.step, o.form, o.n, o.stats);
     }
 };
 struct FleetTuneEntry {
@@ -1585,7 +1586,7 @@ int tune_bucket_plan(cvm_fleet *f, const Bucket &b, const uint8_t *dParent, long
     *out = make_plan(b.tw, b.th, rwF, rhF);
     const int nm = (int)b.members.size();
     if (f->form == CVM_FORM_EXACT || !g_autotune.load() || nm < 4 || !dParent) return CVM_OK;
-    const FleetTuneKey key{pw, ph, b.tw, b.th, f->step, f->form, nm};
+    const FleetTuneKey key{pw, ph, b.tw, b.th, f->step, f->form, nm, stats};
     {
         std::lock_guard<std::mutex> lk(g_tuneMu);
         auto it = g_fleetTune.find(key);

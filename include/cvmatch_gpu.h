@@ -370,7 +370,10 @@ int cvm_fleet_set_overlap(cvm_fleet *f, int on);
  * may hold an extremum (a lower bound of den over blocks of results rules
  * out the rest), with no statistics launch and no den written or read; other
  * buckets, and every exact- or mixed-form bucket, still run the statistics
- * kernel.  Results are the same bits either way.  A fleet on which this was
+ * kernel.  On one tile plan the results are the same bits either way; the
+ * autotuner times a bucket's plans for the source the fleet had when it first
+ * met the frame size, and plans differ within the fast form's rounding.  A
+ * fleet on which this was
  * never called chooses by itself on its first frame of a size (256 RGBA
  * templates on a 2560x1440 frame: 5.6 ms per FindAll with the epilogue, 7.8
  * with the kernel; small templates on flat panels with thin strokes are

@@ -1,0 +1,21 @@
+"""Fleets' host logic on stand-ins for the CUDA runtime and the kernels'
+launchers (tests/host)."""
+import subprocess
+
+import pytest
+
+from test_host_replay import compile_host
+
+
+@pytest.fixture(scope="module")
+def fleet(tmp_path_factory):
+    return compile_host("fleet", tmp_path_factory.mktemp("host"))
+
+
+def _run(exe, what):
+    r = subprocess.run([exe, what], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr
+
+
+def test_plans_are_tuned_per_source_of_den(fleet):
+    _run(fleet, "tuned_per_source")
