@@ -1473,10 +1473,90 @@ struct FleetBucketGeom {
     }
 };
 
+// A fast-form fleet's own choice of den's source on frames of one size, unless
+// cvm_fleet_set_stats said: on demand (CVM_STATS_EPILOGUE) or the statistics
+// kernel.  On demand costs what the results that form their den one by one
+// cost: few, where blocks of results bound den well; many on flat panels beside
+// thin strokes under small templates, whose blocks have no bound, on frames
+// where everything scores like an extremum (a linear gradient), and in fleets so
+// small that all their rows start at once.  The first
+// frame chooses by a sample of its blocks (choose_stats).  Later calls look
+// again now and then, without waiting for the device: on demand, how many warp
+// steps of the rows went for a den; with the kernel, the blocks once more.  The
+// device leaves the tallies in page-locked memory, and the next call that finds
+// them there acts on them.  Results do not depend on it.
+struct DenWatch {
+    DevMember *table = nullptr;  // the members that the summed-area table serves
+    int n = 0;
+    long long steps = 0;         // a frame's warp steps over their results
+    DenTally *tally = nullptr, *dTally = nullptr;  // mapped page-locked
+    std::mutex mu;
+    int source = CVM_STATS_EPILOGUE;
+    uint64_t calls = 0, asked = 0, next = 1;  // asked: the call being tallied (0: none)
+    uint64_t gap = 1, calm = 32;              // calls until the look after the next; its largest value
+
+    // More than kPoorShare of the blocks without a bound, or kFormShare of the
+    // rows' steps forming den, choose the kernel; half of kPoorShare chooses on
+    // demand.  On 1920x1080, on demand / with the kernel in ms: 64 icons of 12..32
+    // px on a user interface (17 % of the blocks) 1.35 / 0.88, 16..64 px (7 %)
+    // 1.48 / 1.10, 24..96 px (none; 11 % of the steps) 1.04 / 1.11; 8 templates of
+    // 24..64 px on a camera's frame (14 % of the steps) 0.28 / 0.30; 32 on a
+    // checkerboard (19 %) 0.62 / 0.64; 32 on half a gradient (47 %) 0.81 / 0.75, on
+    // a whole one (all) 1.10 / 0.78.  Fleets with too few CTAs for any to start
+    // from others' extrema: 2 templates (59 %) 0.167 / 0.148, 12 on 960x540 (26..33
+    // %) 0.134 / 0.137, 24 on 640x480 (28 %) 0.152 / 0.153, 2 there (all) 0.089 /
+    // 0.073.
+    static constexpr double kPoorShare = 1.0 / 32, kFormShare = 1.0 / 4;
+
+    int now() {
+        std::lock_guard<std::mutex> lk(mu);
+        return source;
+    }
+    // Counts a call; true when it should be tallied, as number *seq.
+    bool look(int *src, unsigned *seq) {
+        std::lock_guard<std::mutex> lk(mu);
+        calls++;
+        if (asked && static_cast<volatile DenTally *>(tally)->seq == (unsigned)asked) {
+            std::atomic_thread_fence(std::memory_order_acquire);
+            judge(*tally);
+            asked = 0;
+        }
+        *src = source;
+        if (asked && calls - asked > 4096) asked = 0;  // (its call failed)
+        if (!tally || asked || calls < next) return false;
+        asked = calls;
+        next = calls + gap;
+        gap = std::min(2 * gap, calm);
+        *seq = (unsigned)asked;
+        return true;
+    }
+    void judge(const DenTally &t) {
+        const int was = source;
+        if (t.source == CVM_STATS_EPILOGUE && t.formed > kFormShare * steps) source = CVM_STATS_KERNEL;
+        if (t.source == CVM_STATS_KERNEL && t.poor < 0.5 * kPoorShare * 256 * n) source = CVM_STATS_EPILOGUE;
+        if (source == was) {
+            calm = std::max<uint64_t>(calm / 2, 32);
+        } else if (source == CVM_STATS_EPILOGUE) {
+            gap = 1;  // soon, by the steps
+            next = calls + 1;
+        } else {
+            // (content with bounds whose scores are all extrema comes back
+            // here: it is tried on demand for two calls in ever more)
+            calm = std::min<uint64_t>(4 * calm, 4096);
+            gap = calm;
+            next = calls + gap;
+        }
+    }
+    ~DenWatch() {
+        if (table) cudaFree(table);
+        if (tally) cudaFreeHost(tally);
+    }
+};
+
 struct FleetGeom {
     int pw = 0, ph = 0;
-    int stats = CVM_STATS_KERNEL;  // the library's choice of den's source (choose_stats)
     int form = CVM_FORM_EXACT;  // the form the spectra were built for
+    std::unique_ptr<DenWatch> watch;  // (destroyed after the buckets, whose frees wait for the device)
     std::vector<std::unique_ptr<FleetBucketGeom>> bg;
 };
 
@@ -1763,23 +1843,14 @@ std::vector<Bucket> fast_buckets(const cvm_fleet *f, int pw, int ph) {
     return out;
 }
 
-// Where a fast-form fleet's den comes from on frames like this one, unless
-// cvm_fleet_set_stats said: on demand (CVM_STATS_EPILOGUE) when blocks of its
-// members' results bound den well, else the statistics kernel.  Blocks without
-// a bound -- flat panels beside thin strokes, under small templates -- make
-// their results form den one by one: 64 icons of 12..32 px on a 1920x1080 user
-// interface (13 % of blocks unbounded) 1.44 ms against 1.08 with the kernel,
-// 64 templates of 16..192 x 16..128 there (2 %) 1.05 against 1.25; more than 3
-// % choose the kernel.  Measured on the first frame of a size, outside stream
-// capture (in one: on demand); results do not depend on it.
-constexpr int kPoorShare = 32;
-
-int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, int ph, cudaStream_t cst, int *out) {
-    *out = CVM_STATS_KERNEL;
-    if (f->form != CVM_FORM_FAST || !dParent) return CVM_OK;
-    *out = f->statsMode >= 0 ? f->statsMode : CVM_STATS_EPILOGUE;
-    if (f->statsMode >= 0) return CVM_OK;
+// The first frame's choice of den's source (DenWatch), for a fast-form fleet
+// that cvm_fleet_set_stats left to itself: a sample of its members' blocks.
+// Inside a capture nothing is sampled: on demand, until a later call looks.
+int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, int ph, cudaStream_t cst,
+                 std::unique_ptr<DenWatch> &out) {
+    if (f->form != CVM_FORM_FAST || f->forcedPlan.dftW > 0) return CVM_OK;
     const int np = f->step == 4 ? 4 : 2, hp = (int)align_up((size_t)pw + 1, 32);
+    auto w = std::make_unique<DenWatch>();
     std::vector<DevMember> tab;
     for (const Bucket &b : f->buckets)
         for (int i : b.members) {
@@ -1791,11 +1862,30 @@ int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw
             d.th = m->h;
             d.rw = pw - m->w + 1;
             d.rh = ph - m->h + 1;
-            if (den_table_area(m->w, m->h, f->step)) tab.push_back(d);
+            if (!den_table_area(m->w, m->h, f->step)) continue;
+            tab.push_back(d);
+            w->steps += ((long long)d.rw * d.rh + 31) / 32;
         }
+    if (tab.empty()) return CVM_OK;
+    w->n = (int)tab.size();
+    CVM_CUDA(cudaMalloc(&w->table, tab.size() * sizeof(DevMember)));
+    CVM_CUDA(cudaMemcpy(w->table, tab.data(), tab.size() * sizeof(DevMember), cudaMemcpyHostToDevice));
+    // (without the tallies the first choice stays)
+    if (cudaHostAlloc(reinterpret_cast<void **>(&w->tally), sizeof(DenTally), cudaHostAllocMapped) == cudaSuccess) {
+        memset(w->tally, 0, sizeof(DenTally));
+        if (cudaHostGetDevicePointer(reinterpret_cast<void **>(&w->dTally), w->tally, 0) != cudaSuccess) {
+            cudaFreeHost(w->tally);
+            w->tally = nullptr;
+        }
+    } else {
+        w->tally = nullptr;
+    }
+    cudaGetLastError();
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (tab.empty() || cudaStreamIsCapturing(cst, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    if (f->statsMode >= 0 || !dParent || cudaStreamIsCapturing(cst, &cs) != cudaSuccess ||
+        cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
+        out = std::move(w);
         return CVM_OK;
     }
     CVM_CUDA(cudaStreamSynchronize(cst));  // the frame, written on the caller's stream
@@ -1805,34 +1895,33 @@ int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw
     PoolBuf buf;
     CVM_TRY(pool_alloc(buf,
                        Arena::bytes(n, sizeof(DevParams)) + Arena::bytes(1, sizeof(DevFrame)) +
-                           Arena::bytes(tab.size(), sizeof(DevMember)) + Arena::bytes(1, sizeof(int)) +
-                           Arena::bytes(lanes, 4) + Arena::bytes(sat_scratch_elems(ph, hp, np), 4),
+                           Arena::bytes(1, sizeof(int)) + Arena::bytes(lanes, 4) +
+                           Arena::bytes(sat_scratch_elems(ph, hp, np), 4),
                        ts));
     Arena A;
     A.base = static_cast<char *>(buf.p);
     DevParams *P = A.take<DevParams>(n);
     DevFrame *F = A.take<DevFrame>(1);
-    DevMember *T = A.take<DevMember>(tab.size());
     int *dPoor = A.take<int>(1), poor = 0;
     unsigned int *sat = A.take<unsigned int>(lanes), *blk = A.take<unsigned int>(sat_scratch_elems(ph, hp, np));
     CVM_CUDA(cudaMemsetAsync(F, 0, sizeof(DevFrame), ts));
     CVM_CUDA(cudaMemsetAsync(dPoor, 0, sizeof(int), ts));
-    CVM_CUDA(cudaMemcpyAsync(T, tab.data(), tab.size() * sizeof(DevMember), cudaMemcpyHostToDevice, ts));
     CVM_CUDA(launch_prep(nullptr, 0, 0, 0, f->step, 0, f->step == 4 ? dParent : nullptr, pstride, pw, ph, P, n, 0, 0, 0,
                          F, ts, f->dP));
     CVM_CUDA(launch_sat(dParent, pstride, pw, ph, hp, np, &F->cnMax, blk, sat, ts));
     MemberSet ms;
     memset(&ms, 0, sizeof ms);
-    ms.table = T;
+    ms.table = w->table;
     ms.params = P;
     ms.sat = sat;
     ms.satRow = (size_t)np * hp;
     ms.satAlpha = np == 4 ? (size_t)(ph + 1) * 4 * hp : 0;
     ms.satNp = np;
-    CVM_CUDA(launch_den_poor(ms, (int)tab.size(), dPoor, ts));
+    CVM_CUDA(launch_den_poor(ms, w->n, dPoor, ts));
     CVM_CUDA(cudaMemcpyAsync(&poor, dPoor, sizeof(int), cudaMemcpyDeviceToHost, ts));
     CVM_CUDA(cudaStreamSynchronize(ts));
-    if ((long long)poor * kPoorShare > 256LL * (long long)tab.size()) *out = CVM_STATS_KERNEL;
+    if (poor > DenWatch::kPoorShare * 256 * w->n) w->source = CVM_STATS_KERNEL;
+    out = std::move(w);
     return CVM_OK;
 }
 
@@ -1847,7 +1936,8 @@ int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, 
     fg->pw = pw;
     fg->ph = ph;
     fg->form = f->form;
-    CVM_TRY(choose_stats(f, dParent, pstride, pw, ph, cst, &fg->stats));
+    CVM_TRY(choose_stats(f, dParent, pstride, pw, ph, cst, fg->watch));
+    const int stats = f->statsMode >= 0 ? f->statsMode : (fg->watch ? fg->watch->source : CVM_STATS_KERNEL);
     cudaStream_t st = thread_stream();
     const std::vector<Bucket> buckets =
         f->form != CVM_FORM_EXACT && f->forcedPlan.dftW == 0 ? fast_buckets(f, pw, ph) : f->buckets;
@@ -1858,7 +1948,7 @@ int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, 
         if (f->forcedPlan.dftW > 0)
             plan = f->forcedPlan;
         else
-            CVM_TRY(tune_bucket_plan(f, b, dParent, pstride, pw, ph, cst, fg->stats, &plan));
+            CVM_TRY(tune_bucket_plan(f, b, dParent, pstride, pw, ph, cst, stats, &plan));
         CVM_TRY(make_geom(b.tw, b.th, rwF, rhF, b.th, bg->G, &plan));
         bg->form = effective_form(f->form, bg->G);
         const bool bfast = bg->form != CVM_FORM_EXACT;
@@ -1967,7 +2057,16 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     // area the table serves.  (256 templates on 2560x1440, launches in
     // sequence: statistics 2.72 ms and rows 1.86 ms with the lanes, rows 2.31
     // ms on demand.)
-    const int stats = f->statsMode >= 0 ? f->statsMode : fg->stats;
+    int stats = f->statsMode >= 0 ? f->statsMode : CVM_STATS_KERNEL;
+    bool look = false;  // this call is tallied for the fleet's own choice
+    unsigned lookSeq = 0;
+    if (f->statsMode < 0 && fg->watch) {
+        stats = fg->watch->now();
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (f->roi.empty() && cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone)
+            look = fg->watch->look(&stats, &lookSeq);
+        cudaGetLastError();
+    }
     std::vector<char> satUse(fg->bg.size(), 0);
     bool anySat = false, anyStatsKernel = false;  // anyStatsKernel: a bucket's every member
     for (size_t b = 0; b < fg->bg.size(); b++) {
@@ -2020,8 +2119,10 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     for (const Bucket &b : f->buckets) twMax = std::max(twMax, b.tw);
     const size_t prefixRow = (size_t)(cnP == 4 ? 4 : stat_pitch(cnP)) * hpP;
     const size_t alphaRow = cnP == 4 ? (size_t)2 * hpP : 0;
-    const size_t satElems = anySat ? (size_t)(ph + 1) * (prefixRow + alphaRow) : 0;
-    const size_t satBlkElems = anySat ? sat_scratch_elems(ph, hpP, cnP == 4 ? 4 : 2) : 0;
+    const bool needSat = anySat || look;
+    const size_t satElems = needSat ? (size_t)(ph + 1) * (prefixRow + alphaRow) : 0;
+    const size_t satBlkElems = needSat ? sat_scratch_elems(ph, hpP, cnP == 4 ? 4 : 2) : 0;
+    const size_t tallyElems = look ? kTallyWords : 0;
     const bool blkOk = anyStatsKernel && 16ull * (unsigned)twMax * (cnP == 4 ? 3u : 1u) * 65025ull < (1ull << 32);
     const size_t blkElems = blkOk ? prefixRow * (size_t)(ph / 16) : 0;
     const size_t bytes = Arena::bytes(n, sizeof(DevParams)) + Arena::bytes(1, sizeof(DevFrame)) +
@@ -2030,7 +2131,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
                          (satElems ? Arena::bytes(satElems, sizeof(unsigned int)) +
                                          Arena::bytes(satBlkElems, sizeof(unsigned int))
                                    : 0) +
-                         frameBytes + partBytes + waveBytes;
+                         Arena::bytes(tallyElems, sizeof(unsigned int)) + frameBytes + partBytes + waveBytes;
     // Overlapped waves (fast-form buckets, more than one wave in all): the
     // inverse rows of wave k run on the side stream beside the statistics
     // and columns of wave k + 1, so the waves alternate between two sets of
@@ -2059,6 +2160,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     unsigned int *prefixBlk = blkElems ? A.take<unsigned int>(blkElems) : nullptr;
     unsigned int *sat = satElems ? A.take<unsigned int>(satElems) : nullptr;
     unsigned int *satBlk = satElems ? A.take<unsigned int>(satBlkElems) : nullptr;
+    unsigned int *tally = A.take<unsigned int>(tallyElems);
     char *frameBase = A.base + A.used;
     A.used += frameBytes;
     Partial *parts = reinterpret_cast<Partial *>(A.base + A.used);
@@ -2084,6 +2186,20 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     CVM_CUDA(launch_prep(nullptr, 0, 0, 0, f->step, 0, f->step == 4 ? dParent : nullptr, pstride, pw, ph, P, n, 0, 0,
                          0, F, st, f->dP));
     if (sat) CVM_CUDA(launch_sat(dParent, pstride, pw, ph, hpP, cnP == 4 ? 4 : 2, &F->cnMax, satBlk, sat, st));
+    if (look) {
+        CVM_CUDA(cudaMemsetAsync(tally, 0, kTallyWords * sizeof(unsigned int), st));
+        if (stats == CVM_STATS_KERNEL) {
+            MemberSet ms;
+            memset(&ms, 0, sizeof ms);
+            ms.table = fg->watch->table;
+            ms.params = P;
+            ms.sat = sat;
+            ms.satRow = prefixRow;
+            ms.satAlpha = alphaRow ? (size_t)(ph + 1) * prefixRow : 0;
+            ms.satNp = cnP == 4 ? 4 : 2;
+            CVM_CUDA(launch_den_poor(ms, fg->watch->n, reinterpret_cast<int *>(tally), st));
+        }
+    }
     if (anyStatsKernel) CVM_CUDA(launch_row_prefix(dParent, pstride, f->step, pw, ph, cnP, prefix, hpP, st));
     if (prefixBlk) CVM_CUDA(launch_vblock(prefix, prefixBlk, ph / 16, prefixRow, st));
     for (size_t b = 0; b < fg->bg.size(); b++) {
@@ -2130,6 +2246,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
             ms.satRow = prefixRow;
             ms.satAlpha = alphaRow ? (size_t)(ph + 1) * prefixRow : 0;
             ms.satNp = cnP == 4 ? 4 : 2;
+            ms.formed = look ? tally : nullptr;
         }
         for (int c = 0; c < G.nclass; c++) {
             ms.scratch[c] = scratch[0][c];
@@ -2163,6 +2280,13 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
                                          bg.nparts, parts, counters, dOut, rst, fast, bounds, nm));
             if (overlap) CVM_CUDA(cudaEventRecord(ss->rowsDone[set], rst));
         }
+    }
+    if (look) {
+        if (overlap) {
+            CVM_CUDA(cudaEventRecord(ss->colsDone, ss->waveRows));
+            CVM_CUDA(cudaStreamWaitEvent(st, ss->colsDone, 0));
+        }
+        CVM_CUDA(launch_tally(tally, fg->watch->dTally, lookSeq, stats, st));
     }
     return CVM_OK;
 }

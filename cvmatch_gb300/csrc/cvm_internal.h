@@ -125,6 +125,18 @@ struct MemberSet {
     size_t satRow;     // u32 per row of the main block (satNp * hp)
     size_t satAlpha;   // u32 offset of the (s3, alpha squares) block; 0: none
     int satNp;         // u32 per x in the main block: 4 (RGBA frame), 2 (gray)
+    unsigned int *formed;  // a tallied call: the words of launch_tally (nullptr: no tally)
+};
+
+// What a fleet call tallies for its fleet's choice of den's source: blocks of
+// results without a bound (launch_den_poor), or warp steps of the inverse rows
+// that formed den, spread over words 16 apart from kTallyFormed on.
+constexpr int kTallyFormed = 16, kTallySpread = 64, kTallyWords = kTallyFormed + 16 * kTallySpread;
+struct DenTally {
+    unsigned int seq;           // the tallied call, written last
+    int source;                 // its source of den
+    unsigned int poor;
+    unsigned long long formed;
 };
 
 struct Partial {
@@ -260,6 +272,9 @@ cudaError_t launch_sat(const uint8_t *img, long long istride, int iw, int ih, in
 // table's first nmembers) have no lower bound of den from the summed-area
 // table ms.sat.
 cudaError_t launch_den_poor(const MemberSet &ms, int nmembers, int *poor, cudaStream_t st);
+// Sums a tallied call's words (the first: blocks without a bound) into *out,
+// mapped page-locked memory.
+cudaError_t launch_tally(const unsigned int *words, DenTally *out, unsigned int seq, int source, cudaStream_t st);
 
 // Stores small host values into device memory through kernel arguments
 // (stream ordered, no host buffer lifetime to manage).

@@ -1872,6 +1872,23 @@ __global__ void __launch_bounds__(256) k_den_poor(const __grid_constant__ Member
     if (threadIdx.x == 0) atomicAdd(poor, n);
 }
 
+__global__ void __launch_bounds__(kTallySpread) k_tally(const unsigned int *words, DenTally *out, unsigned int seq, int source) {
+    __shared__ unsigned long long sum[kTallySpread / 32];
+    unsigned long long v = words[kTallyFormed + 16 * threadIdx.x];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sum[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x) return;
+    v = 0;
+    for (int i = 0; i < kTallySpread / 32; i++) v += sum[i];
+    out->source = source;
+    out->poor = words[0];
+    out->formed = v;
+    __threadfence_system();
+    *reinterpret_cast<volatile unsigned int *>(&out->seq) = seq;
+}
+
 // PRE: H is the shared row prefix built for PCN channels (window sum =
 // P[x+tw] - P[x]); its squares are plane PCN (PCN < 4) or planes 4 (RGB)
 // and 5 (alpha) when PCN == 4 (a cn = 3 member leaves alpha out).
@@ -2779,6 +2796,12 @@ cudaError_t launch_sat(const uint8_t *img, long long istride, int iw, int ih, in
 
 cudaError_t launch_den_poor(const MemberSet &ms, int nmembers, int *poor, cudaStream_t st) {
     k_den_poor<<<nmembers, 256, 0, st>>>(ms, poor);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tally(const unsigned int *words, DenTally *out, unsigned int seq, int source, cudaStream_t st) {
+    k_tally<<<1, kTallySpread, 0, st>>>(words, out, seq, source);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -121,8 +121,15 @@ constexpr int kBlocksMax = 1024;  // of a CTA: 8192 results over two rows a pair
 
 // A result above its block's bound: its den, and the ladder unless that
 // already rules it out.
+template <bool COUNT>
 __device__ __noinline__ Track score_table(Track t, float num, const MemberSet &ms, const DevMember &m,
                                           const DevParams &Pm, int y, int x, float denFlat, int l) {
+    if constexpr (COUNT) {
+        // (the warp's lanes that are here, once)
+        const unsigned int here = __activemask();
+        if ((threadIdx.x & 31) == __ffs(here) - 1)
+            atomicAdd(ms.formed + kTallyFormed + 16 * ((blockIdx.x + blockIdx.y) & (kTallySpread - 1)), 1u);
+    }
     const float d = sat_den(ms, m, Pm, y, x);
     if (d > 0.f && num < t.hi * d && num > t.lo * d) return t;
     const float sc = score_fast(num, d, denFlat);
@@ -144,7 +151,7 @@ __device__ __noinline__ Track score_table(Track t, float num, const MemberSet &m
 // with 32x32, RGB: three 27.6 us, six 22.7, seven 24.8; 128 points: three
 // 32.9, six 35.0).
 __host__ __device__ constexpr int lines_ctas(int L, bool fast, int mode) {
-    return mode == 2                   ? (L == 11 ? 4 : (L <= 8 ? 8 : 9))
+    return mode == 2 || mode == 4      ? (L == 11 ? 4 : (L <= 8 ? 8 : 9))
            : mode == 0 && L == 8 && !fast ? 6
                                        : (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 5) : (fast ? 10 : 8))) *
                                              (mode || (L == 11 && fast) ? 4 : 3) / 4;
@@ -155,13 +162,16 @@ __host__ __device__ constexpr int lines_ctas(int L, bool fast, int mode) {
 // from the statistics kernel's lanes.  TABLE: a fast-form fleet's extrema,
 // den on demand.  SOLO: LANES for a single match, whose CTAs all start at once
 // with no extrema of earlier ones to cut by (fleets keep their registers).
-enum Keep { ALL, LANES, TABLE, SOLO };
+// TALLY: TABLE in a tallied call (MemberSet::formed; the test for it alone, in
+// TABLE's registers, cost the rows 4 %).
+enum Keep { ALL, LANES, TABLE, SOLO, TALLY };
 
 // The extrema (and scores) of the CTA's row pairs.
-template <int L, bool FAST, Keep MODE>
+template <int L, bool FAST, Keep KEEP>
 __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const DevMember &m, const DevParams &Pm,
                                           const TileBox &tb, int bw, int bh, int pair0, int P, unsigned int *bnd) {
     using S = Lines<L>;
+    constexpr Keep MODE = KEEP == TALLY ? TABLE : KEEP;
     constexpr bool LEAN = MODE != ALL;
     constexpr int N = S::N, R1 = S::R1, K1 = S::K1, NB = S::NB, G = S::G, NL = S::NL, PITCH = S::PITCH;
     constexpr int NU = NB == 1 ? 1 : 16 / NB;             // last-pass units of a thread
@@ -403,7 +413,7 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                         const float d = den[AHEAD ? it : 0][BOTH && MODE != TABLE ? h : 0][i];
                         const bool cand = x < bw && d != zero && !(num < hp * d && num > lp * d);
                         if constexpr (MODE == TABLE) {
-                            if (cand) t = score_table(t, num, a.ms, m, Pm, y0 + h, tb.x0 + x, denFlat, l);
+                            if (cand) t = score_table<KEEP == TALLY>(t, num, a.ms, m, Pm, y0 + h, tb.x0 + x, denFlat, l);
                         } else if constexpr (LEAN) {
                             if (cand) t = score_track<FAST>(t, num, d, denFlat, l);
                         } else if (x < bw) {
@@ -524,7 +534,7 @@ __global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, MODE)) k_in
 
 template <int L, bool FAST, Keep MODE>
 void lines_one(const InvArgs &a, dim3 grid, cudaStream_t st) {
-    const size_t smem = Lines<L>::SMEM + (MODE == TABLE ? kBlocksMax * sizeof(float) : 0);
+    const size_t smem = Lines<L>::SMEM + (MODE == TABLE || MODE == TALLY ? kBlocksMax * sizeof(float) : 0);
     set_smem(k_inv_lines<L, FAST, MODE>, smem);
     launch_k(k_inv_lines<L, FAST, MODE>, grid, dim3(Lines<L>::CTA), smem, st, a);
 }
@@ -536,7 +546,7 @@ void lines_form(const InvArgs &a, dim3 grid, cudaStream_t st) {
         k == ALL ? lines_one<L, false, ALL>(a, grid, st)
                  : (k == SOLO ? lines_one<L, false, SOLO>(a, grid, st) : lines_one<L, false, LANES>(a, grid, st));
     else if (a.ms.sat)
-        lines_one<L, true, TABLE>(a, grid, st);
+        a.ms.formed ? lines_one<L, true, TALLY>(a, grid, st) : lines_one<L, true, TABLE>(a, grid, st);
     else
         k == ALL ? lines_one<L, true, ALL>(a, grid, st)
                  : (k == SOLO ? lines_one<L, true, SOLO>(a, grid, st) : lines_one<L, true, LANES>(a, grid, st));

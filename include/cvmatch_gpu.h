@@ -373,11 +373,14 @@ int cvm_fleet_set_overlap(cvm_fleet *f, int on);
  * kernel.  On one tile plan the results are the same bits either way; the
  * autotuner times a bucket's plans for the source the fleet had when it first
  * met the frame size, and plans differ within the fast form's rounding.  A
- * fleet on which this was
- * never called chooses by itself on its first frame of a size (256 RGBA
- * templates on a 2560x1440 frame: 5.6 ms per FindAll with the epilogue, 7.8
- * with the kernel; small templates on flat panels with thin strokes are
- * faster with the kernel).  Not to be called while a FindAll on the same
+ * fleet on which this was never called chooses by itself: by a sample of its
+ * first frame of a size, and again whenever a look at a later call, one in
+ * some tens to thousands, shows that the frames are of another kind (256 RGBA
+ * templates on a 2560x1440 frame: 5.5 ms per FindAll with the epilogue, 7.8
+ * with the kernel; small templates on flat panels with thin strokes, linear
+ * gradients and fleets of a few members are faster with the kernel).  A call
+ * inside a stream capture looks at nothing and runs what the fleet chose
+ * before it, or the epilogue.  Not to be called while a FindAll on the same
  * fleet runs. */
 #define CVM_STATS_KERNEL 0
 #define CVM_STATS_EPILOGUE 1

@@ -31,7 +31,10 @@ struct State {
     std::function<cudaError_t(const std::string &)> on_call;
     std::function<void(const char *, const cvm::FftClass &)> on_launch;
     uintptr_t next = 64;
-    unsigned graphs = 0;
+    // what launch_den_poor and launch_tally report: blocks without a bound per
+    // member, and the rows' steps that formed den, per source
+    int poor = 0;
+    std::function<unsigned long long(int)> formed;
 };
 inline State &state() {
     static State *s = new State;  // outlives the library's own statics
@@ -131,7 +134,11 @@ cudaError_t cudaFreeHost(void *p) { FAKE_CALL(cudaFreeHost); return fake::releas
 cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned) { *d = h; return cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) { memset(a, 0, sizeof *a); return cudaSuccess; }
 cudaError_t cudaMemcpy(void *, const void *, size_t, cudaMemcpyKind) { FAKE_CALL(cudaMemcpy); return cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void *, const void *, size_t, cudaMemcpyKind, cudaStream_t) { FAKE_CALL(cudaMemcpyAsync); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
+    FAKE_CALL(cudaMemcpyAsync);
+    if (n <= 16) memcpy(d, s, n);  // (counters are real, pixels and maps are not)
+    return cudaSuccess;
+}
 cudaError_t cudaMemcpy2DAsync(void *, size_t, const void *, size_t, size_t, size_t, cudaMemcpyKind, cudaStream_t) {
     FAKE_CALL(cudaMemcpy2DAsync);
     return cudaSuccess;
@@ -231,6 +238,19 @@ cudaError_t launch_sep_stats(const uint8_t *, long long, int, int, int ih, const
 }
 cudaError_t launch_vblock(const unsigned int *, unsigned int *B, int nblk, size_t n, cudaStream_t) {
     return fake::launched("vblock", nullptr, B, (size_t)nblk * n * 4);
+}
+cudaError_t launch_den_poor(const MemberSet &ms, int n, int *poor, cudaStream_t) {
+    if (!fake::inside(ms.table, (size_t)n * sizeof(DevMember))) abort();
+    *poor = fake::state().poor * n;
+    return fake::launched("den_poor", nullptr, poor, 4);
+}
+cudaError_t launch_tally(const unsigned int *words, DenTally *out, unsigned int seq, int source, cudaStream_t) {
+    const auto &formed = fake::state().formed;
+    out->source = source;
+    out->poor = words[0];
+    out->formed = formed ? formed(source) : 0;
+    out->seq = seq;
+    return fake::launched("tally", nullptr, words, kTallyWords * 4);
 }
 cudaError_t launch_row_prefix(const uint8_t *, long long, int, int, int, int, unsigned int *P, int, cudaStream_t) {
     return fake::launched("row_prefix", nullptr, P, 4);

@@ -3,10 +3,6 @@
 
 #include "../../cvmatch_gb300/csrc/cvm_api.cpp"
 
-namespace cvm {
-cudaError_t launch_den_poor(const MemberSet &, int, int *, cudaStream_t) { return cudaSuccess; }
-}  // namespace cvm
-
 namespace {
 
 std::vector<uint8_t> frame(1920 * 1080 * 4);
@@ -41,12 +37,77 @@ void tuned_per_source() {
     EXPECT(n == 2);
 }
 
+// Contents as the device would report them.
+enum Content { camera, black, icons, gradient };
+void show(Content c, int n, int size, int w = 640, int h = 480) {
+    const double share[] = {0.04, 0.0, 0.6, 1.0};
+    const unsigned long long steps = n * (((long long)(w - size + 1) * (h - size + 1) + 31) / 32);
+    fake::state().poor = c == icons ? 40 : 0;
+    fake::state().formed = [=](int source) { return source == CVM_STATS_EPILOGUE ? (unsigned long long)(share[c] * steps) : 0; };
+}
+
+// Calls whose den came on demand, of n.
+int on_demand(cvm_fleet *f, int n) {
+    int k = 0;
+    for (int i = 0; i < n; i++) {
+        const long before = fake::state().calls["inv_rows_table"];
+        EXPECT(find(f) == CVM_OK);
+        k += fake::state().calls["inv_rows_table"] > before;
+    }
+    return k;
+}
+
+void the_choice_follows() {
+    cvm_set_autotune(0);
+    for (Content first : {camera, black}) {
+        cvm_fleet *f = fleet(8, 20);
+        show(first, 8, 20);
+        EXPECT(on_demand(f, 1) == 1);
+        show(icons, 8, 20);
+        EXPECT(on_demand(f, 1000) <= 8);
+        show(camera, 8, 20);
+        EXPECT(on_demand(f, 1000) >= 900);
+        show(icons, 8, 20);
+        EXPECT(on_demand(f, 1000) <= 200);
+    }
+    cvm_fleet *f = fleet(8, 20);
+    show(gradient, 8, 20);
+    EXPECT(on_demand(f, 4000) <= 60);
+    show(camera, 8, 20);
+    EXPECT(on_demand(f, 10000) >= 5000);
+    // said once, it stays
+    f = fleet(8, 20);
+    EXPECT(cvm_fleet_set_stats(f, CVM_STATS_EPILOGUE) == CVM_OK);
+    show(icons, 8, 20);
+    EXPECT(on_demand(f, 100) == 100);
+}
+
+// A first call inside a caller's capture samples nothing; a later call does.
+void captured_first() {
+    cvm_set_autotune(0);
+    cvm_fleet *f = fleet(8, 20);
+    show(icons, 8, 20);
+    cvm_result r[8];
+    cudaStream_t st;
+    cudaStreamCreateWithFlags(&st, 0);
+    cudaStreamBeginCapture(st, cudaStreamCaptureModeGlobal);
+    EXPECT(cvm_fleet_find_all_device(f, frame.data(), 4 * 640, 640, 480, r, st) == CVM_OK);
+    cudaGraph_t g;
+    cudaStreamEndCapture(st, &g);
+    EXPECT(fake::state().calls["den_poor"] == 0 && fake::state().calls["tally"] == 0);
+    EXPECT(on_demand(f, 100) <= 4);
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "tuned_per_source")
         tuned_per_source();
+    else if (what == "the_choice_follows")
+        the_choice_follows();
+    else if (what == "captured_first")
+        captured_first();
     else
         return 2;
     return 0;

@@ -7,8 +7,6 @@
 
 namespace {
 
-cudaError_t no_den(const MemberSet &, int, int *, cudaStream_t) { return cudaSuccess; }
-
 std::vector<uint8_t> frame(4096 * 4096 * 4), tpl(512 * 512 * 4);
 
 int call(int w, int h, int tw, int th) {
@@ -175,10 +173,6 @@ void memory_given_back() {
 }
 
 }  // namespace
-
-namespace cvm {
-cudaError_t launch_den_poor(const MemberSet &ms, int n, int *poor, cudaStream_t st) { return no_den(ms, n, poor, st); }
-}  // namespace cvm
 
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
