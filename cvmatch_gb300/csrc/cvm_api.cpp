@@ -2320,6 +2320,9 @@ struct cvm_stream {
     int inflight = 0;
     int graphed = 0;
     int launches = 0;
+    // the fleets' spectra for this frame size, which the graphs use (a fleet
+    // itself keeps those of the size and form it met last)
+    std::shared_ptr<FleetGeom> geom[2];
     ~cvm_stream() {
         for (Slot &sl : slot) {
             if (sl.busy && sl.done) cudaEventSynchronize(sl.done);
@@ -2861,6 +2864,11 @@ int cvm_stream_new(cvm_fleet *color, cvm_fleet *gray, int pw, int ph, cvm_stream
     // build the fleets' caches for this frame size, then capture each slot
     CVM_TRY(stream_pipeline(s.get(), s->slot[0]));
     CVM_CUDA(cudaStreamSynchronize(s->cs));
+    for (int i = 0; i < 2; i++)
+        if (cvm_fleet *f = i ? gray : color) {
+            std::lock_guard<std::mutex> lk(f->mu);
+            s->geom[i] = f->geom;
+        }
     for (cvm_stream::Slot &sl : s->slot) stream_capture(s.get(), sl);
     s->graphed = s->slot[0].exec && s->slot[1].exec;
     if (!s->graphed) {

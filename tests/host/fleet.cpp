@@ -98,6 +98,21 @@ void captured_first() {
     EXPECT(on_demand(f, 100) <= 4);
 }
 
+// A stream's graphs hold their fleet's spectra: they outlive the fleet's use at
+// another size and in another form.
+void a_streams_spectra() {
+    cvm_set_autotune(0);
+    cvm_fleet *f = fleet(8, 20);
+    cvm_stream *s;
+    EXPECT(cvm_stream_new(f, nullptr, 640, 480, &s) == CVM_OK);
+    const std::map<char *, size_t> kept = fake::state().device;
+    EXPECT(find(f, 320, 200) == CVM_OK);
+    EXPECT(cvm_fleet_set_form(f, CVM_FORM_EXACT) == CVM_OK && find(f, 320, 200) == CVM_OK);
+    for (const auto &a : kept) EXPECT(fake::inside(a.first, a.second));
+    cvm_stream_free(s);
+    cvm_fleet_free(f);
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -106,6 +121,8 @@ int main(int argc, char **argv) {
         tuned_per_source();
     else if (what == "the_choice_follows")
         the_choice_follows();
+    else if (what == "a_streams_spectra")
+        a_streams_spectra();
     else if (what == "captured_first")
         captured_first();
     else

@@ -24,3 +24,7 @@ def test_plans_are_tuned_per_source_of_den(fleet):
 @pytest.mark.parametrize("what", ["the_choice_follows", "captured_first"])
 def test_the_source_of_den_follows_the_frames(fleet, what):
     _run(fleet, what)
+
+
+def test_a_stream_keeps_the_spectra_that_its_graphs_use(fleet):
+    _run(fleet, "a_streams_spectra")
