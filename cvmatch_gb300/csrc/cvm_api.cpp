@@ -1512,7 +1512,8 @@ struct DenWatch {
         std::lock_guard<std::mutex> lk(mu);
         return source;
     }
-    // Counts a call; true when it should be tallied, as number *seq.
+    // Counts a call; true when it should be tallied, as number *seq (nullptr:
+    // the call would look, but cannot).
     bool look(int *src, unsigned *seq) {
         std::lock_guard<std::mutex> lk(mu);
         calls++;
@@ -1524,6 +1525,7 @@ struct DenWatch {
         *src = source;
         if (asked && calls - asked > 4096) asked = 0;  // (its call failed)
         if (!tally || asked || calls < next) return false;
+        if (!seq) return true;
         asked = calls;
         next = calls + gap;
         gap = std::min(2 * gap, calm);
@@ -1633,8 +1635,9 @@ void table_roi(const cvm_fleet *f, const FleetBucketGeom &bg, std::vector<DevMem
 // Per parent size: every bucket's plan and every member's spectrum on its
 // bucket's plan (buildGeom, fleet.go:337-390), plus the device member
 // tables the tail kernels index.
+// (use: a geometry of the fleet for this size, instead of its current one)
 int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, int ph, cvm_result *dOut,
-                   cudaStream_t st);
+                   cudaStream_t st, const std::shared_ptr<FleetGeom> &use = nullptr);
 
 // The fleet half of the autotuner: a bucket's plan in the fast forms.  The
 // cost of a plan is measured on trial fleets of the bucket's own members
@@ -2008,7 +2011,7 @@ int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, 
 }
 
 int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, int ph, cvm_result *dOut,
-                   cudaStream_t st) {
+                   cudaStream_t st, const std::shared_ptr<FleetGeom> &use) {
     const int n = (int)f->ms.size();
     for (int i = 0; i < n; i++) {
         cvm_matcher *m = f->ms[i];
@@ -2036,8 +2039,8 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
             CVM_CUDA(upload_bytes(dOut + i, &fr, sizeof fr, st));
         }
     if (f->buckets.empty()) return CVM_OK;
-    std::shared_ptr<FleetGeom> fg;
-    CVM_TRY(fleet_geom(f, dParent, pstride, pw, ph, st, fg));
+    std::shared_ptr<FleetGeom> fg = use;
+    if (!fg) CVM_TRY(fleet_geom(f, dParent, pstride, pw, ph, st, fg));
     {
         // regions of interest changed since the member tables were built
         std::lock_guard<std::mutex> lk(f->mu);
@@ -2312,6 +2315,7 @@ struct cvm_stream {
         cvm_result *dOut = nullptr;  // colour results then gray results
         cvm_result *hOut = nullptr;  // page-locked copy of dOut
         cudaGraphExec_t exec = nullptr;
+        int source[2] = {-1, -1};    // the fleets' sources of den in it (colour, gray)
         cudaEvent_t t0 = nullptr, copied = nullptr, done = nullptr;
         bool busy = false;
     } slot[2];
@@ -2320,8 +2324,8 @@ struct cvm_stream {
     int inflight = 0;
     int graphed = 0;
     int launches = 0;
-    // the fleets' spectra for this frame size, which the graphs use (a fleet
-    // itself keeps those of the size and form it met last)
+    // the fleets' spectra and choices of den's source for this frame size, which
+    // the graphs use (a fleet itself keeps those of the size and form it met last)
     std::shared_ptr<FleetGeom> geom[2];
     ~cvm_stream() {
         for (Slot &sl : slot) {
@@ -2357,20 +2361,31 @@ int stream_pipeline(cvm_stream *s, cvm_stream::Slot &sl) {
         CVM_CUDA(cudaEventRecord(s->fork, s->cs));
         CVM_CUDA(cudaStreamWaitEvent(s->gs, s->fork, 0));
         CVM_CUDA(launch_gray(sl.dFrame, (long long)s->pitch, s->pw, s->ph, sl.dGray, (long long)s->gpitch, s->gs));
-        CVM_TRY(fleet_find_dev(s->gray, sl.dGray, (long long)s->gpitch, s->pw, s->ph, sl.dOut + s->nColor, s->gs));
+        CVM_TRY(fleet_find_dev(s->gray, sl.dGray, (long long)s->gpitch, s->pw, s->ph, sl.dOut + s->nColor, s->gs,
+                               s->graphed ? s->geom[1] : nullptr));
         CVM_CUDA(cudaEventRecord(s->join, s->gs));
     }
-    CVM_TRY(fleet_find_dev(s->color, sl.dFrame, (long long)s->pitch, s->pw, s->ph, sl.dOut, s->cs));
+    CVM_TRY(fleet_find_dev(s->color, sl.dFrame, (long long)s->pitch, s->pw, s->ph, sl.dOut, s->cs,
+                           s->graphed ? s->geom[0] : nullptr));
     if (s->gray) CVM_CUDA(cudaStreamWaitEvent(s->cs, s->join, 0));
     CVM_CUDA(cudaMemcpyAsync(sl.hOut, sl.dOut, (size_t)(s->nColor + s->nGray) * sizeof(cvm_result),
                              cudaMemcpyDeviceToHost, s->cs));
     return CVM_OK;
 }
 
+// The source of den of one of the stream's fleets (-1: not its own choice).
+int stream_source(const cvm_stream *s, int i) {
+    const cvm_fleet *f = i ? s->gray : s->color;
+    return f && f->statsMode < 0 && f->roi.empty() && s->geom[i] && s->geom[i]->watch ? s->geom[i]->watch->now() : -1;
+}
+
 // Capture the slot's pipeline as a graph.  The caches it reads (plans,
 // member spectra) are built by an uncaptured run first.  On any capture
 // failure the stream keeps issuing the pipeline launch by launch.
 void stream_capture(cvm_stream *s, cvm_stream::Slot &sl) {
+    if (sl.exec) cudaGraphExecDestroy(sl.exec);  // (its frame has been pulled)
+    sl.exec = nullptr;
+    for (int i = 0; i < 2; i++) sl.source[i] = stream_source(s, i);
     if (cudaStreamBeginCapture(s->cs, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
         return;
@@ -2861,7 +2876,22 @@ int cvm_stream_new(cvm_fleet *color, cvm_fleet *gray, int pw, int ph, cvm_stream
         CVM_CUDA(cudaEventCreate(&sl.done));
         CVM_CUDA(cudaMemsetAsync(sl.dFrame, 0, s->pitch * ph, s->cs));
     }
-    // build the fleets' caches for this frame size, then capture each slot
+    // Build the fleets' caches for this frame size, then capture each slot.  The
+    // plans are timed on this frame: noise, since a blank one's rows end early.
+    // The fleets' choice of den's source follows the frames that are pushed.
+    {
+        const int rows = std::min(ph, 64);
+        std::vector<uint8_t> noise(s->pitch * rows);
+        uint32_t v = 1;
+        for (size_t i = 0; i < noise.size(); i++) {
+            v = v * 1664525u + 1013904223u;
+            noise[i] = i % 4 == 3 ? 255 : (uint8_t)(v >> 24);
+        }
+        for (int y = 0; y < ph; y += rows)
+            CVM_CUDA(cudaMemcpyAsync(s->slot[0].dFrame + (size_t)y * s->pitch, noise.data(),
+                                     s->pitch * std::min(rows, ph - y), cudaMemcpyHostToDevice, s->cs));
+        CVM_CUDA(cudaStreamSynchronize(s->cs));
+    }
     CVM_TRY(stream_pipeline(s.get(), s->slot[0]));
     CVM_CUDA(cudaStreamSynchronize(s->cs));
     for (int i = 0; i < 2; i++)
@@ -2921,11 +2951,26 @@ int cvm_stream_push(cvm_stream *s, const uint8_t *rgba, int64_t stride) {
         }
     } read{direct ? sl.copied : nullptr};
     CVM_CUDA(cudaStreamWaitEvent(s->cs, sl.copied, 0));
+    // A frame that a fleet looks at for its choice of den's source is queued
+    // launch by launch; so is one whose graph has another source than the
+    // fleet has chosen by now, which is captured again behind it.
+    bool queued = !s->graphed, stale = false;
     if (s->graphed)
-        CVM_CUDA(cudaGraphLaunch(sl.exec, s->cs));
-    else
+        for (int i = 0; i < 2; i++) {
+            int src = stream_source(s, i);
+            if (src < 0) continue;
+            if (s->geom[i]->watch->look(&src, nullptr)) queued = true;
+            if (src != sl.source[i]) queued = stale = true;
+        }
+    if (queued)
         CVM_TRY(stream_pipeline(s, sl));
+    else
+        CVM_CUDA(cudaGraphLaunch(sl.exec, s->cs));
     CVM_CUDA(cudaEventRecord(sl.done, s->cs));
+    if (stale) {
+        stream_capture(s, sl);
+        if (!sl.exec) s->graphed = 0;
+    }
     sl.busy = true;
     s->next ^= 1;
     s->inflight++;

@@ -380,7 +380,8 @@ int cvm_fleet_set_overlap(cvm_fleet *f, int on);
  * with the kernel; small templates on flat panels with thin strokes, linear
  * gradients and fleets of a few members are faster with the kernel).  A call
  * inside a stream capture looks at nothing and runs what the fleet chose
- * before it, or the epilogue.  Not to be called while a FindAll on the same
+ * before it, or the epilogue; a frame stream's graphs are captured again when
+ * its fleets choose anew on the frames pushed.  Not to be called while a FindAll on the same
  * fleet runs. */
 #define CVM_STATS_KERNEL 0
 #define CVM_STATS_EPILOGUE 1

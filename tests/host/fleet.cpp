@@ -113,6 +113,42 @@ void a_streams_spectra() {
     cvm_fleet_free(f);
 }
 
+// A stream's graphs follow what its fleet chooses on the frames pushed, also
+// when the fleet goes on to other sizes.
+void a_stream_follows() {
+    cvm_set_autotune(0);
+    cvm_fleet *f = fleet(8, 20);
+    show(camera, 8, 20);
+    cvm_stream *s;
+    EXPECT(cvm_stream_new(f, nullptr, 640, 480, &s) == CVM_OK);
+    std::vector<cvm_result> r(8);
+    auto pushed = [&](int n) {
+        const long before = fake::state().calls["inv_rows_table"], graphs = fake::state().calls["cudaGraphLaunch"];
+        for (int i = 0; i < n; i++) {
+            EXPECT(cvm_stream_push(s, frame.data(), 4 * 640) == CVM_OK);
+            EXPECT(cvm_stream_pull(s, r.data(), nullptr, nullptr) == CVM_OK);
+        }
+        EXPECT(fake::state().calls["cudaGraphLaunch"] - graphs > n * 8 / 10);
+        return fake::state().calls["inv_rows_table"] - before;
+    };
+    pushed(100);
+    show(icons, 8, 20);
+    pushed(100);
+    EXPECT(pushed(1000) == 0);
+    show(camera, 8, 20);
+    pushed(400);
+    EXPECT(pushed(1000) > 0);  // the looks, and a capture before them
+    int graphed = 0, launches = 0;
+    EXPECT(cvm_stream_info(s, &graphed, &launches) == CVM_OK && graphed);
+    // the fleet is used at another size meanwhile
+    EXPECT(find(f, 320, 200) == CVM_OK);
+    show(icons, 8, 20);
+    pushed(200);
+    EXPECT(find(f, 320, 200) == CVM_OK);
+    pushed(200);
+    cvm_stream_free(s);
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -123,6 +159,8 @@ int main(int argc, char **argv) {
         the_choice_follows();
     else if (what == "a_streams_spectra")
         a_streams_spectra();
+    else if (what == "a_stream_follows")
+        a_stream_follows();
     else if (what == "captured_first")
         captured_first();
     else

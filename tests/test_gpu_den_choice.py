@@ -143,3 +143,42 @@ def test_a_capture_uses_what_the_frames_chose():
         torch.cuda.synchronize()
         assert np.array_equal(out.cpu().numpy(), want)
     assert not on_demand(f, frame)
+
+
+@pytest.mark.parametrize("order", [("strokes", "noise"), ("noise", "strokes")])
+def test_a_stream_follows_the_frames_pushed(order):
+    rng = np.random.default_rng(5)
+    frames = {"strokes": _strokes(rng), "noise": _noise(rng)}
+    ms = icons(rng, frames["noise"], 64)
+
+    def device_ms(s, frame):
+        t = []
+        for _ in range(21):
+            s.push(frame)
+            t.append(s.pull()[2])
+        return sorted(t)[10]
+
+    auto = cvm.SetAutotune(False)
+    try:
+        f, fixed = _fleet(ms), {}
+        for mode in (cvm.STATS_KERNEL, cvm.STATS_EPILOGUE):
+            g = _fleet(ms)
+            g.SetStats(mode)
+            fixed[mode] = (g, cvm.NewStream(g, None, W, H))
+        s = cvm.NewStream(f, None, W, H)
+        assert s.info()[0]
+        for name in order:
+            frame = frames[name]
+            want = [tuple(r) for r in fixed[cvm.STATS_KERNEL][0].FindAll(frame)]
+            for k in range(160):
+                s.push(frame)
+                if k % 3 == 0:  # two frames in flight
+                    s.push(frame)
+                    assert [tuple(r) for r in s.pull()[0]] == want
+                assert [tuple(r) for r in s.pull()[0]] == want
+            assert s.info()[0]
+            assert on_demand(f, frame) == (name == "noise")
+            best = min(device_ms(t, frame) for _, t in fixed.values())
+            assert device_ms(s, frame) < 1.1 * best, name
+    finally:
+        cvm.SetAutotune(auto)

@@ -21,7 +21,7 @@ def test_plans_are_tuned_per_source_of_den(fleet):
     _run(fleet, "tuned_per_source")
 
 
-@pytest.mark.parametrize("what", ["the_choice_follows", "captured_first"])
+@pytest.mark.parametrize("what", ["the_choice_follows", "captured_first", "a_stream_follows"])
 def test_the_source_of_den_follows_the_frames(fleet, what):
     _run(fleet, what)
 
