@@ -145,16 +145,19 @@ __device__ __noinline__ Track score_table(Track t, float num, const MemberSet &m
 // 2.01 ms; without them 14 CTAs 2.00 at the same 4096 elements per CTA); the
 // exact form keeps the channel sum of its 16 results, 128 registers (nine
 // CTAs spill: 1.17 against 0.84 ms).  With every score (mode 0) the quotients
-// of all results are in flight: three quarters of the CTAs, but all of them
-// for the fast form's 2048 points (a 4K gray map: three CTAs 56.6 us, four
-// 50.6, five 46.9, six 48.4) and six for the exact form's 256 points (1280x800
-// with 32x32, RGB: three 27.6 us, six 22.7, seven 24.8; 128 points: three
-// 32.9, six 35.0).
+// of all results are in flight too.  Score maps at every length, us with 3, 5,
+// 6, 7 and 8 CTAs, RGB in the exact form and gray in the fast form:
+//    128  320x200, 16x16       exact 17.8 19.2 18.4 19.9 20.0  fast 14.3 14.3 14.4 14.7 14.4
+//    256  1280x800, 32x32      exact 27.6 26.6 23.7 25.6 24.8  fast 16.8 16.5 16.7 17.0 16.7
+//    512  1366x767, 133x71     exact 34.3 28.8 25.0 28.6 28.7  fast 26.8 19.1 19.4 19.9 19.4
+//    512  2560x1440, 100x60    exact 86.2 92.8 81.1 81.0 81.4  fast 64.6 57.2 56.8 50.3 48.7
+//   1024  1920x1080, 96x32     exact 43.4 53.6 49.4 38.0 37.2  fast 26.5 26.8 26.8 20.6 20.2
+//   1024  2560x1440, 128x128   exact 73.9 74.4 69.0 63.5 65.3  fast 45.2 39.4 39.4 34.4 34.9
+//   2048  3840x2160, 256x256   exact 94.4 134.9 170 170 170    fast 56.9 46.1 47.7 46.8 46.0
 __host__ __device__ constexpr int lines_ctas(int L, bool fast, int mode) {
-    return mode == 2 || mode == 4      ? (L == 11 ? 4 : (L <= 8 ? 8 : 9))
-           : mode == 0 && L == 8 && !fast ? 6
-                                       : (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 5) : (fast ? 10 : 8))) *
-                                             (mode || (L == 11 && fast) ? 4 : 3) / 4;
+    return mode == 2 || mode == 4 ? (L == 11 ? 4 : (L <= 8 ? 8 : 9))
+           : mode == 0            ? (fast ? (L == 11 ? 5 : 7) : (L == 7 || L == 11 ? 3 : (L == 10 ? 7 : 6)))
+                                  : (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 5) : (fast ? 10 : 8)));
 }
 
 // What a launch keeps of its results.  ALL: every score may be wanted (a
