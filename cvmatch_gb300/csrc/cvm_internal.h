@@ -117,8 +117,8 @@ struct MemberSet {
     // cores).  Nonzero selects the fast form's arithmetic everywhere else.
     int form;
     // Fast-form fleet waves without score maps or regions of interest: the
-    // frame's summed-area table of the shared row prefix (ih + 1 rows, the
-    // prefix's lanes; all sums modulo 2^32), from which the inverse rows form
+    // frame's summed-area table (launch_sat: ih + 1 rows of hp columns, the
+    // row prefix's lanes; all sums modulo 2^32), from which the inverse rows form
     // the den of the windows that may be extrema (nullptr: the statistics
     // kernel filled `lanes`).
     const unsigned int *sat;

@@ -675,10 +675,12 @@ __global__ void __launch_bounds__(256) k_fwd_rows_t(FwdRowsArgs a, const __grid_
 // z[kk] and its mirror z[N-kk]; the channels accumulate in channel order;
 // the epilogue scores with the per-result (t, den) lanes and keeps
 // first-occurrence extrema merged by each member's last CTA.
-template <int LOG2N, bool FAST>
+// RAW: the raw correlation of the fixed-scratch entry point, for the lengths
+// that cvm_lines.cu scores.
+template <int LOG2N, bool FAST, bool RAW = false>
 // Occupancy: the fast form's radix-16 last pass budgets two CTAs per SM;
-// its radix-4 last pass four (64 registers, with four row pairs per CTA in
-// fleets: rows_fast_pairs), the exact form three.
+// its radix-4 last pass four (64 registers, 4096 elements per CTA in
+// fleets: inv_rows_ctas_per_tile), the exact form three.
 __global__ void __launch_bounds__(256, FAST ? (last_pass_r(LOG2N) == 16 ? 2 : 4) : 3) k_inv_rows_t(InvArgs a) {
     griddep_wait();
     constexpr int N = 1 << LOG2N, LD = Line<LOG2N>::LD, HALF = N / 2;
@@ -717,7 +719,7 @@ __global__ void __launch_bounds__(256, FAST ? (last_pass_r(LOG2N) == 16 ? 2 : 4)
     // the fixed-scratch entry point, which takes the raw correlation)
     // (a radix-16 last pass only in the fast form, which budgets the
     // registers for it: two CTAs per SM)
-    const bool fuse = (last_pass_r(LOG2N) == 4 || FAST) && a.ms.lanes != nullptr;
+    const bool fuse = !RAW && (last_pass_r(LOG2N) == 4 || FAST) && a.ms.lanes != nullptr;
     if (P > 0 && !flat) {
         const int cn = fast ? 1 : Pm.cn;
         const size_t chanStride = (size_t)fc.dftH * hwp;
@@ -776,7 +778,7 @@ __global__ void __launch_bounds__(256, FAST ? (last_pass_r(LOG2N) == 16 ? 2 : 4)
             __syncthreads();
         }
     }
-    if (!a.ms.lanes) {
+    if (RAW || !a.ms.lanes) {
         // No statistics lanes: store the raw correlation for k_norm instead.
         if (P > 0 && !flat) {
             float *corr = a.ms.corr + (size_t)slot * a.ms.corrStride;
@@ -1008,8 +1010,8 @@ void fwd_one(const FwdRowsArgs &a, const CUtensorMap &map, dim3 grid, int thread
 // fixed-scratch entry point (the exact form, no statistics lanes).
 template <int L>
 void inv_raw(const InvArgs &a, dim3 grid, size_t smem, cudaStream_t st) {
-    set_smem(k_inv_rows_t<L, false>, smem);
-    launch_k(k_inv_rows_t<L, false>, grid, dim3(kThreads), smem, st, a);
+    set_smem(k_inv_rows_t<L, false, true>, smem);
+    launch_k(k_inv_rows_t<L, false, true>, grid, dim3(kThreads), smem, st, a);
 }
 
 template <int L>
@@ -1018,19 +1020,14 @@ void inv_one(const InvArgs &a, dim3 grid, size_t smem, cudaStream_t st) {
         set_smem(k_inv_rows_t<L, true>, smem);
         launch_k(k_inv_rows_t<L, true>, grid, dim3(kThreads), smem, st, a);
     } else {
-        inv_raw<L>(a, grid, smem, st);
+        set_smem(k_inv_rows_t<L, false>, smem);
+        launch_k(k_inv_rows_t<L, false>, grid, dim3(kThreads), smem, st, a);
     }
 }
 
 }  // namespace
 
 bool rows_fixed_length(int log2n) { return log2n >= 5 && log2n <= 12; }
-
-// Elements per CTA of a fleet wave's fast-form inverse rows: a radix-4
-// last pass runs four CTAs per SM, whose shared memory holds 4096 elements
-// each (C4's 78-member waves of 1024-point rows: 3.56 -> 3.38 ms per frame
-// against 8192 at three CTAs); a radix-16 last pass keeps 8192 at two.
-int rows_fast_wave_elems(int log2n) { return log2n >= 5 && log2n <= 12 && last_pass_r(log2n) == 4 ? 4096 : 8192; }
 
 void launch_fwd_rows_fixed(const FwdRowsArgs &a, const CUtensorMap &map, dim3 grid, int threads, size_t smem,
                            cudaStream_t st) {
