@@ -1663,21 +1663,25 @@ struct FleetTuneEntry {
 };
 std::map<FleetTuneKey, FleetTuneEntry> g_fleetTune;
 
+// Whether nothing is left to measure for the bucket's plan: tuning off or not
+// for it (*out as it is), or tuned already (*out, when given).
+bool settled_bucket_plan(const cvm_fleet *f, const Bucket &b, int pw, int ph, int stats, Plan *out) {
+    const int nm = (int)b.members.size();
+    if (f->form == CVM_FORM_EXACT || !g_autotune.load() || nm < 4) return true;
+    std::lock_guard<std::mutex> lk(g_tuneMu);
+    auto it = g_fleetTune.find(FleetTuneKey{pw, ph, b.tw, b.th, f->step, f->form, nm, stats});
+    if (it == g_fleetTune.end()) return false;
+    if (out) *out = it->second.plan;
+    return true;
+}
+
 int tune_bucket_plan(cvm_fleet *f, const Bucket &b, const uint8_t *dParent, long long pstride, int pw, int ph,
                      cudaStream_t st, int stats, Plan *out) {
     const int rwF = pw - b.tw + 1, rhF = ph - b.th + 1;
     *out = make_plan(b.tw, b.th, rwF, rhF);
     const int nm = (int)b.members.size();
-    if (f->form == CVM_FORM_EXACT || !g_autotune.load() || nm < 4 || !dParent) return CVM_OK;
+    if (!dParent || settled_bucket_plan(f, b, pw, ph, stats, out)) return CVM_OK;
     const FleetTuneKey key{pw, ph, b.tw, b.th, f->step, f->form, nm, stats};
-    {
-        std::lock_guard<std::mutex> lk(g_tuneMu);
-        auto it = g_fleetTune.find(key);
-        if (it != g_fleetTune.end()) {
-            *out = it->second.plan;
-            return CVM_OK;
-        }
-    }
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
@@ -1847,9 +1851,11 @@ std::vector<Bucket> fast_buckets(const cvm_fleet *f, int pw, int ph) {
 }
 
 // The first frame's choice of den's source (DenWatch), for a fast-form fleet
-// that cvm_fleet_set_stats left to itself: a sample of its members' blocks.
-// Inside a capture nothing is sampled: on demand, until a later call looks.
-int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, int ph, cudaStream_t cst,
+// that cvm_fleet_set_stats left to itself: a sample of its members' blocks,
+// when the call may wait for the caller's stream (wait: it is about to time
+// plans on that frame).  Else, and inside a capture, nothing is sampled: on
+// demand, until a later call looks.
+int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, int ph, cudaStream_t cst, bool wait,
                  std::unique_ptr<DenWatch> &out) {
     if (f->form != CVM_FORM_FAST || f->forcedPlan.dftW > 0) return CVM_OK;
     const int np = f->step == 4 ? 4 : 2, hp = (int)align_up((size_t)pw + 1, 32);
@@ -1885,7 +1891,7 @@ int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw
     }
     cudaGetLastError();
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (f->statsMode >= 0 || !dParent || cudaStreamIsCapturing(cst, &cs) != cudaSuccess ||
+    if (!wait || f->statsMode >= 0 || !dParent || cudaStreamIsCapturing(cst, &cs) != cudaSuccess ||
         cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         out = std::move(w);
@@ -1939,11 +1945,14 @@ int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, 
     fg->pw = pw;
     fg->ph = ph;
     fg->form = f->form;
-    CVM_TRY(choose_stats(f, dParent, pstride, pw, ph, cst, fg->watch));
-    const int stats = f->statsMode >= 0 ? f->statsMode : (fg->watch ? fg->watch->source : CVM_STATS_KERNEL);
-    cudaStream_t st = thread_stream();
     const std::vector<Bucket> buckets =
         f->form != CVM_FORM_EXACT && f->forcedPlan.dftW == 0 ? fast_buckets(f, pw, ph) : f->buckets;
+    bool wait = false;
+    for (const Bucket &b : buckets)
+        wait = wait || !settled_bucket_plan(f, b, pw, ph, CVM_STATS_EPILOGUE, nullptr);
+    CVM_TRY(choose_stats(f, dParent, pstride, pw, ph, cst, wait, fg->watch));
+    const int stats = f->statsMode >= 0 ? f->statsMode : (fg->watch ? fg->watch->source : CVM_STATS_KERNEL);
+    cudaStream_t st = thread_stream();
     for (const Bucket &b : buckets) {
         auto bg = std::make_unique<FleetBucketGeom>();
         const int rwF = pw - b.tw + 1, rhF = ph - b.th + 1;

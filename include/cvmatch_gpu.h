@@ -276,8 +276,8 @@ int cvm_get_form(void);
  * FindAll of a frame size does the same per bucket of four or more members
  * (buildGeom's plan, fleet.go:356-365, against the candidates), timing
  * trial fleets of k and 2k of the bucket's own members so that the cost is
- * shared + members x per-member.  Calls made while their stream is being
- * captured do not tune.  cvm_set_autotune returns the previous setting.
+ * shared + members x per-member; that call waits for the caller's stream.
+ * Calls made while their stream is being captured do not tune.  cvm_set_autotune returns the previous setting.
  * No reference counterpart (the reference always plans with newGoPlan). */
 int cvm_set_autotune(int on);
 /* The tuned shapes as a JSON array (frame, template, mode, cn, step, form,
@@ -374,7 +374,7 @@ int cvm_fleet_set_overlap(cvm_fleet *f, int on);
  * autotuner times a bucket's plans for the source the fleet had when it first
  * met the frame size, and plans differ within the fast form's rounding.  A
  * fleet on which this was never called chooses by itself: by a sample of its
- * first frame of a size, and again whenever a look at a later call, one in
+ * first frame of a size, when plans are timed on it, and again whenever a look at a later call, one in
  * some tens to thousands, shows that the frames are of another kind (256 RGBA
  * templates on a 2560x1440 frame: 5.5 ms per FindAll with the epilogue, 7.8
  * with the kernel; small templates on flat panels with thin strokes, linear

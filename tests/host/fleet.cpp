@@ -149,6 +149,23 @@ void a_stream_follows() {
     cvm_stream_free(s);
 }
 
+// Only a call that times plans waits for the caller's stream.
+void no_waiting() {
+    cvm_result r[8];
+    cudaStream_t st;
+    cudaStreamCreateWithFlags(&st, 0);
+    auto waits = [&](cvm_fleet *f) {
+        fake::state().synced.clear();
+        EXPECT(cvm_fleet_find_all_device(f, frame.data(), 4 * 640, 640, 480, r, st) == CVM_OK);
+        return fake::state().synced.count(st) > 0;
+    };
+    EXPECT(!waits(fleet(3, 20)));                      // too few to tune
+    EXPECT(waits(fleet(8, 20)));                       // tunes
+    EXPECT(!waits(fleet(8, 20)));                      // tuned before
+    cvm_set_autotune(0);
+    EXPECT(!waits(fleet(7, 21)));
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -161,6 +178,8 @@ int main(int argc, char **argv) {
         a_streams_spectra();
     else if (what == "a_stream_follows")
         a_stream_follows();
+    else if (what == "no_waiting")
+        no_waiting();
     else if (what == "captured_first")
         captured_first();
     else

@@ -28,3 +28,7 @@ def test_the_source_of_den_follows_the_frames(fleet, what):
 
 def test_a_stream_keeps_the_spectra_that_its_graphs_use(fleet):
     _run(fleet, "a_streams_spectra")
+
+
+def test_only_a_call_that_times_plans_waits_for_the_callers_stream(fleet):
+    _run(fleet, "no_waiting")
