@@ -840,6 +840,20 @@ int check_image(const void *p, int w, int h) {
     return CVM_OK;
 }
 
+// The address by which a kernel may read the n bytes of host memory at p:
+// anything where the device reads pageable memory coherently, else
+// page-locked memory (its last byte included, in one mapping with the first);
+// nullptr: through the copy engine.
+const uint8_t *device_view(const uint8_t *p, size_t n) {
+    if (dev().pageable) return p;
+    cudaPointerAttributes a, b;
+    const bool ok = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost && a.devicePointer &&
+                    cudaPointerGetAttributes(&b, p + n - 1) == cudaSuccess && b.type == cudaMemoryTypeHost &&
+                    static_cast<const uint8_t *>(b.devicePointer) == static_cast<const uint8_t *>(a.devicePointer) + n - 1;
+    cudaGetLastError();  // an unregistered pointer's query leaves no error behind
+    return ok ? static_cast<const uint8_t *>(a.devicePointer) : nullptr;
+}
+
 // Copies a host image to a device buffer with a 128-byte aligned pitch.
 // Per-thread page-locked staging for small pageable inputs (templates,
 // small frames): the copy out of it is asynchronous, so a call's launches
@@ -884,24 +898,17 @@ int upload_image(PoolBuf &b, const uint8_t *src, long long stride, int w, int h,
     const size_t row = (size_t)w * bpp;
     *pitch = (long long)align_up(row, 128);
     CVM_TRY(pool_alloc(b, (size_t)*pitch * h, st));
-    // Page-locked caller memory that the device can address is read by a
-    // kernel over the host link (several times the copy engine's rate for
-    // a frame); anything else goes through the copy engine.
-    cudaPointerAttributes at;
-    if ((size_t)row * h >= (size_t(1) << 20) && cudaPointerGetAttributes(&at, src) == cudaSuccess &&
-        at.type == cudaMemoryTypeHost && at.devicePointer) {
-        CVM_CUDA(launch_ingest(b.p, (size_t)*pitch, at.devicePointer, (size_t)stride, row, h, st));
-        return CVM_OK;
-    }
-    cudaGetLastError();  // an unregistered pointer's query leaves no error behind
-    // A device that reads pageable host memory coherently (a Grace host's
-    // NVLink-C2C address translation) takes the caller's ordinary memory the
-    // same way: no synchronous staged copy by the driver, so the transfer
-    // overlaps the call's queued launches as a page-locked frame's does.
-    // The caller's buffer stays valid until the call returns (it
-    // synchronises before returning).
-    if (dev().pageable && (size_t)row * h >= (size_t(64) << 10)) {
-        CVM_CUDA(launch_ingest(b.p, (size_t)*pitch, src, (size_t)stride, row, h, st));
+    // Caller memory that the device can read is read by a kernel over the host
+    // link: page-locked frames at several times the copy engine's rate, ordinary
+    // memory (a Grace host's NVLink-C2C address translation) with no synchronous
+    // staged copy by the driver, so that the transfer overlaps the call's queued
+    // launches; anything else goes through the copy engine.  The caller's buffer
+    // stays valid until the call returns (it waits before returning).
+    const uint8_t *view = row * h >= (dev().pageable ? size_t(64) << 10 : size_t(1) << 20)
+                              ? device_view(src, (size_t)(h - 1) * stride + row)
+                              : nullptr;
+    if (view) {
+        CVM_CUDA(launch_ingest(b.p, (size_t)*pitch, view, (size_t)stride, row, h, st));
         return CVM_OK;
     }
     if (row * h <= (size_t(4) << 20)) {
@@ -2934,11 +2941,7 @@ int cvm_stream_push(cvm_stream *s, const uint8_t *rgba, int64_t stride) {
     // through page-locked staging.  (The host's copy into staging took 0.5 ms
     // of an 8.3 MB frame, before the matching could start; the kernel 50 us:
     // two 1920x1080 frames pushed and pulled 2.92 -> 2.35 ms.)
-    const uint8_t *direct = dev().pageable ? rgba : nullptr;
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, rgba) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer)
-        direct = static_cast<const uint8_t *>(at.devicePointer);
-    cudaGetLastError();  // an unregistered pointer's query leaves no error behind
+    const uint8_t *direct = device_view(rgba, (size_t)(s->ph - 1) * stride + row);
     if (direct) {
         CVM_CUDA(cudaEventRecord(sl.t0, s->xs));
         CVM_CUDA(launch_ingest(sl.dFrame, s->pitch, direct, (size_t)stride, row, s->ph, s->xs));

@@ -31,6 +31,9 @@ struct State {
     std::function<cudaError_t(const std::string &)> on_call;
     std::function<void(const char *, const cvm::FftClass &)> on_launch;
     uintptr_t next = 64;
+    // host memory that the device can read: all of it, or one page-locked range
+    int pageable = 1;
+    const char *lockedFrom = nullptr, *lockedTo = nullptr;
     // what launch_den_poor and launch_tally report: blocks without a bound per
     // member, and the rows' steps that formed den, per source
     int poor = 0;
@@ -115,7 +118,10 @@ cudaError_t cudaGetDeviceProperties(cudaDeviceProp *p, int) {
     p->minor = 3;
     return cudaSuccess;
 }
-cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { *v = 1; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
+    *v = a == cudaDevAttrPageableMemoryAccess ? fake::state().pageable : 1;
+    return cudaSuccess;
+}
 cudaError_t cudaDeviceGetStreamPriorityRange(int *least, int *greatest) { *least = 0; *greatest = -5; return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
@@ -132,7 +138,15 @@ cudaError_t cudaFreeAsync(void *p, cudaStream_t) { FAKE_CALL(cudaFreeAsync); ret
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { FAKE_CALL(cudaHostAlloc); return fake::alloc(p, n, fake::state().pinned, false); }
 cudaError_t cudaFreeHost(void *p) { FAKE_CALL(cudaFreeHost); return fake::release(p, fake::state().pinned, false); }
 cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned) { *d = h; return cudaSuccess; }
-cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) { memset(a, 0, sizeof *a); return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {
+    memset(static_cast<void *>(a), 0, sizeof *a);
+    const char *c = static_cast<const char *>(p);
+    if (c >= fake::state().lockedFrom && c < fake::state().lockedTo) {
+        a->type = cudaMemoryTypeHost;
+        a->devicePointer = a->hostPointer = const_cast<char *>(c);
+    }
+    return cudaSuccess;
+}
 cudaError_t cudaMemcpy(void *, const void *, size_t, cudaMemcpyKind) { FAKE_CALL(cudaMemcpy); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
     FAKE_CALL(cudaMemcpyAsync);

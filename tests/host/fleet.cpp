@@ -166,6 +166,28 @@ void no_waiting() {
     EXPECT(!waits(fleet(7, 21)));
 }
 
+// Without coherent access to pageable memory a kernel reads a caller's frame
+// only when all of it is page-locked.
+void partly_locked() {
+    auto &st = fake::state();
+    st.pageable = 0;
+    cvm_set_autotune(0);
+    cvm_fleet *f = fleet(3, 20);
+    cvm_stream *s;
+    EXPECT(cvm_stream_new(f, nullptr, 640, 480, &s) == CVM_OK);
+    std::vector<cvm_result> r(3);
+    for (int locked : {0, 1, 2}) {  // none, half, all of the frame
+        st.lockedFrom = reinterpret_cast<const char *>(frame.data());
+        st.lockedTo = st.lockedFrom + (size_t)locked * 640 * 480 * 2;
+        const long before = st.calls["ingest"];
+        EXPECT(cvm_stream_push(s, frame.data(), 4 * 640) == CVM_OK);
+        EXPECT(cvm_stream_pull(s, r.data(), nullptr, nullptr) == CVM_OK);
+        EXPECT(find(f) == CVM_OK);
+        EXPECT(st.calls["ingest"] - before == (locked == 2 ? 2 : 0));
+    }
+    cvm_stream_free(s);
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -180,6 +202,8 @@ int main(int argc, char **argv) {
         a_stream_follows();
     else if (what == "no_waiting")
         no_waiting();
+    else if (what == "partly_locked")
+        partly_locked();
     else if (what == "captured_first")
         captured_first();
     else

@@ -32,3 +32,7 @@ def test_a_stream_keeps_the_spectra_that_its_graphs_use(fleet):
 
 def test_only_a_call_that_times_plans_waits_for_the_callers_stream(fleet):
     _run(fleet, "no_waiting")
+
+
+def test_a_kernel_reads_only_frames_that_are_locked_whole(fleet):
+    _run(fleet, "partly_locked")
