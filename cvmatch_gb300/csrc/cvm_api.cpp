@@ -1054,6 +1054,12 @@ struct SoloPool {
     size_t bytes = 0;           // of all graphs, idle or not
     int graphs = 0;
     uint64_t tick = 0;
+    // (what a lease's end and a call's count need is here from the start:
+    // neither can throw on the way out of a C entry point)
+    SoloPool() {
+        idle.reserve(kGraphs);
+        shapes.reserve(kGraphShapes);
+    }
 
     // The shape's record (mu held).
     Shape &shape(const SoloKey &key) {
