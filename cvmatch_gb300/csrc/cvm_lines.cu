@@ -160,14 +160,18 @@ __host__ __device__ constexpr int lines_ctas(int L, bool fast, int mode) {
                                   : (L == 11 ? (fast ? 5 : 4) : (L <= 8 ? (fast ? 10 : 5) : (fast ? 10 : 8)));
 }
 
-// What a launch keeps of its results.  ALL: every score may be wanted (a
-// score map, regions of interest).  LANES: the extrema alone, den (and t)
+// What a launch keeps of its results.  ALL: every score is wanted (a score
+// map).  LANES: the extrema alone, den (and t)
 // from the statistics kernel's lanes.  TABLE: a fast-form fleet's extrema,
 // den on demand.  SOLO: LANES for a single match, whose CTAs all start at once
 // with no extrema of earlier ones to cut by (fleets keep their registers).
 // TALLY: TABLE in a tallied call (MemberSet::formed; the test for it alone, in
-// TABLE's registers, cost the rows 4 %).
-enum Keep { ALL, LANES, TABLE, SOLO, TALLY };
+// TABLE's registers, cost the rows 4 %).  ROI: LANES for members with regions of
+// interest, whose results outside are no candidates and whose row pairs outside
+// are not transformed.  (40 gray members on 1280x720, a quarter of the frame
+// each: 254.8 us a call; 393 with every score kept and all results of a CTA that
+// holds any of the region scored.)
+enum Keep { ALL, LANES, TABLE, SOLO, TALLY, ROI };
 
 // The extrema (and scores) of the CTA's row pairs.
 template <int L, bool FAST, Keep KEEP>
@@ -197,7 +201,9 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
     const float *dens = reinterpret_cast<const float *>(lanes);
     const float denFlat = near_flat_den(m.tw, m.th, Pm.templNorm);  // fast form: near-flat windows below it
     float *map = LEAN ? nullptr : a.ms.map;
-    const int rw = m.rw, xlo = m.roiX0 - tb.x0, xhi = m.roiX1 - tb.x0, roiY0 = m.roiY0, roiY1 = m.roiY1;
+    const int rw = m.rw, roiY0 = m.roiY0, roiY1 = m.roiY1;
+    // the columns that may be extrema
+    const int xa = MODE == ROI ? max(m.roiX0 - tb.x0, 0) : 0, xb = MODE == ROI ? min(m.roiX1 - tb.x0, bw) : bw;
     const float2 *triW = fc.triW;
     int j2, b2;
     pass2_unit<L>(lt, j2, b2);
@@ -253,7 +259,8 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
         }
     };
     float2 acc[FAST ? 1 : 16];                        // the earlier channels' sum, the thread's results
-    for (int p = g; p < P; p += NL)
+    for (int p = g; p < P; p += NL) {
+        if (MODE == ROI && (tb.y0 + 2 * (pair0 + p) + 2 <= roiY0 || tb.y0 + 2 * (pair0 + p) >= roiY1)) continue;
 #pragma unroll 1
         for (int k = 0; k < cn; k++) {
             // pass 1: unit k0's elements are Z[k0 + K1 * brev(i)]
@@ -261,7 +268,7 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
             // above (impl.go:405-413)
             const float2 *ur = row_ptr(p, k, 0), *vr = row_ptr(p, k, 1);
             // the member's extrema so far, used at the line's end
-            const bool posted = LEAN && bnd && k == cn - 1 && (MODE == TABLE || p < NL);
+            const bool posted = LEAN && bnd && k == cn - 1 && (MODE == TABLE || MODE == ROI || p < NL);
             uint2 keys = make_uint2(0u, 0u);
             if (posted) {
                 keys.x = *reinterpret_cast<const volatile unsigned int *>(bnd);
@@ -310,7 +317,7 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
             auto load_den = [&](int it, int h) {
                 const int jj = lt + it * G, is = AHEAD ? it : 0, hs = BOTH ? h : 0;
                 const long long row = row0 + h * rw;
-                const int xe = h == 0 || odd ? bw : 0;
+                const int xe = h == 0 || odd ? xb : 0;
 #pragma unroll
                 for (int i = 0; i < RL; i++) {
                     const int x = jj + HL * i;
@@ -318,9 +325,10 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                         den[is][hs][i] = lbs[blockRow + (min(x, bw - 1) >> lgx)];  // its bound
                     } else {
                         float2 td = make_float2(0.f, 0.f);
+                        const bool in = x < xe && (MODE != ROI || x >= xa);
                         if constexpr (FAST)
-                            td.y = x < xe ? ld_once(dens + row + x) : 0.f;
-                        else if (x < xe)
+                            td.y = in ? ld_once(dens + row + x) : 0.f;
+                        else if (in)
                             td = ld_once(lanes + row + x);
                         if constexpr (!FAST) tt[hs][i] = td.x;
                         den[is][hs][i] = td.y;
@@ -408,21 +416,22 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                 for (int h = 0; h < 2; h++) {
                     if (h == 1 && !odd) break;
                     if (h == 1 && !BOTH && MODE != TABLE) load_den(it, 1);
-                    const bool rowIn = y0 + h >= roiY0 && y0 + h < roiY1;
+                    if (MODE == ROI && (y0 + h < roiY0 || y0 + h >= roiY1)) continue;
 #pragma unroll
                     for (int i = 0; i < RL; i++) {
                         const int x = jj + HL * i, l = (2 * p + h) * N + x;
                         const float num = numer(h, i);
                         const float d = den[AHEAD ? it : 0][BOTH && MODE != TABLE ? h : 0][i];
-                        const bool cand = x < bw && d != zero && !(num < hp * d && num > lp * d);
+                        const bool cand = x < xb && (MODE != ROI || x >= xa) && d != zero &&
+                                          !(num < hp * d && num > lp * d);
                         if constexpr (MODE == TABLE) {
                             if (cand) t = score_table<KEEP == TALLY>(t, num, a.ms, m, Pm, y0 + h, tb.x0 + x, denFlat, l);
                         } else if constexpr (LEAN) {
                             if (cand) t = score_track<FAST>(t, num, d, denFlat, l);
                         } else if (x < bw) {
                             const float sc = FAST ? score_fast(num, d, denFlat) : score_exact(num, d);
-                            if (map) map[row0 + h * rw + x] = sc;
-                            if (rowIn && x >= xlo && x < xhi) track(t, sc, l);
+                            map[row0 + h * rw + x] = sc;
+                            track(t, sc, l);
                         }
                     }
                 }
@@ -446,6 +455,7 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                 }
             }
         }
+    }
     // widen: CTA-local (row, x) -> the member's raster index
     auto widen = [&](int l) {
         return l == INT_MAX ? LLONG_MAX
@@ -480,7 +490,7 @@ __global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, MODE)) k_in
     // the CTA's row pairs; none when its results all lie outside the
     // member's region of interest (no transform, no extrema)
     int P = 2 * pair0 < bh ? min(a.pairsPerCta, (bh - 2 * pair0 + 1) >> 1) : 0;
-    if (MODE == ALL && P > 0 && a.ms.anyRoi) {
+    if (MODE == ROI && P > 0) {
         const int ya = tb.y0 + 2 * pair0, yb = tb.y0 + min(2 * (pair0 + P), bh);
         if (ya >= m.roiY1 || yb <= m.roiY0 || tb.x0 >= m.roiX1 || tb.x0 + bw <= m.roiX0) P = 0;
     }
@@ -544,15 +554,17 @@ void lines_one(const InvArgs &a, dim3 grid, cudaStream_t st) {
 
 template <int L>
 void lines_form(const InvArgs &a, dim3 grid, cudaStream_t st) {
-    const Keep k = a.ms.map || a.ms.anyRoi ? ALL : (a.ms.table ? LANES : SOLO);
+    const Keep k = a.ms.map ? ALL : (a.ms.anyRoi ? ROI : (a.ms.table ? LANES : SOLO));
     if (!a.ms.form)
         k == ALL ? lines_one<L, false, ALL>(a, grid, st)
-                 : (k == SOLO ? lines_one<L, false, SOLO>(a, grid, st) : lines_one<L, false, LANES>(a, grid, st));
+        : k == ROI ? lines_one<L, false, ROI>(a, grid, st)
+        : k == SOLO ? lines_one<L, false, SOLO>(a, grid, st) : lines_one<L, false, LANES>(a, grid, st);
     else if (a.ms.sat)
         a.ms.formed ? lines_one<L, true, TALLY>(a, grid, st) : lines_one<L, true, TABLE>(a, grid, st);
     else
         k == ALL ? lines_one<L, true, ALL>(a, grid, st)
-                 : (k == SOLO ? lines_one<L, true, SOLO>(a, grid, st) : lines_one<L, true, LANES>(a, grid, st));
+        : k == ROI ? lines_one<L, true, ROI>(a, grid, st)
+        : k == SOLO ? lines_one<L, true, SOLO>(a, grid, st) : lines_one<L, true, LANES>(a, grid, st);
 }
 
 }  // namespace
