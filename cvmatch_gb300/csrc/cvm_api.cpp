@@ -661,9 +661,15 @@ int run_solo(const SoloJob &J, cudaStream_t st) {
     // template's spectrum (the fast form's sums its own samples) all start at
     // once.
     const bool known = J.mode == 0;
-    // (every CTA of the row kernel sums the template: small ones)
-    const bool early = !J.cachedP && (known ? !fast || (long long)J.tw * J.th <= 8192
-                                            : !J.frameOnSide && (long long)J.tw * J.th <= 65536);
+    // (Every CTA of the fast form's row kernel sums the template, so it takes
+    // small ones early; a large template's rows keep a colour frame's prep and
+    // rows waiting.  Colour matches early / behind k_prep, us: fast form, 640x480
+    // with 32x32 49 / 56, 64x64 59 / 60, 90x90 62 / 60, 1280x720 with 128x128 84 /
+    // 72, 256x256 178 / 91; exact form, 640x480 with 128x128 58 / 64, 181x181 75 /
+    // 65, 1920x1080 with 256x256 181 / 173.)
+    const long long tplArea = (long long)J.tw * J.th;
+    const bool early = !J.cachedP && (known ? !fast || tplArea <= 8192
+                                            : !J.frameOnSide && tplArea <= (fast ? 4096 : 16384));
     if (known && J.frameOnSide) CVM_CUDA(cudaStreamWaitEvent(st, ss.frame, 0));
     if (known || early) CVM_CUDA(cudaEventRecord(ss.fork, st));  // the inputs, P and F zeroed, the pool's buffers
     if (early) {
