@@ -996,7 +996,9 @@ int map_results(const float *dMap, int rw, int rh, float *map, const PeakReq *pk
 // caller's pointer), then run_solo's launches on a workspace of the graph's
 // own.  Inputs of up to kGraphStage bytes are copied behind those addresses by
 // the host first: 64 KB in 3 us, where the device takes 15 us to translate and
-// read a few pageable pages.
+// read a few pageable pages.  (A template beside a frame that is read in place
+// only up to kGraphStageTpl: the device reads it while it waits for the frame.
+// 1920x1080 with 181x181 RGBA, 131 KB: 211 us, 192 in place.)
 //
 // The process keeps up to kGraphs graphs and kGraphBytes of device memory for
 // them, each of at most kGraphBytesEach; a call has one to itself while it
@@ -1008,7 +1010,8 @@ int map_results(const float *dMap, int rw, int rh, float *map, const PeakReq *pk
 // nothing.)  A workspace allocation that fails gives all idle ones back.
 constexpr int kGraphs = 32, kGraphCalls = 3, kGraphShapes = 64;
 constexpr uint64_t kGraphStale = 256;
-constexpr size_t kGraphBytes = size_t(1) << 30, kGraphBytesEach = size_t(256) << 20, kGraphStage = size_t(192) << 10;
+constexpr size_t kGraphBytes = size_t(1) << 30, kGraphBytesEach = size_t(256) << 20, kGraphStage = size_t(192) << 10,
+                 kGraphStageTpl = size_t(32) << 10;
 
 struct SoloKey {
     int iw, ih, tw, th, mode, cn, step, gray, form, tune, map;
@@ -1160,7 +1163,8 @@ bool solo_capture(SoloGraph &g, SoloJob J, const Plan &plan, const SoloLayout &l
     const SoloKey &k = g.key;
     const int bpp = k.gray ? 4 : k.step;
     const size_t bImg = align_up((size_t)k.iw * bpp, 16) * k.ih, bTpl = align_up((size_t)k.tw * bpp, 16) * k.th;
-    const size_t sImg = bImg <= kGraphStage ? align_up(bImg, 256) : 0, sTpl = bTpl <= kGraphStage ? bTpl : 0;
+    const size_t sImg = bImg <= kGraphStage ? align_up(bImg, 256) : 0;
+    const size_t sTpl = bTpl <= (sImg ? kGraphStage : kGraphStageTpl) ? bTpl : 0;
     void *dSrc = nullptr, *dRes = nullptr;
     if (pool_alloc(g.mem, l.total, st) != CVM_OK ||
         cudaHostAlloc(reinterpret_cast<void **>(&g.src), 256 + sImg + sTpl, cudaHostAllocMapped) != cudaSuccess ||

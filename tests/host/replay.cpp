@@ -172,6 +172,22 @@ void memory_given_back() {
     EXPECT(fake::state().deviceBytes < held);
 }
 
+// Templates are staged beside a staged frame, and small ones beside others.
+void staged_templates() {
+    cvm_set_form(CVM_FORM_EXACT);
+    auto pinned = [&](int w, int h, int tw, int th) {
+        size_t before = 0, after = 0;
+        for (auto &a : fake::state().pinned) before += a.second;
+        for (int i = 0; i < 3; i++) EXPECT(call(w, h, tw, th) == CVM_OK);
+        for (auto &a : fake::state().pinned) after += a.second;
+        return after - before;
+    };
+    pinned(100, 90, 10, 10);  // (the thread's own slots)
+    EXPECT(pinned(200, 200, 100, 100) > 200 * 200 * 4 + 100 * 100 * 4);
+    EXPECT(pinned(1920, 1080, 80, 80) > 80 * 80 * 4);
+    EXPECT(pinned(1920, 1080, 181, 181) < 4096);
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -182,6 +198,8 @@ int main(int argc, char **argv) {
         plan_changes_during_the_capture(false);
     else if (what == "errors")
         errors_wait();
+    else if (what == "staged_templates")
+        staged_templates();
     else if (what == "threads_share")
         threads_share();
     else if (what == "threads_bounded")

@@ -39,3 +39,8 @@ def test_an_error_return_has_waited_for_what_reads_the_callers_memory(replay):
 def test_what_the_process_keeps_is_bounded_and_shared(replay, event):
     r = subprocess.run([replay, event], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
+
+
+def test_large_templates_are_read_in_place_beside_large_frames(replay):
+    r = subprocess.run([replay, "staged_templates"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr
