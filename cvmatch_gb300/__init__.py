@@ -394,8 +394,8 @@ class Fleet:
     def SetStats(self, mode: int):
         """STATS_KERNEL (the statistics kernel) or STATS_EPILOGUE (den on
         demand inside the inverse rows, from the frame's summed-area table,
-        where it applies); on one tile plan the results are the same bits.
-        Without a call the fleet chooses by itself.  See cvm_fleet_set_stats."""
+        where it applies); the results are the same bits.  Without a call the
+        fleet chooses by itself.  See cvm_fleet_set_stats."""
         _check(lib().cvm_fleet_set_stats(self._h, mode))
 
     def buckets(self, pw: int, ph: int):

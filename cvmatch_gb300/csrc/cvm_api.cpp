@@ -1502,12 +1502,12 @@ struct FleetBucketGeom {
 // cost: few, where blocks of results bound den well; many on flat panels beside
 // thin strokes under small templates, whose blocks have no bound, on frames
 // where everything scores like an extremum (a linear gradient), and in fleets so
-// small that all their rows start at once.  The first
-// frame chooses by a sample of its blocks (choose_stats).  Later calls look
-// again now and then, without waiting for the device: on demand, how many warp
-// steps of the rows went for a den; with the kernel, the blocks once more.  The
-// device leaves the tallies in page-locked memory, and the next call that finds
-// them there acts on them.  Results do not depend on it.
+// small that all their rows start at once.  A fleet starts by its size; its first
+// call, and later ones now and then, look at their frames without waiting for the
+// device: on demand, how many warp steps of the rows went for a den; with the
+// kernel, a sample of the blocks.  The device leaves the tallies in page-locked
+// memory, and the next call that finds them there acts on them.  Results do not
+// depend on it.
 struct DenWatch {
     DevMember *table = nullptr;  // the members that the summed-area table serves
     int n = 0;
@@ -1530,6 +1530,10 @@ struct DenWatch {
     // %) 0.134 / 0.137, 24 on 640x480 (28 %) 0.152 / 0.153, 2 there (all) 0.089 /
     // 0.073.
     static constexpr double kPoorShare = 1.0 / 32, kFormShare = 1.0 / 4;
+    // Fleets of fewer results (6 million) start with the kernel.  (On demand /
+    // kernel: 3.6 million 1.03, 4.1 million 1.13 and 1.00, 6.2 million 1.00, 7.4
+    // million 0.99, 8 million 0.93, 11 million 0.96 on noise and cameras' frames.)
+    static constexpr long long kFewSteps = 6000000 / 32;
 
     int now() {
         std::lock_guard<std::mutex> lk(mu);
@@ -1669,12 +1673,15 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
 // rest the frame's shared cost, and the bucket's cost is shared + n x
 // per-member.  newGoPlan's plan (fleet.go:356-365) is kept unless another
 // candidate beats it by more than 3 %.  Cached per (frame size, bucket
-// maxima, members, step, form, den's source) for the process.
+// maxima, members, step, form) for the process.  The trials take den from the
+// statistics kernel whatever the fleet does: a few members have no extrema to
+// cut by, so what they form on demand is not the bucket's share (64 templates on
+// 1920x1080, two streamed frames: timed on demand, 1024 x 512 and 2048 x 512
+// look alike and either is chosen, 2.14 or 2.24 ms; so, always 1024 x 512).
 struct FleetTuneKey {
-    int pw, ph, tw, th, step, form, n, stats;  // stats: den's source in the trials (their cost differs)
+    int pw, ph, tw, th, step, form, n;
     bool operator<(const FleetTuneKey &o) const {
-        return std::tie(pw, ph, tw, th, step, form, n, stats) <
-               std::tie(o.pw, o.ph, o.tw, o.th, o.step, o.form, o.n, o.stats);
+        return std::tie(pw, ph, tw, th, step, form, n) < std::tie(o.pw, o.ph, o.tw, o.th, o.step, o.form, o.n);
     }
 };
 struct FleetTuneEntry {
@@ -1687,24 +1694,24 @@ struct FleetTuneEntry {
 std::map<FleetTuneKey, FleetTuneEntry> g_fleetTune;
 
 // Whether nothing is left to measure for the bucket's plan: tuning off or not
-// for it (*out as it is), or tuned already (*out, when given).
-bool settled_bucket_plan(const cvm_fleet *f, const Bucket &b, int pw, int ph, int stats, Plan *out) {
+// for it (*out as it is), or tuned already (*out).
+bool settled_bucket_plan(const cvm_fleet *f, const Bucket &b, int pw, int ph, Plan *out) {
     const int nm = (int)b.members.size();
     if (f->form == CVM_FORM_EXACT || !g_autotune.load() || nm < 4) return true;
     std::lock_guard<std::mutex> lk(g_tuneMu);
-    auto it = g_fleetTune.find(FleetTuneKey{pw, ph, b.tw, b.th, f->step, f->form, nm, stats});
+    auto it = g_fleetTune.find(FleetTuneKey{pw, ph, b.tw, b.th, f->step, f->form, nm});
     if (it == g_fleetTune.end()) return false;
-    if (out) *out = it->second.plan;
+    *out = it->second.plan;
     return true;
 }
 
 int tune_bucket_plan(cvm_fleet *f, const Bucket &b, const uint8_t *dParent, long long pstride, int pw, int ph,
-                     cudaStream_t st, int stats, Plan *out) {
+                     cudaStream_t st, Plan *out) {
     const int rwF = pw - b.tw + 1, rhF = ph - b.th + 1;
     *out = make_plan(b.tw, b.th, rwF, rhF);
     const int nm = (int)b.members.size();
-    if (!dParent || settled_bucket_plan(f, b, pw, ph, stats, out)) return CVM_OK;
-    const FleetTuneKey key{pw, ph, b.tw, b.th, f->step, f->form, nm, stats};
+    if (!dParent || settled_bucket_plan(f, b, pw, ph, out)) return CVM_OK;
+    const FleetTuneKey key{pw, ph, b.tw, b.th, f->step, f->form, nm};
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
@@ -1744,7 +1751,7 @@ int tune_bucket_plan(cvm_fleet *f, const Bucket &b, const uint8_t *dParent, long
                 cvm_fleet trial;
                 trial.step = f->step;
                 trial.form = f->form;
-                trial.statsMode = stats;
+                trial.statsMode = CVM_STATS_KERNEL;
                 trial.forcedPlan = cands[c];
                 Bucket one;
                 one.tw = b.tw;
@@ -1873,15 +1880,10 @@ std::vector<Bucket> fast_buckets(const cvm_fleet *f, int pw, int ph) {
     return out;
 }
 
-// The first frame's choice of den's source (DenWatch), for a fast-form fleet
-// that cvm_fleet_set_stats left to itself: a sample of its members' blocks,
-// when the call may wait for the caller's stream (wait: it is about to time
-// plans on that frame).  Else, and inside a capture, nothing is sampled: on
-// demand, until a later call looks.
-int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, int ph, cudaStream_t cst, bool wait,
-                 std::unique_ptr<DenWatch> &out) {
+// A fast-form fleet's watch over its frames of one size (none where the table
+// serves no member).
+int den_watch(const cvm_fleet *f, int pw, int ph, std::unique_ptr<DenWatch> &out) {
     if (f->form != CVM_FORM_FAST || f->forcedPlan.dftW > 0) return CVM_OK;
-    const int np = f->step == 4 ? 4 : 2, hp = (int)align_up((size_t)pw + 1, 32);
     auto w = std::make_unique<DenWatch>();
     std::vector<DevMember> tab;
     for (const Bucket &b : f->buckets)
@@ -1899,6 +1901,7 @@ int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw
             w->steps += ((long long)d.rw * d.rh + 31) / 32;
         }
     if (tab.empty()) return CVM_OK;
+    if (w->steps < DenWatch::kFewSteps) w->source = CVM_STATS_KERNEL;
     w->n = (int)tab.size();
     CVM_CUDA(cudaMalloc(&w->table, tab.size() * sizeof(DevMember)));
     CVM_CUDA(cudaMemcpy(w->table, tab.data(), tab.size() * sizeof(DevMember), cudaMemcpyHostToDevice));
@@ -1913,46 +1916,6 @@ int choose_stats(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw
         w->tally = nullptr;
     }
     cudaGetLastError();
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (!wait || f->statsMode >= 0 || !dParent || cudaStreamIsCapturing(cst, &cs) != cudaSuccess ||
-        cs != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        out = std::move(w);
-        return CVM_OK;
-    }
-    CVM_CUDA(cudaStreamSynchronize(cst));  // the frame, written on the caller's stream
-    cudaStream_t ts = thread_stream();
-    const int n = (int)f->ms.size();
-    const size_t lanes = (size_t)(ph + 1) * hp * (np == 4 ? 6 : 2);
-    PoolBuf buf;
-    CVM_TRY(pool_alloc(buf,
-                       Arena::bytes(n, sizeof(DevParams)) + Arena::bytes(1, sizeof(DevFrame)) +
-                           Arena::bytes(1, sizeof(int)) + Arena::bytes(lanes, 4) +
-                           Arena::bytes(sat_scratch_elems(ph, hp, np), 4),
-                       ts));
-    Arena A;
-    A.base = static_cast<char *>(buf.p);
-    DevParams *P = A.take<DevParams>(n);
-    DevFrame *F = A.take<DevFrame>(1);
-    int *dPoor = A.take<int>(1), poor = 0;
-    unsigned int *sat = A.take<unsigned int>(lanes), *blk = A.take<unsigned int>(sat_scratch_elems(ph, hp, np));
-    CVM_CUDA(cudaMemsetAsync(F, 0, sizeof(DevFrame), ts));
-    CVM_CUDA(cudaMemsetAsync(dPoor, 0, sizeof(int), ts));
-    CVM_CUDA(launch_prep(nullptr, 0, 0, 0, f->step, 0, f->step == 4 ? dParent : nullptr, pstride, pw, ph, P, n, 0, 0, 0,
-                         F, ts, f->dP));
-    CVM_CUDA(launch_sat(dParent, pstride, pw, ph, hp, np, &F->cnMax, blk, sat, ts));
-    MemberSet ms;
-    memset(&ms, 0, sizeof ms);
-    ms.table = w->table;
-    ms.params = P;
-    ms.sat = sat;
-    ms.satRow = (size_t)np * hp;
-    ms.satAlpha = np == 4 ? (size_t)(ph + 1) * 4 * hp : 0;
-    ms.satNp = np;
-    CVM_CUDA(launch_den_poor(ms, w->n, dPoor, ts));
-    CVM_CUDA(cudaMemcpyAsync(&poor, dPoor, sizeof(int), cudaMemcpyDeviceToHost, ts));
-    CVM_CUDA(cudaStreamSynchronize(ts));
-    if (poor > DenWatch::kPoorShare * 256 * w->n) w->source = CVM_STATS_KERNEL;
     out = std::move(w);
     return CVM_OK;
 }
@@ -1970,11 +1933,7 @@ int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, 
     fg->form = f->form;
     const std::vector<Bucket> buckets =
         f->form != CVM_FORM_EXACT && f->forcedPlan.dftW == 0 ? fast_buckets(f, pw, ph) : f->buckets;
-    bool wait = false;
-    for (const Bucket &b : buckets)
-        wait = wait || !settled_bucket_plan(f, b, pw, ph, CVM_STATS_EPILOGUE, nullptr);
-    CVM_TRY(choose_stats(f, dParent, pstride, pw, ph, cst, wait, fg->watch));
-    const int stats = f->statsMode >= 0 ? f->statsMode : (fg->watch ? fg->watch->source : CVM_STATS_KERNEL);
+    CVM_TRY(den_watch(f, pw, ph, fg->watch));
     cudaStream_t st = thread_stream();
     for (const Bucket &b : buckets) {
         auto bg = std::make_unique<FleetBucketGeom>();
@@ -1983,7 +1942,7 @@ int fleet_geom(cvm_fleet *f, const uint8_t *dParent, long long pstride, int pw, 
         if (f->forcedPlan.dftW > 0)
             plan = f->forcedPlan;
         else
-            CVM_TRY(tune_bucket_plan(f, b, dParent, pstride, pw, ph, cst, stats, &plan));
+            CVM_TRY(tune_bucket_plan(f, b, dParent, pstride, pw, ph, cst, &plan));
         CVM_TRY(make_geom(b.tw, b.th, rwF, rhF, b.th, bg->G, &plan));
         bg->form = effective_form(f->form, bg->G);
         const bool bfast = bg->form != CVM_FORM_EXACT;

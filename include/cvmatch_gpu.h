@@ -370,11 +370,11 @@ int cvm_fleet_set_overlap(cvm_fleet *f, int on);
  * may hold an extremum (a lower bound of den over blocks of results rules
  * out the rest), with no statistics launch and no den written or read; other
  * buckets, and every exact- or mixed-form bucket, still run the statistics
- * kernel.  On one tile plan the results are the same bits either way; the
- * autotuner times a bucket's plans for the source the fleet had when it first
- * met the frame size, and plans differ within the fast form's rounding.  A
- * fleet on which this was never called chooses by itself: by a sample of its
- * first frame of a size, when plans are timed on it, and again whenever a look at a later call, one in
+ * kernel.  Results are the same bits either way (the autotuner's trials run
+ * the kernel, so plans do not depend on it either).  A fleet on which this was
+ * never called chooses by itself: by its size at first (fleets of fewer than 6
+ * million results start with the kernel), and again whenever a look at a call,
+ * its first ones and then one in
  * some tens to thousands, shows that the frames are of another kind (256 RGBA
  * templates on a 2560x1440 frame: 5.5 ms per FindAll with the epilogue, 7.8
  * with the kernel; small templates on flat panels with thin strokes, linear

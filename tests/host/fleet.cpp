@@ -23,8 +23,8 @@ int find(cvm_fleet *f, int w = 640, int h = 480) {
     return cvm_fleet_find_all(f, frame.data(), 4 * w, w, h, r.data());
 }
 
-// Plans are tuned apart for the two sources of den.
-void tuned_per_source() {
+// Plans are timed once, whatever source of den the fleets have.
+void tuned_once() {
     char buf[1 << 14];
     for (int mode : {CVM_STATS_KERNEL, CVM_STATS_EPILOGUE, CVM_STATS_KERNEL}) {
         cvm_fleet *f = fleet(8, 20);
@@ -34,7 +34,8 @@ void tuned_per_source() {
     cvm_autotune_report(buf, sizeof buf);
     int n = 0;
     for (const char *p = buf; (p = strstr(p, "\"fleet\":true")); p++) n++;
-    EXPECT(n == 2);
+    EXPECT(n == 1);
+    EXPECT(fake::state().calls["inv_rows_table"] == 1);  // the on-demand fleet's own call, no trial
 }
 
 // Contents as the device would report them.
@@ -60,21 +61,26 @@ int on_demand(cvm_fleet *f, int n) {
 void the_choice_follows() {
     cvm_set_autotune(0);
     for (Content first : {camera, black}) {
-        cvm_fleet *f = fleet(8, 20);
-        show(first, 8, 20);
+        cvm_fleet *f = fleet(32, 20);
+        show(first, 32, 20);
         EXPECT(on_demand(f, 1) == 1);
-        show(icons, 8, 20);
+        show(icons, 32, 20);
         EXPECT(on_demand(f, 1000) <= 8);
-        show(camera, 8, 20);
+        show(camera, 32, 20);
         EXPECT(on_demand(f, 1000) >= 900);
-        show(icons, 8, 20);
+        show(icons, 32, 20);
         EXPECT(on_demand(f, 1000) <= 200);
     }
-    cvm_fleet *f = fleet(8, 20);
-    show(gradient, 8, 20);
+    cvm_fleet *f = fleet(32, 20);
+    show(gradient, 32, 20);
     EXPECT(on_demand(f, 4000) <= 60);
-    show(camera, 8, 20);
+    show(camera, 32, 20);
     EXPECT(on_demand(f, 10000) >= 5000);
+    // a small fleet starts with the kernel and is tried on demand, briefly
+    f = fleet(2, 20);
+    show(gradient, 2, 20);  // (all its steps form den)
+    EXPECT(on_demand(f, 1) == 0);
+    EXPECT(on_demand(f, 4000) <= 60);
     // said once, it stays
     f = fleet(8, 20);
     EXPECT(cvm_fleet_set_stats(f, CVM_STATS_EPILOGUE) == CVM_OK);
@@ -85,9 +91,9 @@ void the_choice_follows() {
 // A first call inside a caller's capture samples nothing; a later call does.
 void captured_first() {
     cvm_set_autotune(0);
-    cvm_fleet *f = fleet(8, 20);
-    show(icons, 8, 20);
-    cvm_result r[8];
+    cvm_fleet *f = fleet(32, 20);
+    show(icons, 32, 20);
+    cvm_result r[32];
     cudaStream_t st;
     cudaStreamCreateWithFlags(&st, 0);
     cudaStreamBeginCapture(st, cudaStreamCaptureModeGlobal);
@@ -117,11 +123,11 @@ void a_streams_spectra() {
 // when the fleet goes on to other sizes.
 void a_stream_follows() {
     cvm_set_autotune(0);
-    cvm_fleet *f = fleet(8, 20);
-    show(camera, 8, 20);
+    cvm_fleet *f = fleet(32, 20);
+    show(camera, 32, 20);
     cvm_stream *s;
     EXPECT(cvm_stream_new(f, nullptr, 640, 480, &s) == CVM_OK);
-    std::vector<cvm_result> r(8);
+    std::vector<cvm_result> r(32);
     auto pushed = [&](int n) {
         const long before = fake::state().calls["inv_rows_table"], graphs = fake::state().calls["cudaGraphLaunch"];
         for (int i = 0; i < n; i++) {
@@ -132,17 +138,17 @@ void a_stream_follows() {
         return fake::state().calls["inv_rows_table"] - before;
     };
     pushed(100);
-    show(icons, 8, 20);
+    show(icons, 32, 20);
     pushed(100);
     EXPECT(pushed(1000) == 0);
-    show(camera, 8, 20);
+    show(camera, 32, 20);
     pushed(400);
     EXPECT(pushed(1000) > 0);  // the looks, and a capture before them
     int graphed = 0, launches = 0;
     EXPECT(cvm_stream_info(s, &graphed, &launches) == CVM_OK && graphed);
     // the fleet is used at another size meanwhile
     EXPECT(find(f, 320, 200) == CVM_OK);
-    show(icons, 8, 20);
+    show(icons, 32, 20);
     pushed(200);
     EXPECT(find(f, 320, 200) == CVM_OK);
     pushed(200);
@@ -192,8 +198,8 @@ void partly_locked() {
 
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
-    if (what == "tuned_per_source")
-        tuned_per_source();
+    if (what == "tuned_once")
+        tuned_once();
     else if (what == "the_choice_follows")
         the_choice_follows();
     else if (what == "a_streams_spectra")

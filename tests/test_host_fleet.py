@@ -17,8 +17,8 @@ def _run(exe, what):
     assert r.returncode == 0, r.stderr
 
 
-def test_plans_are_tuned_per_source_of_den(fleet):
-    _run(fleet, "tuned_per_source")
+def test_plans_are_timed_once_for_either_source_of_den(fleet):
+    _run(fleet, "tuned_once")
 
 
 @pytest.mark.parametrize("what", ["the_choice_follows", "captured_first", "a_stream_follows"])
