@@ -1555,7 +1555,7 @@ struct DenWatch {
         if (!seq) return true;
         asked = calls;
         next = calls + gap;
-        gap = std::min(2 * gap, calm);
+        gap = gap < 2 ? 2 : calm;  // calls 1, 2 and 4, then every calm-th
         *seq = (unsigned)asked;
         return true;
     }
@@ -2113,19 +2113,21 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     for (const Bucket &b : f->buckets) twMax = std::max(twMax, b.tw);
     const size_t prefixRow = (size_t)(cnP == 4 ? 4 : stat_pitch(cnP)) * hpP;
     const size_t alphaRow = cnP == 4 ? (size_t)2 * hpP : 0;
-    const bool needSat = anySat || look;
-    const size_t satElems = needSat ? (size_t)(ph + 1) * (prefixRow + alphaRow) : 0;
-    const size_t satBlkElems = needSat ? sat_scratch_elems(ph, hpP, cnP == 4 ? 4 : 2) : 0;
-    const size_t tallyElems = look ? kTallyWords : 0;
+    const size_t satElems = anySat || look ? (size_t)(ph + 1) * (prefixRow + alphaRow) : 0;
+    const size_t satBlkElems = anySat || look ? sat_scratch_elems(ph, hpP, cnP == 4 ? 4 : 2) : 0;
+    // (what a look alone needs is apart, so that every call's workspace has one
+    // size, which the pool has at hand)
+    const size_t satBytes =
+        satElems ? Arena::bytes(satElems, sizeof(unsigned int)) + Arena::bytes(satBlkElems, sizeof(unsigned int)) : 0;
+    PoolBuf lookBuf;
+    if (look)
+        CVM_TRY(pool_alloc(lookBuf, Arena::bytes(kTallyWords, sizeof(unsigned int)) + (anySat ? 0 : satBytes), st));
     const bool blkOk = anyStatsKernel && 16ull * (unsigned)twMax * (cnP == 4 ? 3u : 1u) * 65025ull < (1ull << 32);
     const size_t blkElems = blkOk ? prefixRow * (size_t)(ph / 16) : 0;
     const size_t bytes = Arena::bytes(n, sizeof(DevParams)) + Arena::bytes(1, sizeof(DevFrame)) +
                          Arena::bytes((size_t)3 * n, sizeof(int)) + Arena::bytes(prefixElems, sizeof(unsigned int)) +
                          (blkElems ? Arena::bytes(blkElems, sizeof(unsigned int)) : 0) +
-                         (satElems ? Arena::bytes(satElems, sizeof(unsigned int)) +
-                                         Arena::bytes(satBlkElems, sizeof(unsigned int))
-                                   : 0) +
-                         Arena::bytes(tallyElems, sizeof(unsigned int)) + frameBytes + partBytes + waveBytes;
+                         (anySat ? satBytes : 0) + frameBytes + partBytes + waveBytes;
     // Overlapped waves (fast-form buckets, more than one wave in all): the
     // inverse rows of wave k run on the side stream beside the statistics
     // and columns of wave k + 1, so the waves alternate between two sets of
@@ -2152,9 +2154,14 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     int *counters = reinterpret_cast<int *>(bounds + 2 * (size_t)n);
     unsigned int *prefix = A.take<unsigned int>(prefixElems);
     unsigned int *prefixBlk = blkElems ? A.take<unsigned int>(blkElems) : nullptr;
-    unsigned int *sat = satElems ? A.take<unsigned int>(satElems) : nullptr;
-    unsigned int *satBlk = satElems ? A.take<unsigned int>(satBlkElems) : nullptr;
-    unsigned int *tally = A.take<unsigned int>(tallyElems);
+    Arena LA;
+    LA.base = static_cast<char *>(lookBuf.p);
+    unsigned int *tally = look ? LA.take<unsigned int>(kTallyWords) : nullptr;
+    unsigned int *sat = nullptr, *satBlk = nullptr;
+    if (satElems) {
+        sat = (anySat ? A : LA).take<unsigned int>(satElems);
+        satBlk = (anySat ? A : LA).take<unsigned int>(satBlkElems);
+    }
     char *frameBase = A.base + A.used;
     A.used += frameBytes;
     Partial *parts = reinterpret_cast<Partial *>(A.base + A.used);

@@ -119,16 +119,23 @@ __device__ __forceinline__ float2 ld_once(const float2 *p) {
 
 constexpr int kBlocksMax = 1024;  // of a CTA: 8192 results over two rows a pair, in 4 x 4 blocks
 
+// A tallied call's counter in shared memory, behind the blocks' bounds.
+template <int L>
+__device__ __forceinline__ unsigned int *tally_word() {
+    extern __shared__ __align__(16) float2 smem[];
+    return reinterpret_cast<unsigned int *>(reinterpret_cast<float *>(smem + (size_t)Lines<L>::NL * Lines<L>::LINE) +
+                                            kBlocksMax);
+}
+
 // A result above its block's bound: its den, and the ladder unless that
-// already rules it out.
-template <bool COUNT>
+// already rules it out.  (TALLY: the row length of a tallied call, else 0.)
+template <int TALLY>
 __device__ __noinline__ Track score_table(Track t, float num, const MemberSet &ms, const DevMember &m,
                                           const DevParams &Pm, int y, int x, float denFlat, int l) {
-    if constexpr (COUNT) {
+    if constexpr (TALLY > 0) {
         // (the warp's lanes that are here, once)
         const unsigned int here = __activemask();
-        if ((threadIdx.x & 31) == __ffs(here) - 1)
-            atomicAdd(ms.formed + kTallyFormed + 16 * ((blockIdx.x + blockIdx.y) & (kTallySpread - 1)), 1u);
+        if ((threadIdx.x & 31) == __ffs(here) - 1) atomicAdd(tally_word<TALLY>(), 1u);
     }
     const float d = sat_den(ms, m, Pm, y, x);
     if (d > 0.f && num < t.hi * d && num > t.lo * d) return t;
@@ -217,6 +224,7 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
         nbx = (bw + (1 << lgx) - 1) >> lgx;
         const int rows = min(2 * P, bh - 2 * pair0), n = nbx * ((rows + (1 << lgy) - 1) >> lgy);
         bool flat = true;
+        if (KEEP == TALLY && tid == 0) *tally_word<L>() = 0u;
 #pragma unroll 1
         for (int i = tid; i < n; i += S::CTA) {
             const int by = i / nbx, x = (i - by * nbx) << lgx, y = by << lgy;
@@ -425,7 +433,8 @@ __device__ __forceinline__ Ext line_pairs(const InvArgs &a, float2 *smem, const 
                         const bool cand = x < xb && (MODE != ROI || x >= xa) && d != zero &&
                                           !(num < hp * d && num > lp * d);
                         if constexpr (MODE == TABLE) {
-                            if (cand) t = score_table<KEEP == TALLY>(t, num, a.ms, m, Pm, y0 + h, tb.x0 + x, denFlat, l);
+                            if (cand)
+                                t = score_table<KEEP == TALLY ? L : 0>(t, num, a.ms, m, Pm, y0 + h, tb.x0 + x, denFlat, l);
                         } else if constexpr (LEAN) {
                             if (cand) t = score_track<FAST>(t, num, d, denFlat, l);
                         } else if (x < bw) {
@@ -514,6 +523,11 @@ __global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, MODE)) k_in
     }
     // a CTA none of whose results passed its member's cuts has nothing to reduce
     if (__syncthreads_or(e.minI != LLONG_MAX || e.maxI != LLONG_MAX)) ext_block_reduce(e, shExt);
+    if (MODE == TALLY && tid == 0 && P > 0 && !Pm.flat) {
+        const unsigned int formed = *tally_word<L>();
+        if (formed)
+            atomicAdd(a.ms.formed + kTallyFormed + 16 * ((blockIdx.x + blockIdx.y) & (kTallySpread - 1)), formed);
+    }
     if (tid == 0) {
         Partial &o = a.partials[m.partBase + a.partOffset + tileLocal * gridDim.y + blockIdx.y];
         o.minV = e.minV;
@@ -547,7 +561,7 @@ __global__ void __launch_bounds__(Lines<L>::CTA, lines_ctas(L, FAST, MODE)) k_in
 
 template <int L, bool FAST, Keep MODE>
 void lines_one(const InvArgs &a, dim3 grid, cudaStream_t st) {
-    const size_t smem = Lines<L>::SMEM + (MODE == TABLE || MODE == TALLY ? kBlocksMax * sizeof(float) : 0);
+    const size_t smem = Lines<L>::SMEM + (MODE == TABLE || MODE == TALLY ? (kBlocksMax + 1) * sizeof(float) : 0);
     set_smem(k_inv_lines<L, FAST, MODE>, smem);
     launch_k(k_inv_lines<L, FAST, MODE>, grid, dim3(Lines<L>::CTA), smem, st, a);
 }
