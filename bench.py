@@ -1290,7 +1290,7 @@ def main():
     ap.add_argument("--stats", default="auto", choices=["auto", "kernel", "epilogue"],
                     help="--workload fleet: window statistics from the statistics kernel, or formed in the "
                          "inverse-rows epilogue from the frame's summed-area table (cvm_fleet_set_stats); auto: "
-                         "the library chooses on its first frame")
+                         "the library chooses")
     ap.add_argument("--wave", type=int, default=0,
                     help="--workload fleet: member tails per wave (cvm_fleet_set_wave; 0: the workspace budget's)")
     ap.add_argument("--overlap", default="on", choices=["on", "off"],

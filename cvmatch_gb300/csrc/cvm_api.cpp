@@ -990,7 +990,7 @@ int map_results(const float *dMap, int rw, int rh, float *map, const PeakReq *pk
 // A repeated one-shot call as a CUDA graph.  A small host-buffer call queued
 // launch by launch -- some thirty runtime calls over four streams -- is bound
 // by the host: 84 us for a 320x200 gray match, 104 for a 640x480 one from
-// RGBA; replayed 45 and 57 us (GB300, Grace host).  From the kGraphCalls-th call of a shape on, by
+// RGBA; replayed 44 and 54 us (GB300, Grace host).  From the kGraphCalls-th call of a shape on, by
 // whichever threads, its launches are replayed as one graph: the inputs by one kernel that takes the
 // caller's addresses from mapped page-locked memory (so the graph holds no
 // caller's pointer), then run_solo's launches on a workspace of the graph's
@@ -2049,7 +2049,7 @@ int fleet_find_dev(cvm_fleet *f, const uint8_t *dParent, long long pstride, int 
     // the frame's summed-area table (cvm_lines.cu): no statistics kernel, no
     // den lanes.  The rows need a length that kernel takes, the members an
     // area the table serves.  (256 templates on 2560x1440, launches in
-    // sequence: statistics 2.72 ms and rows 1.86 ms with the lanes, rows 2.31
+    // sequence: statistics 2.72 ms and rows 1.86 ms with the lanes, rows 2.34
     // ms on demand.)
     int stats = f->statsMode >= 0 ? f->statsMode : CVM_STATS_KERNEL;
     bool look = false;  // this call is tallied for the fleet's own choice

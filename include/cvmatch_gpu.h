@@ -310,14 +310,16 @@ int cvm_device_status(int *tc_timeouts);
  * Fleet.FindAll (fleet.go:176-332) for a video feed; no reference
  * counterpart as an object.  The per-frame pipeline (frame upload, both
  * FindAlls, the gray conversion, result read-back) is captured once as a
- * CUDA graph per frame slot and replayed; two slots let one frame's upload
+ * CUDA graph per frame slot and replayed (captured again when a fleet changes
+ * its source of den); two slots let one frame's upload
  * overlap the previous frame's matching.  Results are identical to calling
  * cvm_fleet_find_all per frame.  The fleets must outlive the stream. */
 typedef struct cvm_stream cvm_stream;
 int cvm_stream_new(cvm_fleet *color, cvm_fleet *gray_or_null, int pw, int ph, cvm_stream **out);
 /* Queue one frame (pw x ph RGBA, row stride in bytes); the pixels are
- * copied before the call returns.  With both slots in flight it first
- * waits for the oldest frame. */
+ * read before the call returns.  With both slots in flight it is refused:
+ * pull a frame first.  (Now and then a frame is queued launch by launch: see
+ * cvm_fleet_set_stats.) */
 int cvm_stream_push(cvm_stream *s, const uint8_t *rgba, int64_t stride);
 /* Results of the oldest queued frame (waits for it): color_out receives the
  * colour fleet's n results, gray_out the gray fleet's (may be null without
@@ -374,15 +376,14 @@ int cvm_fleet_set_overlap(cvm_fleet *f, int on);
  * the kernel, so plans do not depend on it either).  A fleet on which this was
  * never called chooses by itself: by its size at first (fleets of fewer than 6
  * million results start with the kernel), and again whenever a look at a call,
- * its first ones and then one in
- * some tens to thousands, shows that the frames are of another kind (256 RGBA
- * templates on a 2560x1440 frame: 5.5 ms per FindAll with the epilogue, 7.8
+ * its first ones and then one in some tens to thousands, shows that the frames
+ * are of another kind (256 RGBA templates on a 2560x1440 frame: 5.5 ms per FindAll with the epilogue, 7.8
  * with the kernel; small templates on flat panels with thin strokes, linear
  * gradients and fleets of a few members are faster with the kernel).  A call
  * inside a stream capture looks at nothing and runs what the fleet chose
- * before it, or the epilogue; a frame stream's graphs are captured again when
- * its fleets choose anew on the frames pushed.  Not to be called while a FindAll on the same
- * fleet runs. */
+ * before it; a frame stream's graphs are captured again when its fleets choose
+ * anew on the frames pushed.  Not to be called while a FindAll on the same fleet
+ * runs. */
 #define CVM_STATS_KERNEL 0
 #define CVM_STATS_EPILOGUE 1
 int cvm_fleet_set_stats(cvm_fleet *f, int mode);
