@@ -1518,9 +1518,9 @@ struct DenWatch {
     uint64_t calls = 0, asked = 0, next = 1;  // asked: the call being tallied (0: none)
     uint64_t gap = 1, calm = 32;              // calls until the look after the next; its largest value
 
-    // More than kPoorShare of the blocks without a bound, or kFormShare of the
-    // rows' steps forming den, choose the kernel; half of kPoorShare chooses on
-    // demand.  On 1920x1080, on demand / with the kernel in ms: 64 icons of 12..32
+    // More than kFormShare of the rows' steps forming den choose the kernel; with
+    // it, fewer than kPoorShare of the blocks without a bound choose on demand.
+    // On 1920x1080, on demand / with the kernel in ms: 64 icons of 12..32
     // px on a user interface (17 % of the blocks) 1.35 / 0.88, 16..64 px (7 %)
     // 1.48 / 1.10, 24..96 px (none; 11 % of the steps) 1.04 / 1.11; 8 templates of
     // 24..64 px on a camera's frame (14 % of the steps) 0.28 / 0.30; 32 on a
@@ -1529,7 +1529,7 @@ struct DenWatch {
     // from others' extrema: 2 templates (59 %) 0.167 / 0.148, 12 on 960x540 (26..33
     // %) 0.134 / 0.137, 24 on 640x480 (28 %) 0.152 / 0.153, 2 there (all) 0.089 /
     // 0.073.
-    static constexpr double kPoorShare = 1.0 / 32, kFormShare = 1.0 / 4;
+    static constexpr double kPoorShare = 1.0 / 64, kFormShare = 1.0 / 4;
     // Fleets of fewer results (6 million) start with the kernel.  (On demand /
     // kernel: 3.6 million 1.03, 4.1 million 1.13 and 1.00, 6.2 million 1.00, 7.4
     // million 0.99, 8 million 0.93, 11 million 0.96 on noise and cameras' frames.)
@@ -1562,7 +1562,7 @@ struct DenWatch {
     void judge(const DenTally &t) {
         const int was = source;
         if (t.source == CVM_STATS_EPILOGUE && t.formed > kFormShare * steps) source = CVM_STATS_KERNEL;
-        if (t.source == CVM_STATS_KERNEL && t.poor < 0.5 * kPoorShare * 256 * n) source = CVM_STATS_EPILOGUE;
+        if (t.source == CVM_STATS_KERNEL && t.poor < kPoorShare * 256 * n) source = CVM_STATS_EPILOGUE;
         if (source == was) {
             calm = std::max<uint64_t>(calm / 2, 32);
         } else if (source == CVM_STATS_EPILOGUE) {
