@@ -1546,7 +1546,7 @@ struct DenWatch {
         calls++;
         if (asked && static_cast<volatile DenTally *>(tally)->seq == (unsigned)asked) {
             std::atomic_thread_fence(std::memory_order_acquire);
-            judge(*tally);
+            weigh(*tally);
             asked = 0;
         }
         *src = source;
@@ -1559,7 +1559,7 @@ struct DenWatch {
         *seq = (unsigned)asked;
         return true;
     }
-    void judge(const DenTally &t) {
+    void weigh(const DenTally &t) {
         const int was = source;
         if (t.source == CVM_STATS_EPILOGUE && t.formed > kFormShare * steps) source = CVM_STATS_KERNEL;
         if (t.source == CVM_STATS_KERNEL && t.poor < kPoorShare * 256 * n) source = CVM_STATS_EPILOGUE;
